@@ -96,7 +96,8 @@ def _activations(M, K, gen, dtype):
     return a.to(dtype)
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """The tensors of a case: operands and scales, or a layer's float weight, bias and activations."""
     gen = torch.Generator(device="cuda").manual_seed(int(seed))
     M, N, K = case["M"], case["N"], case["K"]
 
@@ -106,20 +107,24 @@ def prepare(case, seed):
     def scales(*shape):
         return torch.rand(*shape, device="cuda", generator=gen) * 0.02 + 0.001
 
-    state = {"kind": case["kind"]}
     if case["kind"] == "plain":
-        state.update(x=int8(M), y=int8(N), alpha=case["alpha"])
-    elif case["kind"] == "scaled":
-        state.update(x=int8(M), y=int8(N), sx=scales(M), sw=scales(N))
-    elif case["kind"] == "blockwise":
+        return dict(x=int8(M), y=int8(N))
+    if case["kind"] == "scaled":
+        return dict(x=int8(M), y=int8(N), sx=scales(M), sw=scales(N))
+    if case["kind"] == "blockwise":
         kb = -(-K // 128)
-        state.update(x=int8(M), y=int8(N), sx=scales(M, kb), sw=scales(-(-N // 128), kb))
-    else:
-        w = torch.randn(N, K, generator=gen, device="cuda") * 0.02
-        bias = (torch.randn(N, generator=gen, device="cuda") * 0.1).to(torch.bfloat16) if case["bias"] else None
-        state["layer"] = g.Int8Linear.from_float(w, bias, mode=case["mode"], hadamard_block=case["hadamard"] or None)
-        state["x"] = _activations(M, K, gen, torch.bfloat16 if case["act"] == "bf16" else torch.float32)
-    return state
+        return dict(x=int8(M), y=int8(N), sx=scales(M, kb), sw=scales(-(-N // 128), kb))
+    w = torch.randn(N, K, generator=gen, device="cuda") * 0.02
+    bias = (torch.randn(N, generator=gen, device="cuda") * 0.1).to(torch.bfloat16) if case["bias"] else None
+    return dict(w=w, bias=bias, x=_activations(M, K, gen, torch.bfloat16 if case["act"] == "bf16" else torch.float32))
+
+
+def prepare(case, seed):
+    t = _inputs(case, seed)
+    if case["kind"] != "linear":
+        return dict(t, kind=case["kind"], alpha=case["alpha"])
+    layer = g.Int8Linear.from_float(t["w"], t["bias"], mode=case["mode"], hadamard_block=case["hadamard"] or None)
+    return {"kind": "linear", "layer": layer, "x": t["x"]}
 
 
 def run(state):
@@ -153,3 +158,45 @@ def tolerance(case):
     if case["bias"]:
         return {"rel": 9.5e-3, "max": 3.0e-2}
     return {"rel": 6.6e-3, "max": 1.6e-2}
+
+
+def _rotate64(a, block):
+    """Normalised Walsh-Hadamard transform of the rows in blocks of `block`, as a product with the matrix."""
+    h = torch.ones(1, 1, dtype=torch.float64, device=a.device)
+    while h.shape[0] < block:
+        h = torch.cat((torch.cat((h, h), 1), torch.cat((h, -h), 1)), 0)
+    return ((a.reshape(-1, block) @ h) * block ** -0.5).reshape(a.shape)
+
+
+def _rounded(a, rows, cols):
+    """What symmetric int8 quantisation leaves of `a`, one scale per rows x cols tile, in the precision of `a`."""
+    R, C = a.shape
+    p = torch.nn.functional.pad(a, (0, -C % cols, 0, -R % rows))
+    t = p.reshape(p.shape[0] // rows, rows, p.shape[1] // cols, cols)
+    s = t.abs().amax(dim=(1, 3), keepdim=True) / 127.0
+    s = torch.where(s > 0, s, torch.ones_like(s))
+    return (torch.round(t / s).clamp(-127, 127) * s).reshape(p.shape)[:R, :C]
+
+
+def exact(case, seed):
+    """The result in 64 bits.  Quantisation is part of what a layer computes and is carried out in 64 bits as well."""
+    t = _inputs(case, seed)
+    M, N, K = case["M"], case["N"], case["K"]
+    x = t.pop("x").double()
+    if case["kind"] == "linear":
+        w = t.pop("w").double()
+        if case["hadamard"]:
+            x, w = _rotate64(x, case["hadamard"]), _rotate64(w, case["hadamard"])
+        blocks = case["mode"] == "blockwise"
+        x = _rounded(x, 1, 128 if blocks else K)
+        w = _rounded(w, 128 if blocks else 1, 128 if blocks else K)
+        out = x @ w.t()
+        return out if t["bias"] is None else out + t["bias"].double()
+    y = t.pop("y").double()
+    if case["kind"] == "blockwise":
+        x *= t["sx"].double().repeat_interleave(128, dim=1)[:, :K]
+        y *= t["sw"].double().repeat_interleave(128, dim=1)[:, :K].repeat_interleave(128, dim=0)[:N]
+    out = x @ y.t()
+    if case["kind"] == "scaled":
+        out *= t["sx"].double()[:, None] * t["sw"].double()[None, :]
+    return out * case["alpha"] if case["kind"] == "plain" else out
