@@ -766,23 +766,39 @@ __global__ void sum_parts_bf16_kernel(const float* __restrict__ parts, int n_par
 }
 
 template <typename T>
-static int launch_hadamard_quant(const T* in, int8_t* q, float* scales, int64_t M, int K, int KB, int H, cudaStream_t s)
+static void launch_quant_row(const T* in, int8_t* q, float* scales, int64_t M, int K, int blocks, cudaStream_t s)
 {
-    const int threads = H / 4 < kQuantThreads ? H / 4 : kQuantThreads;
-    const int e = H / threads;
-    const size_t smem = threads > 32 ? sizeof(float) * H : 0;
-    const float norm = static_cast<float>(pow(static_cast<double>(H), -0.5));
-    const int64_t blocks = M * (K / H);
+    const int64_t loads = (static_cast<int64_t>(K) * sizeof(T) + kQuantThreads * 16 - 1) / (kQuantThreads * 16);
+    if (loads <= 2) quantize_token_row_kernel<T, 2><<<blocks, kQuantThreads, 0, s>>>(in, q, scales, M, K);
+    else if (loads <= 4) quantize_token_row_kernel<T, 4><<<blocks, kQuantThreads, 0, s>>>(in, q, scales, M, K);
+    else quantize_token_row_kernel<T, 8><<<blocks, kQuantThreads, 0, s>>>(in, q, scales, M, K);
+}
+
+template <typename T, int LOGH>
+static int launch_hadamard_quant(const T* in, int8_t* q, float* scales, int64_t total, cudaStream_t s)
+{
+    using S = HadamardShape<LOGH>;
+    const float norm = static_cast<float>(pow(static_cast<double>(1 << LOGH), -0.5));
+    const int64_t per_cta = static_cast<int64_t>(S::UNITS) << S::LOGU;
+    const int64_t blocks = (total + per_cta - 1) / per_cta;
     if (blocks > INT32_MAX) return fail(GI8_ERR_UNSUPPORTED_SHAPE, "too many rotation blocks");
-    const int grid = static_cast<int>(blocks);
-    switch (e) {
-        case 4: hadamard_quantize_token_block_kernel<T, 4><<<grid, threads, smem, s>>>(in, q, scales, K, KB, H, norm); break;
-        case 8: hadamard_quantize_token_block_kernel<T, 8><<<grid, threads, smem, s>>>(in, q, scales, K, KB, H, norm); break;
-        case 16: hadamard_quantize_token_block_kernel<T, 16><<<grid, threads, smem, s>>>(in, q, scales, K, KB, H, norm); break;
-        default: hadamard_quantize_token_block_kernel<T, 32><<<grid, threads, smem, s>>>(in, q, scales, K, KB, H, norm); break;
-    }
+    hadamard_quantize_token_block_kernel<T, LOGH><<<static_cast<int>(blocks), S::THREADS * S::UNITS, 0, s>>>(in, q, scales, total, norm);
     GI8_CUDA(cudaGetLastError());
     return GI8_OK;
+}
+
+template <typename T>
+static int launch_hadamard_quant(const T* in, int8_t* q, float* scales, int64_t total, int H, cudaStream_t s)
+{
+    switch (H) {
+        case 128: return launch_hadamard_quant<T, 7>(in, q, scales, total, s);
+        case 256: return launch_hadamard_quant<T, 8>(in, q, scales, total, s);
+        case 512: return launch_hadamard_quant<T, 9>(in, q, scales, total, s);
+        case 1024: return launch_hadamard_quant<T, 10>(in, q, scales, total, s);
+        case 2048: return launch_hadamard_quant<T, 11>(in, q, scales, total, s);
+        case 4096: return launch_hadamard_quant<T, 12>(in, q, scales, total, s);
+        default: return launch_hadamard_quant<T, 13>(in, q, scales, total, s);
+    }
 }
 
 extern "C" {
@@ -1075,12 +1091,8 @@ int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, f
     DeviceState* st;
     if (int rc = get_device_state(&st)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int KB = static_cast<int>(K / 128);
-    if (in_dtype == 0)
-        return launch_hadamard_quant(static_cast<const float*>(in), q, scales, M, static_cast<int>(K), KB,
-                                     static_cast<int>(had_block), s);
-    return launch_hadamard_quant(static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), KB,
-                                 static_cast<int>(had_block), s);
+    if (in_dtype == 0) return launch_hadamard_quant(static_cast<const float*>(in), q, scales, M * K, static_cast<int>(had_block), s);
+    return launch_hadamard_quant(static_cast<const __nv_bfloat16*>(in), q, scales, M * K, static_cast<int>(had_block), s);
 }
 
 int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream)
@@ -1094,11 +1106,9 @@ int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, i
     const int64_t cap = static_cast<int64_t>(st->sm_count) * 8;
     if (blocks > cap) blocks = cap;
     if (in_dtype == 0)
-        quantize_token_row_kernel<float><<<static_cast<int>(blocks), kQuantThreads, 0, s>>>(static_cast<const float*>(in), q,
-                                                                                         scales, M, static_cast<int>(K));
+        launch_quant_row(static_cast<const float*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
     else
-        quantize_token_row_kernel<__nv_bfloat16><<<static_cast<int>(blocks), kQuantThreads, 0, s>>>(
-            static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K));
+        launch_quant_row(static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
     GI8_CUDA(cudaGetLastError());
     return GI8_OK;
 }
