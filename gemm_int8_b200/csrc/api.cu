@@ -900,6 +900,7 @@ int gi8_matmul(const int8_t* x, const int8_t* y, void* out, int64_t M, int64_t N
     DenseParams p{};
     p.out = out, p.status = st->status, p.ldo = N, p.M = (int)M, p.N = (int)N, p.K = (int)K, p.alpha = alpha;
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
+    p.pair_ok = (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (N % 2 == 0);
     return dispatch_dense<EPI_ALPHA_BF16>(st, x, y, p, s);
 }
 
@@ -996,6 +997,7 @@ int gi8_matmul_scaled(const int8_t* x, const int8_t* y, const float* sx, const f
     p.out = out, p.sx = sx, p.sw = sw, p.status = st->status, p.ldo = N, p.M = (int)M, p.N = (int)N, p.K = (int)K;
     p.alpha = 1.0f;
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
+    p.pair_ok = (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (N % 2 == 0);
     return dispatch_dense<EPI_ROWCOL_BF16>(st, x, y, p, s);
 }
 
@@ -1144,6 +1146,7 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     p.out = out, p.sa = sa, p.sw = sw, p.status = st->status, p.ldo = N, p.ld_sa = ld_sa, p.ld_sw = ld_sw;
     p.M = (int)M, p.N = (int)N, p.K = (int)K;
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
+    p.pair_ok = (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (N % 2 == 0);
     p.out_f32 = out_f32 ? 1 : 0;
     p.n_out = 1, p.out_col0 = 0;
     p.scale_vec = (KB % 4 == 0) && (ld_sa % 4 == 0) && (ld_sw % 4 == 0) && reinterpret_cast<uintptr_t>(sa) % 16 == 0 &&

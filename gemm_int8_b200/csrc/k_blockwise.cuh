@@ -72,6 +72,7 @@ struct BlockwiseParams {
     int M, N, K;
     int tiles_m, tiles_n;
     int vec_ok;  // out is 16-byte aligned and ldo % 8 == 0
+    int pair_ok; // the same for 4 bytes and ldo % 2 == 0
     int group_m; // row-blocks per rasterisation band
     int tma_store;  // stage blocks of 32 rows in shared memory and write them with TMA stores
     int n_out;      // number of output matrices the TMA-store epilogue writes every block to (1, or the ranks of an
@@ -646,9 +647,10 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                         }
                     }
                 }
-            } else if (p.tma_store) {
+            } else if (!p.out_f32) {
                 // Blocks of 32 rows x STORE_W columns through swizzled shared memory and TMA stores (rows >= M and
-                // columns beyond the tensor map are clipped by the hardware).  The tile's coordinates are derived
+                // columns beyond the tensor map are clipped by the hardware), or, where TMA cannot address the rows of
+                // the output, row by row.  The tile's coordinates are derived
                 // again from an opaque copy of the tile index so that they do not occupy registers across the
                 // promotion loop.
                 int tile_again = tile, mb2, nb2;
@@ -662,7 +664,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                         // box b: segment b / (SEGW / STORE_W), box b % (SEGW / STORE_W) inside it
                         const int col0 = nb2 * BN + cg * kSegStrideCg + (b / (SEGW / STORE_W)) * kSegStrideH + (b % (SEGW / STORE_W)) * STORE_W;
                         if (col0 >= p.N) continue;  // warp-uniform
-                        if (lane == 0) tma_store_wait_read<0>();  // the previous block has been read out of the staging
+                        if (p.tma_store && lane == 0) tma_store_wait_read<0>();  // the previous block has been read out of the staging
                         __syncwarp();
                         // row = lane; 16-byte chunk q of the row goes to chunk q ^ (row % 8) (128-byte swizzle) or
                         // q ^ ((row / 2) % 4) (64-byte swizzle): conflict-free and what the tensor map expects.
@@ -674,6 +676,11 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                                          "r"(pack_bf16x2_of(acc[a0])), "r"(pack_bf16x2_of(acc[a0 + 1])),
                                          "r"(pack_bf16x2_of(acc[a0 + 2])), "r"(pack_bf16x2_of(acc[a0 + 3]))
                                          : "memory");
+                        }
+                        if (!p.tma_store) {
+                            __syncwarp();
+                            store_staged_rows<STORE_W>(stg, static_cast<uint16_t*>(p.out), p.ldo, row0, p.M, col0, p.N, p.pair_ok);
+                            continue;
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
@@ -689,7 +696,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                         }
                     }
                 }
-            } else if (p.out_f32) {
+            } else {
                 if (row_ok) {
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) {
@@ -709,28 +716,6 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                                 if (c0 + 2 * j < p.N) dst[2 * j] = lo;
                                 if (c0 + 2 * j + 1 < p.N) dst[2 * j + 1] = hi;
                             }
-                        }
-                    }
-                }
-            } else if (row_ok) {
-#pragma unroll
-                for (int h = 0; h < SPLIT; ++h) {
-                    const int c0 = col_base + h * kSegStrideH;
-                    if (c0 >= p.N) continue;
-                    uint16_t* dst = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(row) * p.ldo + c0;
-                    const uint64_t* a = acc + h * (SEGW / 2);
-                    if (c0 + SEGW <= p.N && p.vec_ok) {
-#pragma unroll
-                        for (int j = 0; j < SEGW / 2; j += 4)
-                            *reinterpret_cast<uint4*>(dst + 2 * j) = make_uint4(pack_bf16x2_of(a[j]), pack_bf16x2_of(a[j + 1]),
-                                                                                pack_bf16x2_of(a[j + 2]), pack_bf16x2_of(a[j + 3]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < SEGW / 2; ++j) {
-                            float lo, hi;
-                            unpack_f32x2(a[j], lo, hi);
-                            if (c0 + 2 * j < p.N) dst[2 * j] = to_bf16_bits(lo);
-                            if (c0 + 2 * j + 1 < p.N) dst[2 * j + 1] = to_bf16_bits(hi);
                         }
                     }
                 }

@@ -47,6 +47,7 @@ struct DenseParams {
     int M, N, K;
     int tiles_m, tiles_n;
     int vec_ok;           // out is 16-byte aligned and ldo keeps every row 16-byte aligned
+    int pair_ok;          // the same for 4 bytes (bf16 output)
     int group_m;          // row-blocks per rasterisation band
     int tma_store;        // bf16 epilogues: stage 32 x 32 blocks in shared memory and write them with TMA stores
     int tile_end;         // > 0: only tiles [0, tile_end) of the grid are computed here (the rest by the split-K launch)
@@ -94,6 +95,71 @@ GI8_DEVICE void tile_coords(int tile, int tiles_m, int tiles_n, int& mb, int& nb
     const int r = tile - g * per_group;
     mb = first_m + r % rows;
     nb = r / rows;
+}
+
+// Reads of staged blocks: volatile, so that they stay behind the barrier in front of them.
+GI8_DEVICE uint32_t ld_shared_u32(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+GI8_DEVICE uint16_t ld_shared_u16(uint32_t addr)
+{
+    uint16_t v;
+    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(addr));
+    return v;
+}
+
+// Writes a block of 32 rows x W bf16 columns (W = 32 or 64), staged in shared memory at `stg` as the TMA stores want it
+// (64- or 128-byte swizzle), to rows [row0, M) and columns [col0, N) of an output whose rows TMA cannot address (ldo not
+// a multiple of 8, or a base that is not 16-byte aligned).  Whole warp.  A warp writes one or two rows per instruction,
+// 64 or 128 consecutive bytes: a lane per row, as the accumulators lie in tensor memory, touches 32 sectors with every
+// 2-byte store (777 x 5003 x 3088, whose rows have odd length: 62.5 -> 24.5 us a call).  `pairs`: rows are 4-byte aligned, two columns per lane.
+template <int W>
+GI8_DEVICE void store_staged_rows(uint32_t stg, uint16_t* out, int64_t ldo, int row0, int M, int col0, int N, bool pairs)
+{
+    const int lane = threadIdx.x & 31;
+    const int rows = min(32, M - row0);
+    auto at = [&](int r, int c) {  // shared address of row r, column c
+        const int q = c >> 3;
+        const int cq = W == 64 ? (q ^ (r & 7)) : (q ^ ((r >> 1) & 3));
+        return stg + r * (W * 2) + cq * 16 + (c & 7) * 2;
+    };
+    // Eight rows' reads are issued before their stores, so that the shared-memory latency is paid once per eight.
+    if (pairs) {
+        constexpr int kRows = 64 / W;  // rows per instruction
+        const int c = (lane % (W / 2)) * 2;
+        const bool two = col0 + c + 1 < N, one = col0 + c < N;
+        for (int r0 = 0; r0 < rows; r0 += 8 * kRows) {
+            uint32_t v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = ld_shared_u32(at((r0 + i * kRows + lane / (W / 2)) & 31, c));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = r0 + i * kRows + lane / (W / 2);
+                uint16_t* dst = out + static_cast<int64_t>(row0 + r) * ldo + col0 + c;
+                if (r < rows) {
+                    if (two) *reinterpret_cast<uint32_t*>(dst) = v[i];
+                    else if (one) *dst = static_cast<uint16_t>(v[i]);
+                }
+            }
+        }
+    } else {
+        for (int r0 = 0; r0 < rows; r0 += 8) {
+#pragma unroll
+            for (int c0 = 0; c0 < W; c0 += 32) {
+                const int c = c0 + lane;
+                uint16_t v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = ld_shared_u16(at(r0 + i, c));
+                uint16_t* dst = out + static_cast<int64_t>(row0 + r0) * ldo + col0 + c;
+#pragma unroll
+                for (int i = 0; i < 8; ++i, dst += ldo)
+                    if (r0 + i < rows && col0 + c < N) *dst = v[i];
+            }
+        }
+    }
 }
 
 // PAIR: two CTAs on neighbouring SMs (a 2 x 1 x 1 cluster) share one 256 x BN tile.  The leader's MMA thread issues
@@ -329,43 +395,32 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                             f[j] = a * (row_scale * cs);
                         }
                     }
-                    if (p.tma_store) {
-                        // 32 rows x 32 bf16 of this warp go to shared memory in the 64-byte-swizzled layout the
-                        // output tensor map expects (16-byte chunk index xor (row / 2) % 4: conflict-free), then one
-                        // lane issues the TMA store; rows and columns beyond M and N are clipped by the hardware.
-                        const int row0 = mb * kTileM + static_cast<int>(rank) * kBM + quarter * 32;
-                        if (row0 < p.M) {
-                            uint8_t* stg = store_stage + ((warp - 2) * 2 + ((c >> 5) & 1)) * 2048;
-                            if (lane == 0) tma_store_wait_read<1>();  // the block staged two chunks ago has been read
-                            __syncwarp();
+                    // 32 rows x 32 bf16 of this warp go to shared memory in the 64-byte-swizzled layout the output tensor
+                    // map expects (16-byte chunk index xor (row / 2) % 4: conflict-free), then one lane issues the TMA
+                    // store (rows and columns beyond M and N are clipped by the hardware), or, where TMA cannot address
+                    // the rows, the warp writes them out row by row.
+                    const int row0 = mb * kTileM + static_cast<int>(rank) * kBM + quarter * 32;
+                    if (row0 >= p.M) continue;  // warp-uniform
+                    uint8_t* stg = store_stage + ((warp - 2) * 2 + ((c >> 5) & 1)) * 2048;
+                    if (p.tma_store && lane == 0) tma_store_wait_read<1>();  // the block staged two chunks ago has been read
+                    __syncwarp();
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const int cq = q ^ ((lane >> 1) & 3);
-                                *reinterpret_cast<uint4*>(stg + lane * 64 + cq * 16) = make_uint4(
-                                    pack_bf16x2(f[8 * q], f[8 * q + 1]), pack_bf16x2(f[8 * q + 2], f[8 * q + 3]),
-                                    pack_bf16x2(f[8 * q + 4], f[8 * q + 5]), pack_bf16x2(f[8 * q + 6], f[8 * q + 7]));
-                            }
-                            fence_proxy_async_smem();
-                            __syncwarp();
-                            if (lane == 0) {
-                                tma_store_2d(&map_out, stg, col0, row0);
-                                tma_store_commit();
-                            }
-                        }
-                        continue;
+                    for (int q = 0; q < 4; ++q) {
+                        const int cq = q ^ ((lane >> 1) & 3);
+                        *reinterpret_cast<uint4*>(stg + lane * 64 + cq * 16) = make_uint4(
+                            pack_bf16x2(f[8 * q], f[8 * q + 1]), pack_bf16x2(f[8 * q + 2], f[8 * q + 3]),
+                            pack_bf16x2(f[8 * q + 4], f[8 * q + 5]), pack_bf16x2(f[8 * q + 6], f[8 * q + 7]));
                     }
-                    if (!row_ok) continue;
-                    uint16_t* dst = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(row) * p.ldo + col0;
-                    if (col0 + 32 <= p.N && p.vec_ok) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 8)
-                            *reinterpret_cast<uint4*>(dst + j) =
-                                make_uint4(pack_bf16x2(f[j], f[j + 1]), pack_bf16x2(f[j + 2], f[j + 3]),
-                                           pack_bf16x2(f[j + 4], f[j + 5]), pack_bf16x2(f[j + 6], f[j + 7]));
+                    if (p.tma_store) {
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_2d(&map_out, stg, col0, row0);
+                            tma_store_commit();
+                        }
                     } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (col0 + j < p.N) dst[j] = to_bf16_bits(f[j]);
+                        __syncwarp();
+                        store_staged_rows<32>(smem_u32(stg), static_cast<uint16_t*>(p.out), p.ldo, row0, p.M, col0, p.N, p.pair_ok);
                     }
                 }
             }
