@@ -57,8 +57,7 @@ std::atomic<int> g_forced_variant{VAR_AUTO};
 //   GEMM_INT8_TMA_STORE  = 0       bf16 epilogues store from registers instead of through shared memory + TMA
 //   GEMM_INT8_PDL        = 0       no programmatic dependent launch anywhere (small-M kernels, second launches of a GEMM)
 //   GEMM_INT8_SPLITS     = n       small-M kernels: number of K splits
-//   GEMM_INT8_BW_HALVES  = 1 | 2   blockwise 256-wide tile: MMAs with N = 256, or two column halves with N = 128 (default:
-//                                  N = 256 for the one-CTA tile, column halves for the two-CTA tile)
+//   GEMM_INT8_BW_HALVES  = 1 | 2   blockwise 256-wide tile: MMAs with N = 256, or two column halves with N = 128 (default)
 //   GEMM_INT8_BW_ISSUERS = 1 | 2   blockwise kernel without column halves: MMA-issuing threads (default: one for the
 //                                  256-wide tile, two for the narrower ones, whose MMAs are issue bound)
 //   GEMM_INT8_TAIL_SPLIT = 0 | 1 | 2   never / when the cost model says so (default) / whenever possible hand the last wave
@@ -72,7 +71,7 @@ struct Knobs {
     bool tma_store = true;
     bool pdl = true;
     int splits = 0;
-    int bw_halves = 0;   // 0: column halves for the two-CTA tile, N = 256 MMAs for the one-CTA 256-wide tile
+    int bw_halves = 0;   // 0: column halves
     int bw_issuers = 0;  // 0: one for the 256-wide tile, two for the narrower ones
     // The caller promises that the weight operand of the small-M path is not written by the kernel that precedes the
     // call in its stream (weights quantised ahead of time): its first tiles are then requested before that kernel ends.
@@ -246,9 +245,9 @@ int check_common(const void* x, const void* y, const void* out, int64_t M, int64
 // form's cycles per K block, fitted on B200 from device-timed runs (8192^3, 2048 x 11008 x 4096, 128..512 x 8192 x
 // 8192 and the reference benchmark's layer shapes, timed back to back):
 //   dense      256 x 256 two-CTA tile (74 slots) 580 | 128 x 256: 655 | 128 x 128: 465 | 128 x 64: 330
-//   blockwise  128 x 256 (N = 256 MMAs, one issuer): 950 | 256 x 256 two-CTA tile (column halves): 920, but only
-//              ahead on long runs (16384 x 57344 x 8192: 8.72 against 9.00 ms; 16384 x 8192 x 28672: 4.63 against
-//              4.85 ms; level at 8192^3; behind below that), hence its minimum number of waves
+//   blockwise  128 x 256: 950 | 256 x 256 two-CTA tile: 920, but only ahead on long runs, hence its minimum number of waves
+//              (fitted when both converted their partials; without conversions both take 3 to 6 % less, level at 512 x
+//              8192 x 8192 and 8192^3, so the order stands)
 //              | 128 x 128: 650 | 128 x 64: 490
 // The table is data: kDenseForms / kBlockwiseForms below.  The narrow tiles cost more per column (the tensor-core instruction is issue
 // bound below N = 128, and the per-K-block hand-overs do not shrink with the tile) and only pay when the wide tile
@@ -1143,6 +1142,7 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     if (M * ld_sa >= (int64_t(1) << 31) || ((N + 127) / 128) * ld_sw >= (int64_t(1) << 31))
         return fail(GI8_ERR_INVALID_ARGUMENT, "scale arrays of 2^31 or more elements are not supported");
     BlockwiseParams p{};
+    p.x = x, p.y = y;
     p.out = out, p.sa = sa, p.sw = sw, p.status = st->status, p.ldo = N, p.ld_sa = ld_sa, p.ld_sw = ld_sw;
     p.M = (int)M, p.N = (int)N, p.K = (int)K;
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
@@ -1225,7 +1225,7 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
         GI8_CUDA(cudaLaunchKernelEx(&cfg, kernel, mx, my, mo, p));                            \
     } while (0)
     const bool two = knobs().bw_issuers == 2 || (knobs().bw_issuers == 0 && bn < 256);
-    const bool halves = knobs().bw_halves == 2 || (knobs().bw_halves == 0 && pair);
+    const bool halves = knobs().bw_halves != 1;
     if (pair) {
         if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, true, 21);
         else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, true, 22);

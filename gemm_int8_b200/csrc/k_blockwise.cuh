@@ -13,10 +13,22 @@
 //   warps 4..11 promotion (setmaxnreg.inc): warp w owns TMEM lane quarter (w % 4) and BN/2 of the tile's columns
 //               (with column halves: 64 columns of each half), i.e. 32 rows x BN/2 columns, whose fp32
 //               accumulators it keeps in registers (as f32x2 pairs).  Per K block and half: tcgen05.ld the int32
-//               partial in 32-column chunks, hand the half back after the last load, cvt.rn.f32.s32 +
-//               fma.rn.f32x2 with the block's scale.  A warp's segment never straddles a 128-wide weight-scale
-//               block.  At the end of the tile the same warps cast to bf16 and store through swizzled shared
-//               memory and TMA.
+//               partial in 32-column chunks, hand the half back after the last load, and accumulate it with the
+//               block's scale.  A warp's segment never straddles a 128-wide weight-scale block.  At the end of the
+//               tile the same warps cast to bf16 and store through swizzled shared memory and TMA.
+//
+// Two ways to accumulate, both one rounding per K block and element, the same bits:
+//   column halves (SPLIT == 2; both 256-wide forms as dispatched): no conversion.  A fifth MMA per K block, unsigned 255 x 255,
+//     adds kPartialBias to every partial, which makes it a positive 22-bit integer; its bits, read as a float, are a
+//     subnormal, and two fma.rn.f32x2 per pair of columns remove the bias exactly and accumulate (promote_pair_biased).
+//   SPLIT == 1 (narrow tiles): two cvt.rn.f32.s32 and one fma.rn.f32x2 per pair (promote_pair).
+// Conversions take the half-rate integer pipe two cycles each, and they, the multiply-adds and the tensor-memory loads of
+// a scheduler do not overlap as freely as their pipes would allow: with conversions alone or multiply-adds alone the
+// kernel ran at the speed of its MMAs, with both a third slower.  Measured, conversions -> bias (one MMA in four more included):
+// 2048 x 11008 x 4096 98.9 -> 96.1 us, 512 x 8192 x 8192 53.4 -> 51.0, 8192^3 615 -> 589, 2048 x 8192 x 28672 594 -> 568,
+// 16384 x 57344 x 8192 8.64 -> 8.16 ms (back to back, so the long ones under the power cap).  A fixed mixture (half of the
+// columns converted) was slower than either, and so was a branch for the scale products the trick does not cover inside
+// the K loop (15-20 %): they are looked for once per tile.
 //
 // Why eight fat warps (measured on B200 with a stand-alone loop of the same instructions, cycles per 128 x 256
 // K block, tensor core busy in the background): a tcgen05.ld costs about one cycle per 32-lane column whatever its
@@ -63,7 +75,14 @@ constexpr int kLaunchRegs = 168;  // registers per thread at launch: 65536 / 384
 // allocation); an unbalanced pair blocks in hardware for ever.
 static_assert(kPromoWarps * (kPromoRegs - kLaunchRegs) <= 4 * (kLaunchRegs - kControlRegs), "setmaxnreg pool unbalanced");
 
+// One MMA of K = 32 with both operands all 255 (unsigned) adds this to every partial it covers.  |P| of a 128-wide block
+// lies in [-128 * 127 * 128, 2^21], so P + kPartialBias lies in [32, 2^22).
+constexpr uint32_t kPartialBias = 32u * 255u * 255u;
+static_assert(kPartialBias > 128u * 127u * 128u && kPartialBias + (1u << 21) < (1u << 22), "biased partials must be positive 22-bit integers");
+
 struct BlockwiseParams {
+    const int8_t* x;  // [M, K]: the operands that the tensor maps describe, for the scale products that need them again
+    const int8_t* y;  // [N, K]
     void* out;        // bf16 [M,N], leading dimension ldo
     const float* sa;  // [M, KB], row stride ld_sa
     const float* sw;  // [ceil(N/128), KB], row stride ld_sw
@@ -137,6 +156,41 @@ GI8_DEVICE void promote_pair(uint64_t& acc, uint32_t& v0, uint32_t& v1, uint64_t
         : "l"(t2));
 }
 
+// The same for a partial that carries kPartialBias: read as the bits of a float, an integer v in [0, 2^23) is the subnormal
+// v * 2^-149, so one fma with 2^127 gives (v - kPartialBias) * 2^-22 = P * 2^-22 without rounding, and a second one, with
+// ts = t * 2^22, accumulates P * t with the single rounding that fma(fp32(P), t, acc) has -- for every t whose product with
+// 2^22 does not overflow, infinities, NaN and subnormals included.
+GI8_DEVICE void promote_pair_biased(uint64_t& acc, uint32_t v0, uint32_t v1, uint64_t c2, uint64_t b2, uint64_t ts2)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .b64 pv;\n\t"
+        "mov.b64 pv, {%1, %2};\n\t"
+        "fma.rn.f32x2 pv, pv, %3, %4;\n\t"
+        "fma.rn.f32x2 %0, pv, %5, %0;\n\t"
+        "}\n"
+        : "+l"(acc)
+        : "r"(v0), "r"(v1), "l"(c2), "l"(b2), "l"(ts2));
+}
+
+// One accumulator the slow way, for scale products that promote_pair_biased does not cover: the sum over K blocks of one
+// output element, from the operands in global memory (K a multiple of 16, rows 16-byte aligned).
+GI8_DEVICE float chain_from_global(const int8_t* x, const int8_t* y, const float* sa, const float* sw, int K)
+{
+    float acc = 0.0f;
+#pragma unroll 1
+    for (int k0 = 0, kb = 0; k0 < K; k0 += kBK, ++kb) {
+        int32_t P = 0;
+#pragma unroll 1
+        for (int k = k0; k < min(k0 + kBK, K); k += 16) {
+            const int4 a = __ldg(reinterpret_cast<const int4*>(x + k)), b = __ldg(reinterpret_cast<const int4*>(y + k));
+            P = __dp4a(a.w, b.w, __dp4a(a.z, b.z, __dp4a(a.y, b.y, __dp4a(a.x, b.x, P))));
+        }
+        acc = __fmaf_rn(__int2float_rn(P), __fmul_rn(__ldg(sa + kb), __ldg(sw + kb)), acc);
+    }
+    return acc;
+}
+
 GI8_DEVICE uint64_t splat_f32x2(float t)
 {
     uint64_t r;
@@ -199,8 +253,8 @@ GI8_DEVICE int rotate_tile(int tile, int rot, int n)
 // each half.  A half's partial buffer is then held for two loads and one chunk of arithmetic instead of four and
 // three, and the tensor core refills one half while the warps read the other: with only two 256-column buffers in
 // tensor memory the time a buffer is held, plus the latencies of the two hand-overs, is what bounds the K-block
-// period (measured: 1000-1200 cycles per K block with contiguous 128-column ownership, where neither instruction
-// issue (51 %) nor any pipe was saturated).
+// period.  Partials carry a bias and are accumulated without conversions; with NSUB = BN that loop spills (98 -> 124 us at
+// 2048 x 11008 x 4096), so that form converts.
 // SPLIT = 1: MMAs with N = BN; NISS issuing threads (1 or 2) take alternate K blocks.
 // PAIR: two CTAs on neighbouring SMs (a 2 x 1 x 1 cluster) share one 256 x BN tile, as in the dense kernel: the
 // leader's issuers run tcgen05.mma.cta_group::2 (M = 256), each CTA loads its own 128 rows of x and HALF of the BN
@@ -238,6 +292,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     // buffer that the same warp hands back after the awaited K block (see the protocol above).
     static_assert(STAGES >= NBUF, "the stage ring must be at least as deep as the partial-buffer ring");
     static_assert(!PAIR || BN == 256, "two-CTA tiles are 256 wide");
+    constexpr bool BIASED = SPLIT == 2;
     constexpr int kTileM = PAIR ? 2 * kBM : kBM;  // rows of the (pair's) tile
     constexpr int kRowsB = PAIR ? BN / 2 : BN;    // rows of y this CTA loads
     constexpr uint32_t kBytesA = kBM * kBK;
@@ -258,6 +313,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     __shared__ __align__(8) uint64_t bar_part_empty[SPLIT][NBUF];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile uint32_t abort_flag;
+    __shared__ __align__(128) uint32_t ones_tile[BIASED ? 256 : 1];  // bytes of 255: both operands of the bias MMA
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -281,6 +337,10 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         fence_barrier_init();
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_y);
+    }
+    if constexpr (BIASED) {
+        if (threadIdx.x < 256) ones_tile[threadIdx.x] = 0xffffffffu;
+        fence_proxy_async_smem();
     }
     if (warp == 2) {
         if constexpr (PAIR) {
@@ -367,6 +427,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             uint32_t s = first, ph = 0, buf = first, bph = 0;
             uint64_t* const done_h = &bar_done[h][0];
             uint64_t* const empty_h = &bar_part_empty[h][0];
+            [[maybe_unused]] const uint64_t d_ones = make_smem_desc_ones(smem_u32(ones_tile));
             for (uint32_t it = first; it < total; it += kStep) {
                 // The operands first (they land long before the partial buffer is free), so that nothing but the
                 // MMAs stands between the buffer hand-back and the tensor core.
@@ -389,6 +450,10 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     for (int k = 0; k < kBK / kUmmaK; ++k) {
                         if constexpr (PAIR) umma_i8_pair(tmem_d, da + 2 * k, db + 2 * k, kIdesc, k != 0 ? 1u : 0u);
                         else umma_i8(tmem_d, da + 2 * k, db + 2 * k, kIdesc, k != 0 ? 1u : 0u);
+                    }
+                    if constexpr (BIASED) {
+                        if constexpr (PAIR) umma_i8_pair(tmem_d, d_ones, d_ones, make_idesc_u8(kTileM, NSUB), 1u);
+                        else umma_i8(tmem_d, d_ones, d_ones, make_idesc_u8(kTileM, NSUB), 1u);
                     }
                     if constexpr (PAIR) {
                         umma_commit_pair(map_to_cta(smem_u32(&done_h[s]), 0));
@@ -432,6 +497,8 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         // lay under that arithmetic.  Otherwise the bounded wait runs; the branch is taken on a vote, which makes it
         // warp-uniform.
         bool polled = false;
+        [[maybe_unused]] const uint64_t unbias_c2 = splat_f32x2(0x1p127f);
+        [[maybe_unused]] const uint64_t unbias_b2 = splat_f32x2(-static_cast<float>(kPartialBias) * 0x1p-22f);
         // (so, sp): byte offset of the stage's barrier in its ring and the parity awaited there.
         auto wait_partial = [&](int h, uint32_t so, uint32_t sp) {
             if (!__all_sync(0xffffffffu, polled)) {
@@ -499,6 +566,9 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             }
             GI8_PIN(sa_off);
 
+            // Largest scale magnitudes met (NaN ignored): whether t * 2^22 can have overflowed is looked at once per tile.  The
+            // test per K block, three instructions on the pipe that has least room, had cost 6 %.
+            [[maybe_unused]] float max_sa = 0.0f, max_sw = 0.0f;
             uint64_t acc[CW / 2];  // fp32 accumulators as f32x2 pairs: segment h, columns (2j, 2j + 1) in acc[h * SEGW / 2 + j]
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j) acc[j] = 0ull;
@@ -524,7 +594,8 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                 for (int h = 0; h < SPLIT; ++h) {
                     if (!wait_partial(h, so, sp)) return false;
-                    const uint64_t t2 = splat_f32x2(t[h]);
+                    const float ts = BIASED ? t[h] * 0x1p22f : t[h];
+                    const uint64_t t2 = splat_f32x2(ts);
                     const uint32_t taddr = tm_warp + bc + h * NSUB;
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
@@ -536,7 +607,11 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                             poll_next(h, so, sp);
                         }
 #pragma unroll
-                        for (int q = 0; q < CHW / 2; ++q) promote_pair(acc[h * (SEGW / 2) + c * (CHW / 2) + q], v[2 * q], v[2 * q + 1], t2);
+                        for (int q = 0; q < CHW / 2; ++q) {
+                            uint64_t& a = acc[h * (SEGW / 2) + c * (CHW / 2) + q];
+                            if constexpr (BIASED) promote_pair_biased(a, v[2 * q], v[2 * q + 1], unbias_c2, unbias_b2, t2);
+                            else promote_pair(a, v[2 * q], v[2 * q + 1], t2);
+                        }
                     }
                 }
                 if constexpr (J < 0) next_k_block();
@@ -554,6 +629,11 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                 for (int h = 0; h < SPLIT; ++h) sw_c[h] = ldg4_in_place(p.sw + sw_off[h]);
                 for (int kb = 0; kb < num_kb && ok; kb += 4) {
+                    if constexpr (BIASED) {
+                        max_sa = max3_abs(sa_c.x, sa_c.y, max3_abs(sa_c.z, sa_c.w, max_sa));
+#pragma unroll
+                        for (int h = 0; h < SPLIT; ++h) max_sw = max3_abs(sw_c[h].x, sw_c[h].y, max3_abs(sw_c[h].z, sw_c[h].w, max_sw));
+                    }
                     float4 sa_n = sa_c, sw_n[SPLIT];
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) sw_n[h] = sw_c[h];
@@ -598,6 +678,11 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     float t[SPLIT];
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_q[j], sw_q[j][h]);
+                    if constexpr (BIASED) {
+                        max_sa = fmaxf(max_sa, fabsf(sa_q[j]));
+#pragma unroll
+                        for (int h = 0; h < SPLIT; ++h) max_sw = fmaxf(max_sw, fabsf(sw_q[j][h]));
+                    }
                     if (kb + 2 < num_kb) {
                         sa_q[j] = ldg_in_place(p.sa + (sa_off + kb + 2));
 #pragma unroll
@@ -611,6 +696,38 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 }
             }
             if (!ok) break;
+
+            if constexpr (BIASED) {
+                // Scale products t of 2^106 and more, whose t * 2^22 overflows: correct, not fast.  (Infinite ones are covered.)
+                bool huge = false;
+                if (max_sa * max_sw >= 0x1p106f) {
+#pragma unroll 1
+                    for (int kb = 0; kb < num_kb; ++kb) {
+#pragma unroll
+                        for (int h = 0; h < SPLIT; ++h) {
+                            const float t = fabsf(__fmul_rn(__ldg(p.sa + sa_off + kb), __ldg(p.sw + sw_off[h] + kb)));
+                            huge |= t >= 0x1p106f && t < INFINITY;
+                        }
+                    }
+                }
+                if (__any_sync(0xffffffffu, huge)) {
+#pragma unroll 1
+                    for (int c = 0; c < CW; ++c) {
+                        const int col = min(col_base + (c / SEGW) * kSegStrideH + c % SEGW, p.N - 1);
+                        const float r = chain_from_global(p.x + static_cast<int64_t>(row_ok ? row : 0) * p.K, p.y + static_cast<int64_t>(col) * p.K,
+                                                          p.sa + sa_off, p.sw + static_cast<int64_t>(col / 128) * p.ld_sw, p.K);
+#pragma unroll
+                        for (int j = 0; j < CW / 2; ++j) {
+                            float lo, hi;
+                            unpack_f32x2(acc[j], lo, hi);
+                            if (c == 2 * j) lo = r;
+                            if (c == 2 * j + 1) hi = r;
+                            asm("mov.b64 %0, {%1, %2};" : "=l"(acc[j]) : "f"(lo), "f"(hi));
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
 
             if (p.scatter_ranks > 0) {
                 // fp32 accumulators, 32 rows x 32 columns per box (128-byte rows, 128-byte swizzle: the same staging

@@ -72,20 +72,6 @@ GI8_DEVICE uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// max(|a|, |b|, |c|): ignoring NaN, and propagating it.
-GI8_DEVICE float max3_abs(float a, float b, float c)
-{
-    float r;
-    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-GI8_DEVICE float max3_abs_nan(float a, float b, float c)
-{
-    float r;
-    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-
 // Largest magnitude of N pairs (NaN ignored, as fmaxf does).
 template <int N>
 GI8_DEVICE float amax_pairs(const uint64_t* v)

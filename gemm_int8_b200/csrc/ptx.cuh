@@ -257,6 +257,25 @@ __host__ __device__ constexpr uint32_t make_idesc_i8(uint32_t m, uint32_t n, boo
     return (saturate ? (1u << 3) : 0u) | (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
+// The same with unsigned operands.
+__host__ __device__ constexpr uint32_t make_idesc_u8(uint32_t m, uint32_t n)
+{
+    return (2u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
+
+// Descriptor of a K-major operand, 32 bytes wide and up to 256 rows high, all of whose bytes are equal: no swizzle, core
+// matrices (8 rows x 16 bytes, 128 bytes in a row) that start 16 bytes apart in both directions and overlap, which is
+// harmless as they hold the same bytes.  Reads 16 + 31 * 16 + 128 = 640 bytes from smem_addr (16-byte aligned).
+GI8_DEVICE uint64_t make_smem_desc_ones(uint32_t smem_addr)
+{
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4);
+    d |= static_cast<uint64_t>(1) << 16;
+    d |= static_cast<uint64_t>(1) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    return d;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T.  Issued by ONE thread.  accumulate == 0 overwrites D.
 GI8_DEVICE void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
 {
@@ -321,6 +340,20 @@ GI8_DEVICE uint32_t pack_bf16x2(float lo, float hi)
     return r;
 }
 
+
+// max(|a|, |b|, |c|): ignoring NaN, and propagating it.
+GI8_DEVICE float max3_abs(float a, float b, float c)
+{
+    float r;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+GI8_DEVICE float max3_abs_nan(float a, float b, float c)
+{
+    float r;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 
 GI8_DEVICE uint16_t to_bf16_bits(float f)
 {
