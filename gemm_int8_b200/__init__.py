@@ -39,6 +39,7 @@ _libdef.define("int8_matmul_blockwise_f32(Tensor A, Tensor B, Tensor A_scale, Te
 _libdef.define("quantize_token_block(Tensor a) -> (Tensor, Tensor)")
 _libdef.define("quantize_token(Tensor a) -> (Tensor, Tensor)")
 _libdef.define("hadamard_quantize_token_block(Tensor a, int block) -> (Tensor, Tensor)")
+_libdef.define("int8_linear(Tensor x, Tensor weight_q, Tensor weight_scale, Tensor? bias, bool blockwise, int? hadamard) -> Tensor")
 
 
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
@@ -311,6 +312,52 @@ def _quantize(a: torch.Tensor, per_block: bool):
     return q, s
 
 
+def _int8_linear_cuda(x: torch.Tensor, w: torch.Tensor, w_scale: torch.Tensor, bias: torch.Tensor | None, blockwise: bool, hadamard: int | None):
+    """Quantiser and product with one call into the library, which launches the second as a programmatic dependent of
+    the first; the quantised activations live in one scratch tensor.  hadamard: rotation block, or None."""
+    name = "int8_linear"
+    if not x.is_cuda or x.dim() != 2 or x.dtype not in (torch.float32, torch.bfloat16):
+        raise RuntimeError(f"{name}: x must be a 2-D float32 or bfloat16 CUDA tensor")
+    if w.device != x.device or w.dtype != torch.int8 or w.dim() != 2 or not w.is_contiguous():
+        raise RuntimeError(f"{name}: the weight must be a contiguous 2-D int8 tensor on {x.device}")
+    if x.shape[1] != w.shape[1]:
+        raise RuntimeError(f"{name}: x has {x.shape[1]} features, the weight {w.shape[1]}")
+    if hadamard is not None and hadamard <= 0:
+        raise RuntimeError(f"{name}: rotation block {hadamard}")
+    (M, K), N = x.shape, w.shape[0]
+    KB, NB = -(-K // KBLOCK), -(-N // KBLOCK)
+    ld = 0
+    if blockwise:
+        _check_scale(name, "weight_scale", w_scale, (NB, KB), x.device)
+        if w_scale.stride(1) != 1 and KB > 1:
+            w_scale = w_scale.contiguous()
+        ld = w_scale.stride(0) if NB > 1 else KB
+        if ld < KB:
+            w_scale, ld = w_scale.contiguous(), KB
+    else:
+        w_scale = w_scale.reshape(-1) if w_scale.dim() == 2 and w_scale.shape[-1] == 1 else w_scale
+        _check_scale(name, "weight_scale", w_scale, (N,), x.device)
+        w_scale = w_scale.contiguous()
+    if bias is not None:
+        if bias.device != x.device or tuple(bias.shape) != (N,):
+            raise RuntimeError(f"{name}: bias must have shape [{N}] on {x.device}")
+        bias = bias.to(torch.bfloat16).contiguous()
+    x = x.contiguous()
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    q_bytes = -(-M * K // 256) * 256
+    scratch = torch.empty(q_bytes + 4 * M * (KB if blockwise else 1), dtype=torch.uint8, device=x.device)
+    with _on_device(x.device):
+        rc = _C.gi8_linear(_ptr(x), 0 if x.dtype == torch.float32 else 1, _ptr(w), _ptr(w_scale), ld, None if bias is None else _ptr(bias),
+                           int(blockwise), hadamard or 0, _ptr(scratch), ctypes.c_void_p(scratch.data_ptr() + q_bytes), _ptr(out), M, N, K,
+                           _stream_ptr(x.device))
+    if rc == 6 and not blockwise:  # GI8_ERR_WORKSPACE: a forced variant that the single call does not have
+        xq, xs = _quantize(x, False)
+        out = _int8_matmul_scaled_cuda(xq, w, xs, w_scale)
+        return out if bias is None else out + bias
+    _lib.check(_C, rc)
+    return out
+
+
 def _hadamard_quantize(a: torch.Tensor, block: int):
     if not a.is_cuda:
         raise RuntimeError("hadamard_quantize: input must be a CUDA tensor (the torch reference lives in gemm_int8_b200.quant)")
@@ -330,6 +377,7 @@ def _hadamard_quantize(a: torch.Tensor, block: int):
 
 
 _libdef.impl("hadamard_quantize_token_block", _hadamard_quantize, "CUDA")
+_libdef.impl("int8_linear", _int8_linear_cuda, "CUDA")
 _libdef.impl("quantize_token_block", lambda a: _quantize(a, True), "CUDA")
 _libdef.impl("quantize_token", lambda a: _quantize(a, False), "CUDA")
 
@@ -348,6 +396,14 @@ def _(a: torch.Tensor, block: int):
     kb = (a.shape[1] + KBLOCK - 1) // KBLOCK
     return (torch.empty(a.shape[0], a.shape[1], device=a.device, dtype=torch.int8),
             torch.empty(a.shape[0], kb, device=a.device, dtype=torch.float32))
+
+
+@torch.library.register_fake(f"{_NS}::int8_linear")
+def _(x: torch.Tensor, weight_q: torch.Tensor, weight_scale: torch.Tensor, bias: torch.Tensor | None, blockwise: bool, hadamard: int | None):
+    torch._check(len(x.shape) == 2 and len(weight_q.shape) == 2, lambda: "x and weight_q must be 2D tensors")
+    torch._check(weight_q.dtype == torch.int8, lambda: "weight_q must be an int8 tensor")
+    torch._check(x.shape[1] == weight_q.shape[1], lambda: "x.shape[1] must be equal to weight_q.shape[1]")
+    return torch.empty(x.shape[0], weight_q.shape[0], device=x.device, dtype=torch.bfloat16)
 
 
 @torch.library.register_fake(f"{_NS}::quantize_token")

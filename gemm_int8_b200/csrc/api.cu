@@ -354,6 +354,37 @@ int ensure_smem(DeviceState* st, int slot, Kernel kernel, size_t bytes)
     return GI8_OK;
 }
 
+// Launch on `stream`, as a cluster of (1, cluster_y, 1) or (cluster_x, 1, 1) CTAs, and with `pdl` as a programmatic dependent: the
+// kernel may then be started before the one in front of it in the stream has ended, and must itself wait for that one
+// (griddepcontrol.wait) before it touches anything that one writes or reads.
+template <typename Kernel, typename... Args>
+int launch(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, dim3 cluster, bool pdl, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (cluster.x * cluster.y > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster.x;
+        attr[n].val.clusterDim.y = cluster.y;
+        attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    GI8_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    return GI8_OK;
+}
+
 // Tensor map over the bf16 output [M, N] (row stride ldo elements) for the epilogue's TMA stores: boxes of 32 rows x
 // box_cols columns, 64-byte swizzle (32 columns) or 128-byte swizzle (64 columns).
 int make_output_map(CUtensorMap* map, void* out, int64_t M, int64_t N, int64_t ldo, int box_cols = 32)
@@ -385,9 +416,7 @@ int launch_dense(DeviceState* st, int slot, const int8_t* x, const int8_t* y, De
     p.group_m = pick_group_m(p.K);
     const int64_t tiles = p.tile_end > 0 ? p.tile_end : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
     const int grid = static_cast<int>(tiles < st->sm_count ? tiles : st->sm_count);
-    kernel<<<grid, kDenseThreads, smem, stream>>>(mx, my, mo, p);
-    GI8_CUDA(cudaGetLastError());
-    return GI8_OK;
+    return launch(kernel, dim3(grid), kDenseThreads, smem, stream, dim3(1), p.after_quant, mx, my, mo, p);
 }
 
 // Two-CTA form of the dense kernel: 256 x 256 tiles, one CTA pair (2 x 1 x 1 cluster) per tile.
@@ -413,20 +442,7 @@ int launch_dense_pair(DeviceState* st, int slot, const int8_t* x, const int8_t* 
     p.group_m = pick_group_m(p.K) / 2 > 0 ? pick_group_m(p.K) / 2 : 1;
     const int64_t tiles = p.tile_end > 0 ? p.tile_end : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
     const int pairs = static_cast<int>(tiles < st->sm_count / 2 ? tiles : st->sm_count / 2);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(2 * pairs, 1, 1);
-    cfg.blockDim = dim3(kDenseThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    GI8_CUDA(cudaLaunchKernelEx(&cfg, kernel, mx, my, mo, p));
-    return GI8_OK;
+    return launch(kernel, dim3(2 * pairs), kDenseThreads, smem, stream, dim3(2), p.after_quant, mx, my, mo, p);
 }
 
 // Split-K launch for tiles [tile_begin, tile_begin + units / halves) of the grid described by p (tiles_m, tiles_n,
@@ -441,22 +457,7 @@ int launch_dense_splitk(DeviceState* st, int slot, const int8_t* x, const int8_t
     CUtensorMap mx, my;
     if (int rc = make_operand_map(&mx, x, p.M, p.K, kBM)) return rc;
     if (int rc = make_operand_map(&my, y, p.N, p.K, kSplitKBN)) return rc;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(q.units * q.splits, 1, 1);
-    cfg.blockDim = dim3(kDenseThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = q.splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = q.after_main ? 2 : 1;
-    GI8_CUDA(cudaLaunchKernelEx(&cfg, kernel, mx, my, p, q));
-    return GI8_OK;
+    return launch(kernel, dim3(q.units * q.splits), kDenseThreads, smem, stream, dim3(q.splits), q.after_main || p.after_quant, mx, my, p, q);
 }
 
 // The last wave of a persistent grid costs as much as a full one however few tiles it holds.  When it is thin -- or
@@ -567,6 +568,7 @@ int dispatch_dense(DeviceState* st, const int8_t* x, const int8_t* y, DenseParam
             pt.tiles_m = static_cast<int>((p.M + (pair ? 2 * kBM : kBM) - 1) / (pair ? 2 * kBM : kBM));
             pt.tiles_n = static_cast<int>((p.N + 255) / 256);
             pt.group_m = pair ? (pick_group_m(p.K) / 2 > 0 ? pick_group_m(p.K) / 2 : 1) : pick_group_m(p.K);
+            if (t.tile_end > 0) pt.after_quant = 0;  // the main launch waits before it releases the split-K launch
             if (t.tile_end > 0) {
                 if (int rc = pair ? launch_dense_pair<EPI>(st, 45 + EPI, x, y, pm, stream)
                                   : launch_dense<256, 4, EPI>(st, EPI * 3 + 0, x, y, pm, stream))
@@ -667,24 +669,9 @@ int launch_smallm_cluster(DeviceState* st, int slot, const int8_t* x, const int8
     CUtensorMap mw, mx;
     if (int rc = make_operand_map(&mw, w, p.N, p.K, kSmallMTileN)) return rc;
     if (int rc = make_operand_map(&mx, x, p.M, p.K, MT)) return rc;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(pl.tiles_n, pl.splits, 1);
-    cfg.blockDim = dim3(kSmallMThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = pl.splits;
-    attr[0].val.clusterDim.z = 1;
     // Programmatic dependent launch: this kernel's set-up overlaps the tail of the previous kernel in the stream
     // (it waits with griddepcontrol.wait before its first global access).
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = knobs().pdl ? 2 : 1;
-    GI8_CUDA(cudaLaunchKernelEx(&cfg, kernel, mw, mx, p));
-    return GI8_OK;
+    return launch(kernel, dim3(pl.tiles_n, pl.splits), kSmallMThreads, smem, stream, dim3(1, pl.splits), knobs().pdl, mw, mx, p);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -765,12 +752,11 @@ __global__ void sum_parts_bf16_kernel(const float* __restrict__ parts, int n_par
 }
 
 template <typename T>
-static void launch_quant_row(const T* in, int8_t* q, float* scales, int64_t M, int K, int blocks, cudaStream_t s)
+static int launch_quant_row(const T* in, int8_t* q, float* scales, int64_t M, int K, int blocks, cudaStream_t s)
 {
     const int64_t loads = (static_cast<int64_t>(K) * sizeof(T) + kQuantThreads * 16 - 1) / (kQuantThreads * 16);
-    if (loads <= 2) quantize_token_row_kernel<T, 2><<<blocks, kQuantThreads, 0, s>>>(in, q, scales, M, K);
-    else if (loads <= 4) quantize_token_row_kernel<T, 4><<<blocks, kQuantThreads, 0, s>>>(in, q, scales, M, K);
-    else quantize_token_row_kernel<T, 8><<<blocks, kQuantThreads, 0, s>>>(in, q, scales, M, K);
+    auto kernel = loads <= 2 ? quantize_token_row_kernel<T, 2> : loads <= 4 ? quantize_token_row_kernel<T, 4> : quantize_token_row_kernel<T, 8>;
+    return launch(kernel, dim3(blocks), kQuantThreads, 0, s, dim3(1), knobs().pdl, in, q, scales, M, K);
 }
 
 template <typename T, int LOGH>
@@ -781,9 +767,8 @@ static int launch_hadamard_quant(const T* in, int8_t* q, float* scales, int64_t 
     const int64_t per_cta = static_cast<int64_t>(S::UNITS) << S::LOGU;
     const int64_t blocks = (total + per_cta - 1) / per_cta;
     if (blocks > INT32_MAX) return fail(GI8_ERR_UNSUPPORTED_SHAPE, "too many rotation blocks");
-    hadamard_quantize_token_block_kernel<T, LOGH><<<static_cast<int>(blocks), S::THREADS * S::UNITS, 0, s>>>(in, q, scales, total, norm);
-    GI8_CUDA(cudaGetLastError());
-    return GI8_OK;
+    return launch(hadamard_quantize_token_block_kernel<T, LOGH>, dim3(static_cast<int>(blocks)), S::THREADS * S::UNITS, 0, s, dim3(1),
+                  knobs().pdl, in, q, scales, total, norm);
 }
 
 template <typename T>
@@ -929,8 +914,10 @@ int64_t gi8_matmul_scaled_workspace_bytes(int64_t M, int64_t N, int64_t K)
     return pl.use ? pl.total_bytes : 0;
 }
 
-int gi8_matmul_scaled(const int8_t* x, const int8_t* y, const float* sx, const float* sw, void* out, int64_t M,
-                      int64_t N, int64_t K, void* workspace, int64_t workspace_bytes, void* stream)
+// bias: bf16 [N] or null.  after_quant: the launch directly in front of this one in the stream is the quantiser that writes
+// x and sx (it has waited for everything before it, the weights' writers included, before it lets a dependent start).
+static int scaled_impl(const int8_t* x, const int8_t* y, const float* sx, const float* sw, void* out, int64_t M, int64_t N, int64_t K,
+                       void* workspace, int64_t workspace_bytes, void* stream, const uint16_t* bias, bool after_quant)
 {
     if (int rc = check_common(x, y, out, M, N, K, 2)) return rc;
     if (M == 0 || N == 0) return GI8_OK;
@@ -948,7 +935,8 @@ int gi8_matmul_scaled(const int8_t* x, const int8_t* y, const float* sx, const f
             SmallMParams q{};
             q.out = out, q.sx = sx, q.sw = sw, q.status = st->status, q.ldo = N;
             q.M = (int)M, q.N = (int)N, q.K = (int)K, q.kb_per_split = pl.kb_per_split, q.splits = pl.splits;
-            q.static_w = knobs().static_weights && knobs().pdl;
+            q.static_w = (knobs().static_weights || after_quant) && knobs().pdl;
+            q.bias = bias;
             // Pipeline depth: two CTAs share an SM (about 100 KB each, the receive area of a cluster CTA included).  A
             // deeper pipeline with one CTA per SM measured slower even for grids of at most one CTA per SM: the next
             // kernel's CTAs could no longer move in beside the running ones, and its set-up no longer overlapped.
@@ -970,6 +958,7 @@ int gi8_matmul_scaled(const int8_t* x, const int8_t* y, const float* sx, const f
         }
     }
     if (forced == VAR_SMALLM) {
+        if (bias) return fail(GI8_ERR_WORKSPACE, "the scratch variant has no bias");
         const SmallMPlan pl = plan_smallm(M, N, K, st->sm_count, true);
         if (pl.use) {
             SmallMParams q{};
@@ -997,7 +986,15 @@ int gi8_matmul_scaled(const int8_t* x, const int8_t* y, const float* sx, const f
     p.alpha = 1.0f;
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
     p.pair_ok = (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (N % 2 == 0);
+    p.bias = bias, p.bias_vec = reinterpret_cast<uintptr_t>(bias) % 16 == 0;
+    p.after_quant = after_quant && knobs().pdl;
     return dispatch_dense<EPI_ROWCOL_BF16>(st, x, y, p, s);
+}
+
+int gi8_matmul_scaled(const int8_t* x, const int8_t* y, const float* sx, const float* sw, void* out, int64_t M,
+                      int64_t N, int64_t K, void* workspace, int64_t workspace_bytes, void* stream)
+{
+    return scaled_impl(x, y, sx, sw, out, M, N, K, workspace, workspace_bytes, stream, nullptr, false);
 }
 
 int gi8_matmul_scaled_static(const int8_t* x, const int8_t* y, const float* sx, const float* sw, void* out, int64_t M,
@@ -1070,13 +1067,10 @@ int gi8_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* sca
     const int64_t cap = static_cast<int64_t>(st->sm_count) * 16;
     if (blocks > cap) blocks = cap;
     if (in_dtype == 0)
-        quantize_token_block_kernel<float><<<static_cast<int>(blocks), kQuantThreads, 0, s>>>(
-            static_cast<const float*>(in), q, scales, M, static_cast<int>(K), KB);
-    else
-        quantize_token_block_kernel<__nv_bfloat16><<<static_cast<int>(blocks), kQuantThreads, 0, s>>>(
-            static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), KB);
-    GI8_CUDA(cudaGetLastError());
-    return GI8_OK;
+        return launch(quantize_token_block_kernel<float>, dim3(static_cast<int>(blocks)), kQuantThreads, 0, s, dim3(1), knobs().pdl,
+                      static_cast<const float*>(in), q, scales, M, static_cast<int>(K), KB);
+    return launch(quantize_token_block_kernel<__nv_bfloat16>, dim3(static_cast<int>(blocks)), kQuantThreads, 0, s, dim3(1), knobs().pdl,
+                  static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), KB);
 }
 
 int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K,
@@ -1106,12 +1100,8 @@ int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, i
     int64_t blocks = M;
     const int64_t cap = static_cast<int64_t>(st->sm_count) * 8;
     if (blocks > cap) blocks = cap;
-    if (in_dtype == 0)
-        launch_quant_row(static_cast<const float*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
-    else
-        launch_quant_row(static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
-    GI8_CUDA(cudaGetLastError());
-    return GI8_OK;
+    if (in_dtype == 0) return launch_quant_row(static_cast<const float*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
+    return launch_quant_row(static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
 }
 
 // gather != nullptr: the N-sharded form.  This GEMM's [M,N] result is columns [col0, col0 + N) of an [M, n_total]
@@ -1120,7 +1110,7 @@ int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, i
 static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw, int64_t ld_sw,
                           void* out, int64_t M, int64_t N, int64_t K, void* stream, void* const* gather, int n_out,
                           int64_t n_total, int64_t col0, bool out_f32 = false, int force_bn = 0, int pdl_role = 0,
-                          int scatter_me = -1)
+                          int scatter_me = -1, const uint16_t* bias = nullptr, bool after_quant = false)
 {
     // scatter_me >= 0: `gather` holds the n_out ranks' receive areas of the K-sharded reduce-scatter form
     const bool scatter = scatter_me >= 0;
@@ -1149,6 +1139,8 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     p.pair_ok = (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (N % 2 == 0);
     p.out_f32 = out_f32 ? 1 : 0;
     p.n_out = 1, p.out_col0 = 0;
+    p.bias = bias, p.bias_vec = reinterpret_cast<uintptr_t>(bias) % 16 == 0;
+    p.after_quant = after_quant && knobs().pdl;
     p.scale_vec = (KB % 4 == 0) && (ld_sa % 4 == 0) && (ld_sw % 4 == 0) && reinterpret_cast<uintptr_t>(sa) % 16 == 0 &&
                   reinterpret_cast<uintptr_t>(sw) % 16 == 0;
     const int forced = g_forced_variant;
@@ -1203,50 +1195,42 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
         if (p.tma_store)
             if (int rc = make_output_map(&mo.m[0], out, M, N, N, box_cols)) return rc;
     }
-#define GI8_LAUNCH_BW(BN_, ST_, SPLIT_, NISS_, PAIR_, SLOT_)                                  \
+#define GI8_LAUNCH_BW(BN_, ST_, SPLIT_, NISS_, PAIR_, BIAS_, SLOT_)                           \
     do {                                                                                      \
         constexpr size_t smem = blockwise_smem_bytes(BN_, ST_, PAIR_);                        \
-        auto kernel = blockwise_gemm_kernel<BN_, ST_, SPLIT_, NISS_, PAIR_>;                  \
+        auto kernel = blockwise_gemm_kernel<BN_, ST_, SPLIT_, NISS_, PAIR_, BIAS_>;           \
         if (int rc = ensure_smem(st, SLOT_, kernel, smem)) return rc;                         \
-        cudaLaunchConfig_t cfg{};                                                             \
-        cfg.gridDim = dim3(grid, 1, 1);                                                       \
-        cfg.blockDim = dim3(kBlockwiseThreads, 1, 1);                                         \
-        cfg.dynamicSmemBytes = smem;                                                          \
-        cfg.stream = s;                                                                       \
-        cudaLaunchAttribute attr[2];                                                          \
-        attr[0].id = cudaLaunchAttributeClusterDimension;                                     \
-        attr[0].val.clusterDim.x = PAIR_ ? 2 : 1;                                             \
-        attr[0].val.clusterDim.y = 1;                                                         \
-        attr[0].val.clusterDim.z = 1;                                                         \
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;                      \
-        attr[1].val.programmaticStreamSerializationAllowed = 1;                               \
-        cfg.attrs = attr;                                                                     \
-        cfg.numAttrs = pdl_role == 2 ? 2 : 1;                                                 \
-        GI8_CUDA(cudaLaunchKernelEx(&cfg, kernel, mx, my, mo, p));                            \
+        return launch(kernel, dim3(grid), kBlockwiseThreads, smem, s, dim3(PAIR_ ? 2 : 1), pdl_role == 2 || p.after_quant, mx, my, mo, p); \
     } while (0)
     const bool two = knobs().bw_issuers == 2 || (knobs().bw_issuers == 0 && bn < 256);
     const bool halves = knobs().bw_halves != 1;
+    if (bias) {  // (the knobs below choose among forms without one)
+        if (pair) GI8_LAUNCH_BW(256, 4, 2, 2, true, true, 28);
+        if (bn == 256) GI8_LAUNCH_BW(256, 4, 2, 2, false, true, 29);
+        if (bn == 128) GI8_LAUNCH_BW(128, 6, 1, 2, false, true, 30);
+        GI8_LAUNCH_BW(64, 8, 1, 2, false, true, 31);
+    }
     if (pair) {
-        if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, true, 21);
-        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, true, 22);
-        else GI8_LAUNCH_BW(256, 4, 1, 1, true, 23);
+        if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, true, false, 21);
+        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, true, false, 22);
+        else GI8_LAUNCH_BW(256, 4, 1, 1, true, false, 23);
     } else if (bn == 256) {
-        if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, false, 13);
-        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, false, 15);
-        else GI8_LAUNCH_BW(256, 4, 1, 1, false, 16);
+        if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, false, false, 13);
+        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, false, false, 15);
+        else GI8_LAUNCH_BW(256, 4, 1, 1, false, false, 16);
     } else if (bn == 128) {
-        if (two) GI8_LAUNCH_BW(128, 6, 1, 2, false, 17);
-        else GI8_LAUNCH_BW(128, 6, 1, 1, false, 18);
+        if (two) GI8_LAUNCH_BW(128, 6, 1, 2, false, false, 17);
+        else GI8_LAUNCH_BW(128, 6, 1, 1, false, false, 18);
     } else {
-        if (two) GI8_LAUNCH_BW(64, 8, 1, 2, false, 19);
-        else GI8_LAUNCH_BW(64, 8, 1, 1, false, 20);
+        if (two) GI8_LAUNCH_BW(64, 8, 1, 2, false, false, 19);
+        else GI8_LAUNCH_BW(64, 8, 1, 1, false, false, 20);
     }
 #undef GI8_LAUNCH_BW
-    return GI8_OK;
 }
 
-int gi8_matmul_blockwise(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw,
-                         int64_t ld_sw, void* out, int64_t M, int64_t N, int64_t K, void* stream)
+// (bias, after_quant: see scaled_impl)
+static int blockwise_dispatch(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw, int64_t ld_sw, void* out,
+                              int64_t M, int64_t N, int64_t K, void* stream, const uint16_t* bias, bool after_quant)
 {
     if (g_forced_variant == VAR_AUTO && M > 0 && N > 0 && K > 0 && out && reinterpret_cast<uintptr_t>(out) % 16 == 0 && N % 8 == 0) {
         DeviceState* st;
@@ -1258,14 +1242,43 @@ int gi8_matmul_blockwise(const int8_t* x, const int8_t* y, const float* sa, int6
                 // both launches write through a tensor map of the whole [M, N] matrix, each its own columns
                 void* outs[1] = {out};
                 const bool pdl = knobs().pdl;  // GEMM_INT8_PDL=0: two ordinary launches, one after the other
-                if (int rc = blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, nullptr, M, c.n1, K, stream, outs, 1, N, 0, false, 256, pdl ? 1 : 0))
+                if (int rc = blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, nullptr, M, c.n1, K, stream, outs, 1, N, 0, false, 256, pdl ? 1 : 0, -1, bias, after_quant))
                     return rc;
                 return blockwise_impl(x, y + c.n1 * K, sa, ld_sa, sw ? sw + (c.n1 / 128) * ld_sw : sw, ld_sw, nullptr, M, N - c.n1, K,
-                                      stream, outs, 1, N, c.n1, false, c.bn_tail, pdl ? 2 : 0);
+                                      stream, outs, 1, N, c.n1, false, c.bn_tail, pdl ? 2 : 0, -1, bias ? bias + c.n1 : nullptr, false);
             }
         }
     }
-    return blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, out, M, N, K, stream, nullptr, 1, N, 0);
+    return blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, out, M, N, K, stream, nullptr, 1, N, 0, false, 0, 0, -1, bias, after_quant);
+}
+
+int gi8_matmul_blockwise(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw,
+                         int64_t ld_sw, void* out, int64_t M, int64_t N, int64_t K, void* stream)
+{
+    return blockwise_dispatch(x, y, sa, ld_sa, sw, ld_sw, out, M, N, K, stream, nullptr, false);
+}
+
+int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale, int64_t ld_sw, const void* bias, int blockwise,
+               int64_t had_block, int8_t* xq, float* xs, void* out, int64_t M, int64_t N, int64_t K, void* stream)
+{
+    // Everything that the GEMM refuses is refused before the quantiser is launched.
+    if (int rc = check_common(xq, w, out, M, N, K, 2)) return rc;
+    if (int rc = check_quant(x, x_dtype, xq, xs, M, K)) return rc;
+    if (had_block && !blockwise) return fail(GI8_ERR_INVALID_ARGUMENT, "a rotation needs block scales");
+    if (reinterpret_cast<uintptr_t>(bias) % 2) return fail(GI8_ERR_MISALIGNED, "bias must be 2-byte aligned");
+    if (M == 0 || N == 0) return GI8_OK;
+    if (K == 0 && bias) return fail(GI8_ERR_UNSUPPORTED_SHAPE, "K must be positive for a product with a bias");
+    if (!blockwise && g_forced_variant == VAR_SMALLM)
+        return fail(GI8_ERR_WORKSPACE, "the scratch variant needs a workspace; call the quantiser and gi8_matmul_scaled");
+    const uint16_t* b = static_cast<const uint16_t*>(bias);
+    if (!blockwise) {
+        if (int rc = gi8_quantize_token(x, x_dtype, xq, xs, M, K, stream)) return rc;
+        return scaled_impl(xq, w, xs, w_scale, out, M, N, K, nullptr, 0, stream, b, K > 0);
+    }
+    if (int rc = had_block ? gi8_hadamard_quantize_token_block(x, x_dtype, xq, xs, M, K, had_block, stream)
+                           : gi8_quantize_token_block(x, x_dtype, xq, xs, M, K, stream))
+        return rc;
+    return blockwise_dispatch(xq, w, xs, (K + 127) / 128, w_scale, ld_sw, out, M, N, K, stream, b, K > 0);
 }
 
 int gi8_matmul_blockwise_f32(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw,

@@ -107,6 +107,9 @@ struct BlockwiseParams {
     int scatter_me;     // memory for j != me) at row block scatter_me, as 32 x 32 fp32 TMA-store boxes; R % 32 == 0
     int tile_rot;       // the tile sequence starts at this tile (and wraps): in the scattering form rank r starts with its
                         // own rows, so that at any moment the ranks send to different owners instead of all to the same
+    const uint16_t* bias;  // bf16 [N] added to the rounded result (BIAS kernels)
+    int bias_vec;   // bias is 16-byte aligned
+    int after_quant;  // launched as the programmatic dependent of the quantiser that writes x and sa (and of nothing else)
     int out_f32;    // store the fp32 accumulators themselves (out is float [M,N]) instead of their bf16 cast; the
                     // partial results of a K-sharded GEMM, and the bit-exact check of the accumulation order
 };
@@ -268,7 +271,9 @@ GI8_DEVICE int rotate_tile(int tile, int rot, int n)
 // An N = 128 two-CTA MMA (column halves) takes 64 rows of y from each CTA, so half h of the partial holds tile
 // columns [64 h, 64 h + 64) and [128 + 64 h, 128 + 64 h + 64): a promotion warp's 64-column segment of half h is then
 // tile columns cg * 128 + h * 64 .. (still contiguous and inside one weight-scale block).
-template <int BN, int STAGES, int SPLIT, int NISS, bool PAIR = false>
+// BIAS: a bf16 vector is added to the rounded result.  A template parameter, not a branch: with the branch in the epilogue
+// the K loop of the 256-wide forms was compiled 6 % slower (2048 x 11008 x 4096: 97 -> 103 us).
+template <int BN, int STAGES, int SPLIT, int NISS, bool PAIR = false, bool BIAS = false>
 __global__ void __launch_bounds__(kBlockwiseThreads, 1)
 blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                       const __grid_constant__ OutputMaps outs, const BlockwiseParams p)
@@ -325,7 +330,6 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (threadIdx.x == 0) {
-        if (p.pdl_role == 1) pdl_launch_dependents();
         abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&bar_full[s], 1);
@@ -356,6 +360,13 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers exist before anything signals them remotely
     tcgen05_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    // A programmatic dependent waits here for the kernel that writes x and sa; without one in front this returns at once.
+    // (The second of two launches has nothing to wait for, see pdl_role.)  Behind a quantiser the producer warp of the narrow
+    // tiles, which decode uses, requests its first weights before it waits.
+    const bool early_weights = BN < 256 && p.after_quant;
+    if (BN == 256 || (p.pdl_role != 2 && !(early_weights && warp == 0))) pdl_wait();
+    // (after that wait: the launch behind this one does not wait for anything before it reads x)
+    if (p.pdl_role == 1 && threadIdx.x == 0) pdl_launch_dependents();
 
     if (warp < 4) {
         setmaxnreg_dec<kControlRegs>();
@@ -370,10 +381,34 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             uint32_t s = 0, ph = 0;  // stage and phase parity of the running K-block counter
             uint32_t armed = 0;
             bool ok = true;
+            int kb_early = 0;  // K blocks of the first tile that are under way before the loop
+            if constexpr (BN < 256) {
+                if (early_weights) {
+                    // (tiles there are as many as CTAs at least, and all stages are free)
+                    int mb, nb;
+                    tile_coords(rotate_tile(first_tile, p.tile_rot, num_tiles), p.tiles_m, p.tiles_n, mb, nb, p.group_m);
+                    kb_early = min(num_kb, STAGES);
+                    if (elect_one()) {
+                        for (int kb = 0; kb < kb_early; ++kb) {
+                            mbar_arrive_expect_tx(&bar_full[kb], kStageBytes);
+                            tma_load_2d(smem + kb * kStageBytes + kBytesA, &map_y, &bar_full[kb], kb * kBK, nb * BN);
+                        }
+                    }
+                    __syncwarp();
+                    pdl_wait();
+                    if (elect_one()) {
+                        for (int kb = 0; kb < kb_early; ++kb) tma_load_2d(smem + kb * kStageBytes, &map_x, &bar_full[kb], kb * kBK, mb * kBM);
+                    }
+                    __syncwarp();
+                    armed = static_cast<uint32_t>(kb_early);
+                    s = armed;
+                    if (s == STAGES) s = 0, ph ^= 1;
+                }
+            }
             for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
                 int mb, nb;
                 tile_coords(rotate_tile(tile, p.tile_rot, num_tiles), p.tiles_m, p.tiles_n, mb, nb, p.group_m);
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = tile == first_tile ? kb_early : 0; kb < num_kb; ++kb) {
                     bool freed = wait_or_abort(&bar_done[0][s], ph ^ 1, &abort_flag);
                     if (SPLIT == 2 && freed) freed = wait_or_abort(&bar_done[SPLIT - 1][s], ph ^ 1, &abort_flag);
                     if (!freed) {
@@ -789,9 +824,14 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                         for (int q = 0; q < STORE_W / 8; ++q) {
                             const int cq = STORE_W == 64 ? (q ^ (lane & 7)) : (q ^ ((lane >> 1) & 3));
                             const int a0 = b * (STORE_W / 2) + 4 * q;
+                            uint4 w = make_uint4(pack_bf16x2_of(acc[a0]), pack_bf16x2_of(acc[a0 + 1]), pack_bf16x2_of(acc[a0 + 2]),
+                                                 pack_bf16x2_of(acc[a0 + 3]));
+                            if constexpr (BIAS) {
+                                const uint4 bv = load_bias8(p.bias, col0 + 8 * q, p.N, p.bias_vec);
+                                w = make_uint4(add_bf16x2(w.x, bv.x), add_bf16x2(w.y, bv.y), add_bf16x2(w.z, bv.z), add_bf16x2(w.w, bv.w));
+                            }
                             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * (STORE_W * 2) + cq * 16),
-                                         "r"(pack_bf16x2_of(acc[a0])), "r"(pack_bf16x2_of(acc[a0 + 1])),
-                                         "r"(pack_bf16x2_of(acc[a0 + 2])), "r"(pack_bf16x2_of(acc[a0 + 3]))
+                                         "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w)
                                          : "memory");
                         }
                         if (!p.tma_store) {

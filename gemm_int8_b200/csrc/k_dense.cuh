@@ -53,6 +53,9 @@ struct DenseParams {
     int tile_end;         // > 0: only tiles [0, tile_end) of the grid are computed here (the rest by the split-K launch)
     int pdl_role;         // 1: an independent launch over other output tiles follows: let it start as SMs free up
     float alpha;
+    const uint16_t* bias; // bf16 [N] added to the rounded result, or null (EPI_ROWCOL_BF16)
+    int bias_vec;         // bias is 16-byte aligned
+    int after_quant;      // launched as the programmatic dependent of the kernel that writes x and sx: wait for it first
 };
 
 // Records the first error of the grid and raises the CTA-wide abort flag.
@@ -206,7 +209,6 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (threadIdx.x == 0) {
-        if (p.pdl_role == 1) pdl_launch_dependents();
         abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&bar_full[s], 1);
@@ -235,6 +237,9 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers exist before anything signals them remotely
     tcgen05_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    if (p.after_quant) pdl_wait();
+    // (after that wait: the launch behind this one does not wait for anything before it reads x)
+    if (p.pdl_role == 1 && threadIdx.x == 0) pdl_launch_dependents();
 
     // The producer and the MMA issuer run their loops with the WHOLE warp (uniform control flow) and elect one lane
     // only around the TMA / MMA / commit instructions.  Inside an `if (lane == 0)` region the compiler treats
@@ -407,9 +412,15 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int cq = q ^ ((lane >> 1) & 3);
-                        *reinterpret_cast<uint4*>(stg + lane * 64 + cq * 16) = make_uint4(
-                            pack_bf16x2(f[8 * q], f[8 * q + 1]), pack_bf16x2(f[8 * q + 2], f[8 * q + 3]),
-                            pack_bf16x2(f[8 * q + 4], f[8 * q + 5]), pack_bf16x2(f[8 * q + 6], f[8 * q + 7]));
+                        uint4 w = make_uint4(pack_bf16x2(f[8 * q], f[8 * q + 1]), pack_bf16x2(f[8 * q + 2], f[8 * q + 3]),
+                                             pack_bf16x2(f[8 * q + 4], f[8 * q + 5]), pack_bf16x2(f[8 * q + 6], f[8 * q + 7]));
+                        if constexpr (EPI == EPI_ROWCOL_BF16) {
+                            if (p.bias) {
+                                const uint4 b = load_bias8(p.bias, col0 + 8 * q, p.N, p.bias_vec);
+                                w = make_uint4(add_bf16x2(w.x, b.x), add_bf16x2(w.y, b.y), add_bf16x2(w.z, b.z), add_bf16x2(w.w, b.w));
+                            }
+                        }
+                        *reinterpret_cast<uint4*>(stg + lane * 64 + cq * 16) = w;
                     }
                     if (p.tma_store) {
                         fence_proxy_async_smem();

@@ -107,6 +107,7 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     __syncthreads();
     tcgen05_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    if (p.after_quant) pdl_wait();  // (a lone split-K launch; one behind a main launch relies on that launch's wait)
 
     bool acc_ok = num_kb > 0;  // epilogue warps: the accumulator holds this CTA's partial
     if (warp == 0) {
@@ -230,14 +231,17 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 f3 = col + 3 < p.N ? __int2float_rn(a3) * (rs * __ldg(p.sw + col + 3)) : 0.0f;
             }
             uint16_t* dst = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(row) * p.ldo + col;
-            if (col + 4 <= p.N && p.vec_ok) {
-                *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(f0, f1), pack_bf16x2(f2, f3));
-            } else {
-                dst[0] = to_bf16_bits(f0);
-                if (col + 1 < p.N) dst[1] = to_bf16_bits(f1);
-                if (col + 2 < p.N) dst[2] = to_bf16_bits(f2);
-                if (col + 3 < p.N) dst[3] = to_bf16_bits(f3);
+            uint2 w = make_uint2(pack_bf16x2(f0, f1), pack_bf16x2(f2, f3));
+            if constexpr (EPI == EPI_ROWCOL_BF16) {
+                if (p.bias) {
+                    uint32_t b[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) b[j] = col + j < p.N ? __ldg(p.bias + col + j) : 0u;
+                    w = make_uint2(add_bf16x2(w.x, b[0] | (b[1] << 16)), add_bf16x2(w.y, b[2] | (b[3] << 16)));
+                }
             }
+            // (the dispatch takes this kernel only where rows are 16-byte aligned, so four columns never straddle N)
+            *reinterpret_cast<uint2*>(dst) = w;
         }
     }
     if (warp == 1) {

@@ -13,6 +13,15 @@ namespace gi8 {
 
 constexpr int kQuantThreads = 256;
 
+// First statement of every quantiser: it may have been started while the kernel before it was still running, so nothing
+// is read or written before that kernel has ended.  Only then may a dependent kernel start: the GEMM behind a quantiser
+// reads its weights without waiting for the quantiser, and must find what the kernel before the quantiser wrote.
+GI8_DEVICE void quant_dependency()
+{
+    pdl_wait();
+    pdl_launch_dependents();
+}
+
 GI8_DEVICE float warp_max(float v)
 {
 #pragma unroll
@@ -197,6 +206,7 @@ __global__ void __launch_bounds__(kQuantThreads, 4)
 quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K,
                             int KB)
 {
+    quant_dependency();
     constexpr int EPL = 16 / sizeof(T);   // elements per lane and load
     constexpr int LPB = 128 / EPL;        // lanes per 128-wide block
     constexpr int BPL = 32 / LPB;         // blocks per warp and load
@@ -255,6 +265,7 @@ template <typename T, int LOADS>
 __global__ void __launch_bounds__(kQuantThreads)
 quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K)
 {
+    quant_dependency();
     constexpr int EPL = 16 / sizeof(T);
     constexpr int kStep = kQuantThreads * EPL;
     __shared__ float warp_amax[2][kQuantThreads / 32];
@@ -346,6 +357,7 @@ __global__ void __launch_bounds__(HadamardShape<LOGH>::THREADS * HadamardShape<L
 hadamard_quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t total,
                                      float norm)
 {
+    quant_dependency();
     using S = HadamardShape<LOGH>;
     __shared__ __align__(16) float stage[S::UNITS][S::WORDS];
     const int t = threadIdx.x % S::THREADS;

@@ -34,6 +34,7 @@ struct SmallMParams {
     int M, N, K;
     int kb_per_split;   // K blocks (of 128) per split
     int splits;
+    const uint16_t* bias;  // bf16 [N] added to the rounded result, or null (cluster variant)
     int static_w;       // weights are not written by the preceding kernel: their first tiles may be fetched before it ends
 };
 
@@ -335,6 +336,8 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const uint32_t my_rank = p.splits > 1 ? cluster_cta_rank() : 0u;
     const uint32_t rows_per_owner = (static_cast<uint32_t>(p.M) + nranks - 1) / nranks;
     float col_scale = 0.0f;  // of this thread's output column (epilogue warps)
+    uint16_t col_bias = 0;
+    const bool has_bias = p.bias != nullptr;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -391,6 +394,7 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int n = tile_n * kSmallMTileN + n_local;
         // The scales are fetched while the weights stream, not between the last MMA and the stores.
         col_scale = n < p.N ? __ldg(p.sw + n) : 0.0f;
+        if (has_bias && n < p.N) col_bias = __ldg(p.bias + n);
         {
             const int t = static_cast<int>(threadIdx.x) - 64;
             if (t < MT) sx_s[t] = t < p.M ? __ldg(p.sx + t) : 0.0f;
@@ -422,9 +426,10 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 if (n < p.N) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (c + j < p.M)
-                            static_cast<uint16_t*>(p.out)[static_cast<int64_t>(c + j) * p.ldo + n] =
-                                to_bf16_bits(__int2float_rn(static_cast<int32_t>(t16[j])) * (sx_s[c + j] * col_scale));
+                        if (c + j < p.M) {
+                            const uint16_t r = to_bf16_bits(__int2float_rn(static_cast<int32_t>(t16[j])) * (sx_s[c + j] * col_scale));
+                            static_cast<uint16_t*>(p.out)[static_cast<int64_t>(c + j) * p.ldo + n] = has_bias ? add_bf16(r, col_bias) : r;
+                        }
                 }
             } else {
 #pragma unroll
@@ -448,9 +453,8 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 int32_t total = 0;
                 for (uint32_t r = 0; r < nranks; ++r)
                     total += recv[(r * rows_per_owner + row_local) * kSmallMTileN + n_local];
-                if (n < p.N)
-                    static_cast<uint16_t*>(p.out)[static_cast<int64_t>(m) * p.ldo + n] =
-                        to_bf16_bits(__int2float_rn(total) * (sx_s[m] * col_scale));
+                const uint16_t v = to_bf16_bits(__int2float_rn(total) * (sx_s[m] * col_scale));
+                if (n < p.N) static_cast<uint16_t*>(p.out)[static_cast<int64_t>(m) * p.ldo + n] = has_bias ? add_bf16(v, col_bias) : v;
             }
         }
     } else {

@@ -362,6 +362,34 @@ GI8_DEVICE uint16_t to_bf16_bits(float f)
     return r;
 }
 
+// A packed pair of results that have been rounded to bf16, plus a packed pair of bf16 bias values: added in fp32 and rounded
+// once more, i.e. what a bf16 tensor addition behind the product gives.
+GI8_DEVICE uint32_t add_bf16x2(uint32_t v, uint32_t bias)
+{
+    return pack_bf16x2(__uint_as_float(v << 16) + __uint_as_float(bias << 16),
+                       __uint_as_float(v & 0xffff0000u) + __uint_as_float(bias & 0xffff0000u));
+}
+
+GI8_DEVICE uint16_t add_bf16(uint16_t v, uint16_t bias)
+{
+    return to_bf16_bits(__uint_as_float(static_cast<uint32_t>(v) << 16) + __uint_as_float(static_cast<uint32_t>(bias) << 16));
+}
+
+// Eight bias values of columns col .. col + 7 (zero beyond N) as four packed pairs.  vec: 16-byte loads are possible
+// (aligned base, col a multiple of 8).  The same address in every lane of a warp: one transaction.
+GI8_DEVICE uint4 load_bias8(const uint16_t* bias, int col, int N, bool vec)
+{
+    if (vec && col + 8 <= N) return __ldg(reinterpret_cast<const uint4*>(bias + col));
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = col + 2 * j < N ? __ldg(bias + col + 2 * j) : 0u;
+        const uint32_t hi = col + 2 * j + 1 < N ? __ldg(bias + col + 2 * j + 1) : 0u;
+        w[j] = lo | (hi << 16);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Thread-block clusters and two-CTA (cta_group::2) forms
 // ---------------------------------------------------------------------------------------------

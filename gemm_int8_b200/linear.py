@@ -8,6 +8,7 @@ or the per-token x per-channel GEMM.  Inference only (the reference has no autog
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 from . import quant
 
@@ -60,21 +61,20 @@ class Int8Linear(torch.nn.Module):
         return self.weight_q.shape[0]
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        import gemm_int8_b200 as g
-
         lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1])
+        x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
         if x2.dtype not in (torch.float32, torch.bfloat16):
             x2 = x2.to(torch.bfloat16)
-        if self.mode == "blockwise":
-            if self.hadamard_block is not None:
-                xq, xs = g.hadamard_quantize_per_token_block(x2, self.hadamard_block)
-            else:
-                xq, xs = g.quantize_per_token_block(x2)
-            out = g.matmul_blockwise(xq, self.weight_q, xs, self.weight_scale)
-        else:
-            xq, xs = g.quantize_per_token(x2)
-            out = g.matmul_scaled(xq, self.weight_q, xs, self.weight_scale)
-        if self.bias is not None:
-            out = out + self.bias.to(out.dtype)
-        return out.to(self.out_dtype).reshape(*lead, self.out_features)
+        weight, bias = self.weight_q, self.bias
+        # The bias goes into the product's epilogue where it is the plain vector of a layer.  One that broadcasts in some
+        # other way, that is differentiated, or K = 0 takes the tensor addition.
+        fused = bias
+        if bias is not None and (bias.shape != weight.shape[:1] or bias.requires_grad or weight.shape[1] == 0
+                                 or forward_ad._current_level >= 0):
+            fused = None
+        out = torch.ops.gemm_int8_CUDA.int8_linear(x2, weight, self.weight_scale, fused, self.mode == "blockwise", self.hadamard_block)
+        if bias is not None and fused is None:
+            out = out + bias.to(out.dtype)
+        if out.dtype != self.out_dtype:
+            out = out.to(self.out_dtype)
+        return out if x.dim() == 2 else out.reshape(*lead, weight.shape[0])

@@ -197,6 +197,21 @@ int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, f
                                       int64_t had_block, void* stream);
 
 /*
+ * A whole W8A8 linear layer: out[M,N] = bf16( product ) (+ bias), the activations quantised on the way.  Two launches, the
+ * second a programmatic dependent of the first.
+ *   x        activations [M,K], fp32 (x_dtype 0) or bf16 (1), as for the quantisers
+ *   w        int8 [N,K]; w_scale: fp32 [N] (blockwise 0) or [ceil(N/128), ceil(K/128)] with row stride ld_sw (blockwise 1)
+ *   bias     bf16 [N] or NULL; added to the bf16 result in fp32 and rounded once more
+ *   had_block  0, or the rotation block of gi8_hadamard_quantize_token_block (blockwise 1 only)
+ *   xq, xs   scratch that receives the quantised activations and their scales: int8 [M,K] (16-byte aligned) and fp32 [M] or
+ *            [M, ceil(K/128)]
+ * Results are those of the quantiser, gi8_matmul_scaled or gi8_matmul_blockwise, and a bf16 addition, bit for bit.
+ */
+int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale, int64_t ld_sw, const void* bias_bf16, int blockwise,
+               int64_t had_block, int8_t* xq, float* xs, void* out_bf16, int64_t M, int64_t N, int64_t K, void* stream);
+
+
+/*
  * Forces a kernel variant for the calling process (tuning and tests); NULL or "" restores the fitted
  * per-shape dispatch that replaces the reference's shape table (csrc/kernels/gemm.cu:136-161).
  * Names: "dense_bn256", "dense_bn128", "dense_bn64" (tile width of the dense and of the blockwise kernel), "smallm"
