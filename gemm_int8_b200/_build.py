@@ -1,4 +1,5 @@
-"""Builds libgemm_int8_b200.so in-tree with nvcc for sm_100a (no libtorch, no CUTLASS).
+"""Builds libgemm_int8_b200.so in-tree with nvcc for sm_100a (no libtorch, no CUTLASS), and libgemm_int8_b200_torch.so, the
+torch operators over it, with g++ against the installed torch.
 
 Replaces the reference's CMake/ninja build of gemm_int8_CUDA.so (CMakeLists.txt, build.sh): one
 translation unit, one nvcc command, a few seconds.
@@ -16,6 +17,10 @@ SOURCES = [os.path.join(_PKG, "csrc", "api.cu")]
 HEADERS = [os.path.join(_PKG, "csrc", f) for f in ("ptx.cuh", "k_dense.cuh", "k_dense_splitk.cuh", "k_blockwise.cuh", "k_smallm.cuh", "k_quant.cuh")]
 HEADERS.append(os.path.join(os.path.dirname(_PKG), "include", "gemm_int8_b200.h"))
 
+OPS_NAME = "libgemm_int8_b200_torch.so"
+OPS_PATH = os.path.join(_PKG, OPS_NAME)
+OPS_SOURCE = os.path.join(_PKG, "csrc", "torch_ops.cpp")
+
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
@@ -30,26 +35,46 @@ def _nvcc() -> str:
     return cand
 
 
-def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _stale(target: str, sources: list[str]) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.exists(f) and os.path.getmtime(f) > t for f in SOURCES + HEADERS)
+    t = os.path.getmtime(target)
+    return any(os.path.exists(f) and os.path.getmtime(f) > t for f in sources)
+
+
+def is_stale() -> bool:
+    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(OPS_PATH, [OPS_SOURCE, HEADERS[-1]])
+
+
+def _run(cmd: list[str], verbose: bool) -> None:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(os.path.basename(cmd[0]) + " failed:\n" + res.stdout + res.stderr)
+    if verbose:
+        print(res.stderr)
+
+
+def _build_ops(verbose: bool) -> None:
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{d}" for d in include),
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", OPS_PATH, OPS_SOURCE,
+          f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+          f"-L{_PKG}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"], verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources; returns its path."""
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB_PATH, *SOURCES]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+    """Compile both libraries if they are missing or older than their sources; returns the path of the first."""
+    if force or _stale(LIB_PATH, SOURCES + HEADERS):
+        _run([_nvcc(), *(["-Xptxas", "-v"] if verbose else []), *NVCC_FLAGS, "-o", LIB_PATH, *SOURCES], verbose)
+    if force or _stale(OPS_PATH, [OPS_SOURCE, HEADERS[-1]]):
+        _build_ops(verbose)
     return LIB_PATH
 
 

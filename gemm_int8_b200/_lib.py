@@ -11,6 +11,8 @@ import os
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libgemm_int8_b200.so")
 
+OPS_PATH = os.path.join(_PKG, "libgemm_int8_b200_torch.so")
+
 STATUS_NAMES = {
     0: "GI8_OK",
     1: "GI8_ERR_INVALID_ARGUMENT",
@@ -67,6 +69,15 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
         fn.restype = res
         fn.argtypes = args
     return lib
+
+
+def load_ops(path: str = OPS_PATH) -> None:
+    """Loads the library that registers the operators' CUDA implementations with torch (after their schemas)."""
+    if not os.path.exists(path):
+        raise ImportError(f"Could not find the compiled operator library {path}; build it with `python gemm_int8_b200/_build.py`.")
+    import torch
+
+    torch.ops.load_library(path)
 
 
 class GemmInt8Error(RuntimeError):
