@@ -98,10 +98,9 @@ struct BlockwiseParams {
                     // N-sharded group: each rank's full [M, N_total] matrix, peers through mapped peer memory)
     int out_col0;   // column of this GEMM's first output column in those matrices
     int scale_vec;  // ceil(K/128) % 4 == 0 and the rows of sa and sw are 16-byte aligned: scales are loaded four at a time
-    int pdl_role;   // 0: none.  1: this launch is followed by an independent launch over other output columns: let it start
-                    // as SMs free up (griddepcontrol.launch_dependents).  2: that second launch: it reads nothing the first
-                    // one writes and therefore does not wait before working, but it waits for the first before it ends,
-                    // so that the completion of the pair means the completion of both.
+    int pdl_role;   // 2: the second launch of a pair over other output columns.  It reads nothing the first one writes and
+                    // therefore does not wait before working, but it waits for the first before it ends, so that the
+                    // completion of the pair means the completion of both.
     int scatter_ranks;  // > 0: K-sharded reduce-scatter form.  The fp32 accumulators of tile rows [j R, (j + 1) R), R =
     int scatter_rows;   // scatter_rows, go to output matrix j (rank j's receive area, float [ranks, R, N], mapped peer
     int scatter_me;     // memory for j != me) at row block scatter_me, as 32 x 32 fp32 TMA-store boxes; R % 32 == 0
@@ -365,8 +364,9 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     // tiles, which decode uses, requests its first weights before it waits.
     const bool early_weights = BN < 256 && p.after_quant;
     if (BN == 256 || (p.pdl_role != 2 && !(early_weights && warp == 0))) pdl_wait();
-    // (after that wait: the launch behind this one does not wait for anything before it reads x)
-    if (p.pdl_role == 1 && threadIdx.x == 0) pdl_launch_dependents();
+    // What follows in the stream may start as SMs free up: only after that wait, for the second of two launches does not wait
+    // for anything before it reads x and y.  (early_weights: the waiting warp is not this one.)
+    if (p.pdl_role != 2 && threadIdx.x == 0) pdl_launch_dependents();
 
     if (warp < 4) {
         setmaxnreg_dec<kControlRegs>();

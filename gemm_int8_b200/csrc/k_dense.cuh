@@ -51,11 +51,10 @@ struct DenseParams {
     int group_m;          // row-blocks per rasterisation band
     int tma_store;        // bf16 epilogues: stage 32 x 32 blocks in shared memory and write them with TMA stores
     int tile_end;         // > 0: only tiles [0, tile_end) of the grid are computed here (the rest by the split-K launch)
-    int pdl_role;         // 1: an independent launch over other output tiles follows: let it start as SMs free up
     float alpha;
     const uint16_t* bias; // bf16 [N] added to the rounded result, or null (EPI_ROWCOL_BF16)
     int bias_vec;         // bias is 16-byte aligned
-    int after_quant;      // launched as the programmatic dependent of the kernel that writes x and sx: wait for it first
+    int dependent;        // launched as a programmatic dependent: wait for the kernel in front before the first access
 };
 
 // Records the first error of the grid and raises the CTA-wide abort flag.
@@ -237,9 +236,10 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers exist before anything signals them remotely
     tcgen05_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
-    if (p.after_quant) pdl_wait();
-    // (after that wait: the launch behind this one does not wait for anything before it reads x)
-    if (p.pdl_role == 1 && threadIdx.x == 0) pdl_launch_dependents();
+    if (p.dependent) pdl_wait();
+    // What follows in the stream may start as SMs free up.  Only after that wait: a split-K launch over the last tiles of this
+    // grid reads x and y without waiting for anything itself.
+    if (threadIdx.x == 0) pdl_launch_dependents();
 
     // The producer and the MMA issuer run their loops with the WHOLE warp (uniform control flow) and elect one lane
     // only around the TMA / MMA / commit instructions.  Inside an `if (lane == 0)` region the compiler treats

@@ -107,7 +107,10 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     __syncthreads();
     tcgen05_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
-    if (p.after_quant) pdl_wait();  // (a lone split-K launch; one behind a main launch relies on that launch's wait)
+    if (p.dependent) {  // a lone split-K launch; one behind a main launch relies on that launch's wait, and releases nothing
+        pdl_wait();
+        if (threadIdx.x == 0) pdl_launch_dependents();
+    }
 
     bool acc_ok = num_kb > 0;  // epilogue warps: the accumulator holds this CTA's partial
     if (warp == 0) {
