@@ -245,9 +245,12 @@ int check_common(const void* x, const void* y, const void* out, int64_t M, int64
 // form's cycles per K block, fitted on B200 from device-timed runs (8192^3, 2048 x 11008 x 4096, 128..512 x 8192 x
 // 8192 and the reference benchmark's layer shapes, timed back to back):
 //   dense      256 x 256 two-CTA tile (74 slots) 580 | 128 x 256: 655 | 128 x 128: 465 | 128 x 64: 330
-//   blockwise  128 x 256: 950 | 256 x 256 two-CTA tile: 920, but only ahead on long runs, hence its minimum number of waves
-//              (fitted when both converted their partials; without conversions both take 3 to 6 % less, level at 512 x
-//              8192 x 8192 and 8192^3, so the order stands)
+//   blockwise  128 x 256: 950 | 256 x 256 two-CTA tile: 920 | (fitted when both converted their partials; without conversions
+//              both take 3 to 6 % less, the order stands).  The two-CTA tile gains by fewer operand bytes per MAC, which counts
+//              the longer the run and the longer K: 0.15 s of back-to-back calls, one-CTA against two-CTA, 2048 x 8192 x
+//              28672 577 -> 549 us, 4096 x 4096 x 14336 285 -> 275, 700 x 9000 x 12288 115 -> 111, 1024 x 4096 x 14336 72.5 ->
+//              70.9, 2048 x 11008 x 4096 110.1 -> 107.9; in short bursts, below the power cap, level up to 8192^3.  Hence its
+//              minimum: twenty waves, or 96 K blocks
 //              | 128 x 128: 650 | 128 x 64: 490
 // The table is data: kDenseForms / kBlockwiseForms below.  The narrow tiles cost more per column (the tensor-core instruction is issue
 // bound below N = 128, and the per-K-block hand-overs do not shrink with the tile) and only pay when the wide tile
@@ -257,12 +260,13 @@ struct TileForm {
     int bn;
     bool pair;
     double kblock_cycles;
-    int min_waves;  // the form is considered only for grids of at least this many waves
+    int min_waves;  // the form is considered only for grids of at least this many waves ...
+    int min_kb;     // ... or for at least this many K blocks
 };
-constexpr TileForm kDenseForms[] = {{256, true, 580.0, 0}, {256, false, 655.0, 0}, {128, false, 465.0, 0}, {64, false, 330.0, 0}};
-constexpr TileForm kBlockwiseForms[] = {{256, true, 920.0, 20}, {256, false, 950.0, 0}, {128, false, 650.0, 0}, {64, false, 490.0, 0}};
+constexpr TileForm kDenseForms[] = {{256, true, 580.0, 0, 0}, {256, false, 655.0, 0, 0}, {128, false, 465.0, 0, 0}, {64, false, 330.0, 0, 0}};
+constexpr TileForm kBlockwiseForms[] = {{256, true, 920.0, 20, 96}, {256, false, 950.0, 0, 0}, {128, false, 650.0, 0, 0}, {64, false, 490.0, 0, 0}};
 
-int pick_bn(int64_t M, int64_t N, int sms, bool blockwise, bool* pair = nullptr, double* cost_per_kb = nullptr)
+int pick_bn(int64_t M, int64_t N, int64_t K, int sms, bool blockwise, bool* pair = nullptr, double* cost_per_kb = nullptr)
 {
     if (pair) *pair = false;
     const TileForm* forms = blockwise ? kBlockwiseForms : kDenseForms;
@@ -276,7 +280,7 @@ int pick_bn(int64_t M, int64_t N, int sms, bool blockwise, bool* pair = nullptr,
         const int64_t tiles = ((M + tile_m - 1) / tile_m) * ((N + f.bn - 1) / f.bn);
         const int64_t slots = f.pair ? sms / 2 : sms;
         const int64_t waves = (tiles + slots - 1) / slots;
-        if (waves < f.min_waves) continue;
+        if (waves < f.min_waves && (K + kBK - 1) / kBK < f.min_kb) continue;
         // (a wave also pays a fixed part per tile: prologue, epilogue, tile turnover -- about 20 K blocks' worth at
         // K = 4096; the model only ranks forms for one K, so it enters as a small constant)
         const double cost = static_cast<double>(waves) * (f.kblock_cycles + 16.0);
@@ -313,6 +317,7 @@ struct ColumnSplit {
     bool use;
     int64_t n1;   // columns of the first launch (a multiple of 256)
     int bn_tail;  // tile width of the second launch
+    double cost;  // of both launches, in cycles
 };
 
 ColumnSplit plan_column_split(int64_t M, int64_t N, int64_t K, int sms)
@@ -339,7 +344,27 @@ ColumnSplit plan_column_split(int64_t M, int64_t N, int64_t K, int sms)
     const double now = static_cast<double>(W + 1) * form * kb;
     const double split = (static_cast<double>(W) * form + best + 16.0) * kb + kColumnSplitFixedCycles;
     if (knobs().tail_split == 1 && split >= 0.98 * now) return c;
-    c.use = true, c.n1 = n1;
+    c.use = true, c.n1 = n1, c.cost = split;
+    return c;
+}
+
+// The automatic choice for the blockwise entry point.  Where the grid's last wave is thin and whole column bands lie before it,
+// the column split is weighed against the form that would run instead.
+struct BlockwiseChoice {
+    int bn;
+    bool pair;
+    ColumnSplit split;
+};
+
+BlockwiseChoice choose_blockwise(int64_t M, int64_t N, int64_t K, int sms)
+{
+    BlockwiseChoice c{};
+    double cost = 0.0;
+    c.bn = pick_bn(M, N, K, sms, true, &c.pair, &cost);
+    if (c.bn == 256 && N % 8 == 0) {
+        c.split = plan_column_split(M, N, K, sms);
+        if (c.pair && knobs().tail_split == 1 && c.split.cost >= cost * static_cast<double>((K + kBK - 1) / kBK)) c.split.use = false;
+    }
     return c;
 }
 
@@ -527,7 +552,7 @@ DenseChoice choose_dense(int64_t M, int64_t N, int64_t K, int sms)
 {
     DenseChoice c{};
     double cost = 0.0;
-    c.bn = pick_bn(M, N, sms, false, &c.pair, &cost);
+    c.bn = pick_bn(M, N, K, sms, false, &c.pair, &cost);
     if (c.bn == 256) {
         c.tail = plan_tail(M, N, K, c.pair, c.pair ? kDenseForms[0].kblock_cycles : kDenseForms[1].kblock_cycles, sms);
     } else {
@@ -814,12 +839,10 @@ const char* gi8_pick_variant(int kind, int64_t M, int64_t N, int64_t K)
     if (forced != VAR_AUTO) return kVariantNames[forced];
     if (kind == 1 && plan_smallm(M, N, K, sms, false).use) return "smallm_cluster";
     if (kind == 2) {
-        bool pair = false;
-        const int bn = pick_bn(M, N, sms, true, &pair);
-        if (bn == 256 && !pair && N % 8 == 0) {
-            const ColumnSplit c = plan_column_split(M, N, K, sms);
-            if (c.use) return c.bn_tail == 128 ? "blockwise_bn256+columns_bn128" : "blockwise_bn256+columns_bn64";
-        }
+        const BlockwiseChoice c = choose_blockwise(M, N, K, sms);
+        const int bn = c.bn;
+        const bool pair = c.pair;
+        if (c.split.use) return c.split.bn_tail == 128 ? "blockwise_bn256+columns_bn128" : "blockwise_bn256+columns_bn64";
         return pair ? "blockwise_pair" : bn == 256 ? "blockwise_bn256" : bn == 128 ? "blockwise_bn128" : "blockwise_bn64";
     }
     const DenseChoice c = choose_dense(M, N, K, sms);
@@ -1150,7 +1173,7 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
         case VAR_DENSE_BN128: bn = 128; break;
         case VAR_DENSE_BN64: bn = 64; break;
         case VAR_PAIR: bn = 256, pair = true; break;
-        default: bn = pick_bn(M, N, st->sm_count, true, &pair);
+        default: bn = pick_bn(M, N, K, st->sm_count, true, &pair);
     }
     if (force_bn) bn = force_bn, pair = false;
     if (scatter && bn == 64) bn = 128;  // a 32 x 32 fp32 box needs the 4 KB staging block of the wider tiles
@@ -1238,18 +1261,15 @@ static int blockwise_dispatch(const int8_t* x, const int8_t* y, const float* sa,
     if (g_forced_variant == VAR_AUTO && M > 0 && N > 0 && K > 0 && out && reinterpret_cast<uintptr_t>(out) % 16 == 0 && N % 8 == 0) {
         DeviceState* st;
         if (int rc = get_device_state(&st)) return rc;
-        bool pair = false;
-        if (pick_bn(M, N, st->sm_count, true, &pair) == 256 && !pair) {
-            const ColumnSplit c = plan_column_split(M, N, K, st->sm_count);
-            if (c.use) {
-                // both launches write through a tensor map of the whole [M, N] matrix, each its own columns
-                void* outs[1] = {out};
-                const bool pdl = knobs().pdl;  // GEMM_INT8_PDL=0: two ordinary launches, one after the other
-                if (int rc = blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, nullptr, M, c.n1, K, stream, outs, 1, N, 0, false, 256, 0, -1, bias, after_quant))
-                    return rc;
-                return blockwise_impl(x, y + c.n1 * K, sa, ld_sa, sw ? sw + (c.n1 / 128) * ld_sw : sw, ld_sw, nullptr, M, N - c.n1, K,
-                                      stream, outs, 1, N, c.n1, false, c.bn_tail, pdl ? 2 : 0, -1, bias ? bias + c.n1 : nullptr, false);
-            }
+        const ColumnSplit c = choose_blockwise(M, N, K, st->sm_count).split;
+        if (c.use) {
+            // both launches write through a tensor map of the whole [M, N] matrix, each its own columns
+            void* outs[1] = {out};
+            const bool pdl = knobs().pdl;  // GEMM_INT8_PDL=0: two ordinary launches, one after the other
+            if (int rc = blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, nullptr, M, c.n1, K, stream, outs, 1, N, 0, false, 256, 0, -1, bias, after_quant))
+                return rc;
+            return blockwise_impl(x, y + c.n1 * K, sa, ld_sa, sw ? sw + (c.n1 / 128) * ld_sw : sw, ld_sw, nullptr, M, N - c.n1, K,
+                                  stream, outs, 1, N, c.n1, false, c.bn_tail, pdl ? 2 : 0, -1, bias ? bias + c.n1 : nullptr, false);
         }
     }
     return blockwise_impl(x, y, sa, ld_sa, sw, ld_sw, out, M, N, K, stream, nullptr, 1, N, 0, false, 0, 0, -1, bias, after_quant);
