@@ -662,6 +662,20 @@ SmallMPlan plan_smallm(int64_t M, int64_t N, int64_t K, int sms, bool forced, in
     return pl;
 }
 
+constexpr int kMaxClusterSplits = 8;  // portable thread-block cluster size
+
+// The plain product takes the small-M kernel where it beat the dense forms (device times over graph replays, operands rotated
+// beyond L2, dense against small-M): always up to 16 tokens (16 x 4096 x 14336 29.8 -> 12.3 us, 16 x 14336 x 4096 20.6 -> 13.7,
+// 16 x 57344 x 14336 135 -> 123, 16 x 1000 x 1024 4.5 -> 3.4); above, where K is long and cut into eight splits, or seven (64 x 4096 x 14336
+// 30.0 -> 15.1, 64 x 4096 x 4096 10.8 -> 9.1, 64 x 1000 x 4096 9.9 -> 6.4).  Elsewhere the reduction, or the wider token tile, costs more
+// than it gains (64 x 4096 x 1024 4.7 -> 7.6, 64 x 14336 x 4096 13.7 -> 18.1).
+SmallMPlan plan_smallm_plain(int64_t M, int64_t N, int64_t K, int sms)
+{
+    SmallMPlan pl = plan_smallm(M, N, K, sms, false, kMaxClusterSplits);
+    if (M > 16 && !(pl.splits >= kMaxClusterSplits - 1 && K >= 4096)) pl.use = false;  // (33 K blocks make seven splits of five)
+    return pl;
+}
+
 template <int MT, int STAGES>
 int launch_smallm(DeviceState* st, int slot, const int8_t* x, const int8_t* w, SmallMParams p, const SmallMPlan& pl,
                   cudaStream_t stream)
@@ -679,7 +693,6 @@ int launch_smallm(DeviceState* st, int slot, const int8_t* x, const int8_t* w, S
     return GI8_OK;
 }
 
-constexpr int kMaxClusterSplits = 8;  // portable thread-block cluster size
 
 // RECV: room behind the pipeline buffers for the partial sums the cluster peers send (needed when splits > 1).
 template <int MT, int STAGES, bool RECV>
@@ -837,7 +850,7 @@ const char* gi8_pick_variant(int kind, int64_t M, int64_t N, int64_t K)
     if (get_device_state(&st) == GI8_OK) sms = st->sm_count;
     const int forced = g_forced_variant;
     if (forced != VAR_AUTO) return kVariantNames[forced];
-    if (kind == 1 && plan_smallm(M, N, K, sms, false).use) return "smallm_cluster";
+    if ((kind == 1 && plan_smallm(M, N, K, sms, false).use) || (kind == 0 && plan_smallm_plain(M, N, K, sms).use)) return "smallm_cluster";
     if (kind == 2) {
         const BlockwiseChoice c = choose_blockwise(M, N, K, sms);
         const int bn = c.bn;
@@ -896,6 +909,8 @@ int gi8_device_status(uint32_t* code)
     return GI8_OK;
 }
 
+static int launch_smallm_cluster(DeviceState* st, const int8_t* x, const int8_t* y, const SmallMParams& q, const SmallMPlan& pl, cudaStream_t s);
+
 int gi8_matmul(const int8_t* x, const int8_t* y, void* out, int64_t M, int64_t N, int64_t K, float alpha, void* stream)
 {
     if (int rc = check_common(x, y, out, M, N, K, 2)) return rc;
@@ -904,6 +919,17 @@ int gi8_matmul(const int8_t* x, const int8_t* y, void* out, int64_t M, int64_t N
     if (int rc = get_device_state(&st)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (K == 0) return zero_output(out, M * N * 2, s);
+    if (g_forced_variant == VAR_AUTO) {
+        // Few tokens: the small-M kernel with scales 1 and alpha, whose product is alpha.
+        const SmallMPlan pl = plan_smallm_plain(M, N, K, st->sm_count);
+        if (pl.use) {
+            SmallMParams q{};
+            q.out = out, q.alpha = alpha, q.status = st->status, q.ldo = N;
+            q.M = (int)M, q.N = (int)N, q.K = (int)K, q.kb_per_split = pl.kb_per_split, q.splits = pl.splits;
+            q.static_w = knobs().static_weights && knobs().pdl;
+            return launch_smallm_cluster(st, x, y, q, pl, s);
+        }
+    }
     DenseParams p{};
     p.out = out, p.status = st->status, p.ldo = N, p.M = (int)M, p.N = (int)N, p.K = (int)K, p.alpha = alpha;
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
@@ -937,6 +963,28 @@ int64_t gi8_matmul_scaled_workspace_bytes(int64_t M, int64_t N, int64_t K)
     return pl.use ? pl.total_bytes : 0;
 }
 
+static int launch_smallm_cluster(DeviceState* st, const int8_t* x, const int8_t* y, const SmallMParams& q, const SmallMPlan& pl, cudaStream_t s)
+{
+    // Pipeline depth: two CTAs share an SM (about 100 KB each, the receive area of a cluster CTA included).  A
+    // deeper pipeline with one CTA per SM measured slower even for grids of at most one CTA per SM: the next
+    // kernel's CTAs could no longer move in beside the running ones, and its set-up no longer overlapped.
+    if (pl.splits > 1) {
+        switch (pl.mt) {
+            case 16: return launch_smallm_cluster<16, 5, true>(st, 48, x, y, q, pl, s);
+            case 32: return launch_smallm_cluster<32, 4, true>(st, 49, x, y, q, pl, s);
+            case 64: return launch_smallm_cluster<64, 3, true>(st, 50, x, y, q, pl, s);
+            default: return launch_smallm_cluster<128, 3, true>(st, 51, x, y, q, pl, s);
+        }
+    } else {
+        switch (pl.mt) {
+            case 16: return launch_smallm_cluster<16, 6, false>(st, 52, x, y, q, pl, s);
+            case 32: return launch_smallm_cluster<32, 5, false>(st, 53, x, y, q, pl, s);
+            case 64: return launch_smallm_cluster<64, 4, false>(st, 54, x, y, q, pl, s);
+            default: return launch_smallm_cluster<128, 3, true>(st, 51, x, y, q, pl, s);
+        }
+    }
+}
+
 // bias: bf16 [N] or null.  after_quant: the launch directly in front of this one in the stream is the quantiser that writes
 // x and sx (it has waited for everything before it, the weights' writers included, before it lets a dependent start).
 static int scaled_impl(const int8_t* x, const int8_t* y, const float* sx, const float* sw, void* out, int64_t M, int64_t N, int64_t K,
@@ -960,24 +1008,7 @@ static int scaled_impl(const int8_t* x, const int8_t* y, const float* sx, const 
             q.M = (int)M, q.N = (int)N, q.K = (int)K, q.kb_per_split = pl.kb_per_split, q.splits = pl.splits;
             q.static_w = (knobs().static_weights || after_quant) && knobs().pdl;
             q.bias = bias;
-            // Pipeline depth: two CTAs share an SM (about 100 KB each, the receive area of a cluster CTA included).  A
-            // deeper pipeline with one CTA per SM measured slower even for grids of at most one CTA per SM: the next
-            // kernel's CTAs could no longer move in beside the running ones, and its set-up no longer overlapped.
-            if (pl.splits > 1) {
-                switch (pl.mt) {
-                    case 16: return launch_smallm_cluster<16, 5, true>(st, 48, x, y, q, pl, s);
-                    case 32: return launch_smallm_cluster<32, 4, true>(st, 49, x, y, q, pl, s);
-                    case 64: return launch_smallm_cluster<64, 3, true>(st, 50, x, y, q, pl, s);
-                    default: return launch_smallm_cluster<128, 3, true>(st, 51, x, y, q, pl, s);
-                }
-            } else {
-                switch (pl.mt) {
-                    case 16: return launch_smallm_cluster<16, 6, false>(st, 52, x, y, q, pl, s);
-                    case 32: return launch_smallm_cluster<32, 5, false>(st, 53, x, y, q, pl, s);
-                    case 64: return launch_smallm_cluster<64, 4, false>(st, 54, x, y, q, pl, s);
-                    default: return launch_smallm_cluster<128, 3, true>(st, 51, x, y, q, pl, s);
-                }
-            }
+            return launch_smallm_cluster(st, x, y, q, pl, s);
         }
     }
     if (forced == VAR_SMALLM) {

@@ -25,7 +25,7 @@ constexpr int kSmallMTileN = 128;  // weight rows per CTA = UMMA M
 
 struct SmallMParams {
     void* out;          // bf16 [M,N], leading dimension ldo
-    const float* sx;    // [M]
+    const float* sx;    // [M]   (cluster variant: null with sw for the plain product, whose scale is alpha)
     const float* sw;    // [N]
     int32_t* scratch;   // [tiles_n][MT][128] int32 partial sums, zero on entry and on exit (SPLITS > 1)
     uint32_t* counters; // [tiles_n] arrival counters, zero on entry and on exit (SPLITS > 1)
@@ -35,6 +35,7 @@ struct SmallMParams {
     int kb_per_split;   // K blocks (of 128) per split
     int splits;
     const uint16_t* bias;  // bf16 [N] added to the rounded result, or null (cluster variant)
+    float alpha;
     int static_w;       // weights are not written by the preceding kernel: their first tiles may be fetched before it ends
 };
 
@@ -393,11 +394,11 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int n_local = quarter * 32 + lane;
         const int n = tile_n * kSmallMTileN + n_local;
         // The scales are fetched while the weights stream, not between the last MMA and the stores.
-        col_scale = n < p.N ? __ldg(p.sw + n) : 0.0f;
+        col_scale = !p.sw ? p.alpha : n < p.N ? __ldg(p.sw + n) : 0.0f;
         if (has_bias && n < p.N) col_bias = __ldg(p.bias + n);
         {
             const int t = static_cast<int>(threadIdx.x) - 64;
-            if (t < MT) sx_s[t] = t < p.M ? __ldg(p.sx + t) : 0.0f;
+            if (t < MT) sx_s[t] = !p.sx ? 1.0f : t < p.M ? __ldg(p.sx + t) : 0.0f;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
         bool ok = true;
