@@ -920,13 +920,13 @@ int gi8_matmul(const int8_t* x, const int8_t* y, void* out, int64_t M, int64_t N
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (K == 0) return zero_output(out, M * N * 2, s);
     if (g_forced_variant == VAR_AUTO) {
-        // Few tokens: the small-M kernel with scales 1 and alpha, whose product is alpha.
+        // Few tokens: the small-M kernel with scales 1 and alpha, whose product is alpha.  static_w stays 0 whatever
+        // GEMM_INT8_STATIC_WEIGHTS says: that promise is about a layer's weights, and y here may be what the kernel in front wrote.
         const SmallMPlan pl = plan_smallm_plain(M, N, K, st->sm_count);
         if (pl.use) {
             SmallMParams q{};
             q.out = out, q.alpha = alpha, q.status = st->status, q.ldo = N;
             q.M = (int)M, q.N = (int)N, q.K = (int)K, q.kb_per_split = pl.kb_per_split, q.splits = pl.splits;
-            q.static_w = knobs().static_weights && knobs().pdl;
             return launch_smallm_cluster(st, x, y, q, pl, s);
         }
     }

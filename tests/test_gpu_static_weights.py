@@ -1,0 +1,54 @@
+"""GEMM_INT8_STATIC_WEIGHTS=1 promises that the weight operand of the scaled product is not written by the work directly in front of
+it.  What the promise does not cover must be ordered as without it: the second operand of the plain product, and weights that a
+kernel further back in the stream writes.  The writers here are the library's own quantisers, which let the next kernel start before
+they have written anything; the data alternate, so that a read that came too early would see the other set.  All checks are
+bit comparisons with the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def g(monkeypatch):
+    import gemm_int8_b200
+
+    monkeypatch.setenv("GEMM_INT8_STATIC_WEIGHTS", "1")
+    gemm_int8_b200.reload_env()
+    yield gemm_int8_b200
+    monkeypatch.delenv("GEMM_INT8_STATIC_WEIGHTS")
+    gemm_int8_b200.reload_env()
+    assert gemm_int8_b200.device_status() == 0
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _quantise_into(g, a, q, s):
+    """Per-row quantiser into fixed buffers (the operators allocate theirs)."""
+    rc = g._C.gi8_quantize_token(_p(a), 1, _p(q), _p(s), a.shape[0], a.shape[1], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, g._C.gi8_last_error()
+
+
+def _pair(M, K, gen):
+    return [torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2)]
+
+
+@pytest.mark.parametrize("M, N, K", [(1, 4096, 4096), (16, 8192, 1024), (64, 2048, 8192), (16, 1001, 272)])
+def test_plain_product_of_an_operand_quantised_in_front(g, oracle, M, N, K):
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    assert g.pick_variant(0, M, N, K) == "smallm_cluster"
+    sources = _pair(N, K, gen)
+    x = torch.randint(-128, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+    want = [oracle.c_matmul(x.cpu(), g.quantize_per_token(a)[0].cpu(), -0.37) for a in sources]
+    y, s = torch.empty(N, K, dtype=torch.int8, device="cuda"), torch.empty(N, device="cuda")
+    outs = []
+    for i in range(40):
+        _quantise_into(g, sources[i % 2], y, s)
+        outs.append(g.matmul(x, y, -0.37))
+    for i, out in enumerate(outs):
+        assert np.array_equal(oracle.bf16_bits(out), want[i % 2]), i
