@@ -301,7 +301,6 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         fence_proxy_async_smem();
         prefetch_tensormap(&map_w);
         prefetch_tensormap(&map_x);
-        pdl_launch_dependents();  // the next kernel may be scheduled as soon as SMs free up
         const uint64_t pol_w = l2_policy_evict_first();
         const uint64_t pol_x = l2_policy_evict_last();
         const int first = min(num_kb, STAGES);
@@ -330,6 +329,9 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     tcgen05_fence_after_sync();
     pdl_wait();  // every thread: scales are read and the output is written only after the previous kernel is done
+    // What follows in the stream may start as SMs free up, but only now: a dependent that requests its weights before its own
+    // wait must find everything written in front of THIS kernel, not only what this kernel writes.
+    if (threadIdx.x == 0) pdl_launch_dependents();
     const uint32_t tmem_base = tmem_base_slot;
     // [sender][row of this owner][128] int32, behind the pipeline buffers
     int32_t* recv = reinterpret_cast<int32_t*>(smem + STAGES * kStageBytes);

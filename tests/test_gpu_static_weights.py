@@ -52,3 +52,52 @@ def test_plain_product_of_an_operand_quantised_in_front(g, oracle, M, N, K):
         outs.append(g.matmul(x, y, -0.37))
     for i, out in enumerate(outs):
         assert np.array_equal(oracle.bf16_bits(out), want[i % 2]), i
+
+
+def _product_in_front(g, form, gen):
+    """A call of this library that stands between the writer of the weights and their reader."""
+    M = 16
+    if form in ("smallm", "smallm_split", "dense"):
+        M, N, K = (200, 2048, 1024) if form == "dense" else (16, 16384, 512) if form == "smallm" else (16, 1024, 8192)
+        x = torch.randint(-128, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+        w = torch.randint(-128, 128, (N, K), dtype=torch.int8, device="cuda", generator=gen)
+        sx, sw = torch.rand(M, device="cuda", generator=gen), torch.rand(N, device="cuda", generator=gen)
+        return lambda: g.matmul_scaled(x, w, sx, sw)
+    layer = g.Int8Linear.from_float(torch.randn(1024, 1024, device="cuda", generator=gen), mode=form)
+    x = torch.randn(M, 1024, device="cuda", generator=gen).to(torch.bfloat16)
+    return lambda: layer(x)
+
+
+@pytest.mark.parametrize("form", ["smallm", "smallm_split", "dense", "channel", "blockwise"])
+@pytest.mark.parametrize("captured", [False, True])
+def test_weights_written_two_calls_back(g, oracle, form, captured):
+    """writer of w -> another product -> product with w: w is not written by the work directly in front, so the promise holds."""
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    M, N, K = 16, 8192, 1024
+    sources = _pair(N, K, gen)
+    x = torch.randint(-128, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+    sx = torch.rand(M, device="cuda", generator=gen)
+    quantised = [g.quantize_per_token(a) for a in sources]
+    want = [oracle.c_matmul_scaled(x.cpu(), q.cpu(), sx.cpu(), s.cpu()) for q, s in quantised]
+    between = _product_in_front(g, form, gen)
+    first = between().clone()
+    w, sw = torch.empty(N, K, dtype=torch.int8, device="cuda"), torch.empty(N, device="cuda")
+
+    def step(i):
+        _quantise_into(g, sources[i % 2], w, sw)
+        other = between()
+        return g.matmul_scaled(x, w, sx, sw), other
+
+    if captured:
+        step(0)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [step(i) for i in range(4)]
+        for _ in range(10):
+            graph.replay()
+    else:
+        outs = [step(i) for i in range(40)]
+    for i, (out, other) in enumerate(outs):
+        assert np.array_equal(oracle.bf16_bits(out), want[i % 2]), i
+        assert torch.equal(other.view(torch.int16), first.view(torch.int16)), i
