@@ -364,9 +364,10 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     // tiles, which decode uses, requests its first weights before it waits.
     const bool early_weights = BN < 256 && p.after_quant;
     if (BN == 256 || (p.pdl_role != 2 && !(early_weights && warp == 0))) pdl_wait();
-    // What follows in the stream may start as SMs free up: only after that wait, for the second of two launches does not wait
-    // for anything before it reads x and y.  (early_weights: the waiting warp is not this one.)
-    if (p.pdl_role != 2 && threadIdx.x == 0) pdl_launch_dependents();
+    // What follows in the stream may start as SMs free up, once this CTA has waited: the second of two launches, and a small-M
+    // kernel with static weights, read before they wait themselves.  The thread is one of warp 1, which has waited in every
+    // case; warp 0 has not where it requests weights early.
+    if (p.pdl_role != 2 && threadIdx.x == 32) pdl_launch_dependents();
 
     if (warp < 4) {
         setmaxnreg_dec<kControlRegs>();

@@ -101,3 +101,31 @@ def test_weights_written_two_calls_back(g, oracle, form, captured):
     for i, (out, other) in enumerate(outs):
         assert np.array_equal(oracle.bf16_bits(out), want[i % 2]), i
         assert torch.equal(other.view(torch.int16), first.view(torch.int16)), i
+
+
+@pytest.mark.parametrize("blockwise, M", [(1, 128), (0, 64), (0, 200)])
+def test_weights_written_by_the_quantiser_of_the_layer_in_front(g, oracle, blockwise, M):
+    """The quantised activations of a layer are the weights of the product behind it: the layer's own product, which may request
+    its weights under its quantiser, stands between their writer and their reader."""
+    gen = torch.Generator(device="cuda").manual_seed(13)
+    N, K = 2048, 1024
+    if blockwise:
+        assert g.pick_variant(2, M, N, K) in ("blockwise_bn64", "blockwise_bn128")
+    sources = _pair(M, K, gen)
+    layer = g.Int8Linear.from_float(torch.randn(N, K, device="cuda", generator=gen), mode="blockwise" if blockwise else "channel")
+    a = torch.randint(-128, 128, (16, K), dtype=torch.int8, device="cuda", generator=gen)
+    sx, sw = torch.rand(16, device="cuda", generator=gen), torch.rand(M, device="cuda", generator=gen)
+    quantise = g.quantize_per_token_block if blockwise else g.quantize_per_token
+    want = [(oracle.c_matmul_scaled(a.cpu(), quantise(x)[0].cpu(), sx.cpu(), sw.cpu()), layer(x)) for x in sources]
+    xq, xs = torch.empty(M, K, dtype=torch.int8, device="cuda"), torch.empty(M, 8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    outs = []
+    for i in range(40):
+        out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        rc = g._C.gi8_linear(_p(sources[i % 2]), 1, _p(layer.weight_q), _p(layer.weight_scale), K // 128, None, blockwise, 0, _p(xq), _p(xs), _p(out),
+                             M, N, K, stream)
+        assert rc == 0, g._C.gi8_last_error()
+        outs.append((g.matmul_scaled(a, xq, sx, sw), out))
+    for i, (scaled, out) in enumerate(outs):
+        assert np.array_equal(oracle.bf16_bits(scaled), want[i % 2][0]), i
+        assert torch.equal(out.view(torch.int16), want[i % 2][1].view(torch.int16)), i
