@@ -239,6 +239,28 @@ int check_common(const void* x, const void* y, const void* out, int64_t M, int64
     return GI8_OK;
 }
 
+int check_scale_pointers(const float* sx, const float* sw)
+{
+    if (!sx || !sw) return fail(GI8_ERR_INVALID_ARGUMENT, "null scale pointer");
+    if (reinterpret_cast<uintptr_t>(sx) % 4 || reinterpret_cast<uintptr_t>(sw) % 4)
+        return fail(GI8_ERR_MISALIGNED, "scale pointers must be 4-byte aligned");
+    return GI8_OK;
+}
+
+int check_block_scales(const float* sa, int64_t ld_sa, const float* sw, int64_t ld_sw, int64_t M, int64_t N, int64_t K)
+{
+    const int64_t KB = (K + kBK - 1) / kBK;
+    if (!sa || !sw) return fail(GI8_ERR_INVALID_ARGUMENT, "null scale pointer");
+    if (ld_sa < KB || ld_sw < KB)
+        return fail(GI8_ERR_INVALID_ARGUMENT, "scale row strides (%lld, %lld) must be at least ceil(K/128) = %lld",
+                    (long long)ld_sa, (long long)ld_sw, (long long)KB);
+    if (int rc = check_scale_pointers(sa, sw)) return rc;
+    // The kernels index the scale arrays with 32-bit element offsets.
+    if (M * ld_sa >= (int64_t(1) << 31) || ((N + 127) / 128) * ld_sw >= (int64_t(1) << 31))
+        return fail(GI8_ERR_INVALID_ARGUMENT, "scale arrays of 2^31 or more elements are not supported");
+    return GI8_OK;
+}
+
 // ---------------------------------------------------------------------------------------------------
 // Dispatch: picks the tile form for the dense/blockwise kernels (replaces the reference's five-branch shape table,
 // csrc/kernels/gemm.cu:136-161).  Model: the persistent grid runs ceil(tiles / slots) waves, and a wave costs the
@@ -992,9 +1014,7 @@ static int scaled_impl(const int8_t* x, const int8_t* y, const float* sx, const 
 {
     if (int rc = check_common(x, y, out, M, N, K, 2)) return rc;
     if (M == 0 || N == 0) return GI8_OK;
-    if (!sx || !sw) return fail(GI8_ERR_INVALID_ARGUMENT, "null scale pointer");
-    if (reinterpret_cast<uintptr_t>(sx) % 4 || reinterpret_cast<uintptr_t>(sw) % 4)
-        return fail(GI8_ERR_MISALIGNED, "scale pointers must be 4-byte aligned");
+    if (int rc = check_scale_pointers(sx, sw)) return rc;
     DeviceState* st;
     if (int rc = get_device_state(&st)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1058,9 +1078,7 @@ int gi8_matmul_scaled_static(const int8_t* x, const int8_t* y, const float* sx, 
     if (M > 128)
         return fail(GI8_ERR_UNSUPPORTED_SHAPE, "gi8_matmul_scaled_static covers M <= 128 only (got M=%lld); use "
                     "gi8_matmul_scaled", (long long)M);
-    if (!sx || !sw) return fail(GI8_ERR_INVALID_ARGUMENT, "null scale pointer");
-    if (reinterpret_cast<uintptr_t>(sx) % 4 || reinterpret_cast<uintptr_t>(sw) % 4)
-        return fail(GI8_ERR_MISALIGNED, "scale pointers must be 4-byte aligned");
+    if (int rc = check_scale_pointers(sx, sw)) return rc;
     DeviceState* st;
     if (int rc = get_device_state(&st)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1104,6 +1122,16 @@ static int check_quant(const void* in, int in_dtype, const int8_t* q, const floa
     return GI8_OK;
 }
 
+static int check_rotation(int64_t had_block, int64_t K)
+{
+    if (had_block < 128 || had_block > 8192 || (had_block & (had_block - 1)))
+        return fail(GI8_ERR_UNSUPPORTED_SHAPE, "rotation block %lld must be a power of two in [128, 8192]", (long long)had_block);
+    if (K % had_block)
+        return fail(GI8_ERR_UNSUPPORTED_SHAPE, "K=%lld must be a multiple of the rotation block %lld", (long long)K,
+                    (long long)had_block);
+    return GI8_OK;
+}
+
 int gi8_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream)
 {
     if (int rc = check_quant(in, in_dtype, q, scales, M, K)) return rc;
@@ -1130,11 +1158,7 @@ int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, f
                                       int64_t had_block, void* stream)
 {
     if (int rc = check_quant(in, in_dtype, q, scales, M, K)) return rc;
-    if (had_block < 128 || had_block > 8192 || (had_block & (had_block - 1)))
-        return fail(GI8_ERR_UNSUPPORTED_SHAPE, "rotation block %lld must be a power of two in [128, 8192]", (long long)had_block);
-    if (K % had_block)
-        return fail(GI8_ERR_UNSUPPORTED_SHAPE, "K=%lld must be a multiple of the rotation block %lld", (long long)K,
-                    (long long)had_block);
+    if (int rc = check_rotation(had_block, K)) return rc;
     if (M == 0 || K == 0) return GI8_OK;
     DeviceState* st;
     if (int rc = get_device_state(&st)) return rc;
@@ -1175,15 +1199,7 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (K == 0) return zero_output(out, M * N * (out_f32 ? 4 : 2), s);
     const int64_t KB = (K + kBK - 1) / kBK;
-    if (!sa || !sw) return fail(GI8_ERR_INVALID_ARGUMENT, "null scale pointer");
-    if (ld_sa < KB || ld_sw < KB)
-        return fail(GI8_ERR_INVALID_ARGUMENT, "scale row strides (%lld, %lld) must be at least ceil(K/128) = %lld",
-                    (long long)ld_sa, (long long)ld_sw, (long long)KB);
-    if (reinterpret_cast<uintptr_t>(sa) % 4 || reinterpret_cast<uintptr_t>(sw) % 4)
-        return fail(GI8_ERR_MISALIGNED, "scale pointers must be 4-byte aligned");
-    // The kernels index the scale arrays with 32-bit element offsets.
-    if (M * ld_sa >= (int64_t(1) << 31) || ((N + 127) / 128) * ld_sw >= (int64_t(1) << 31))
-        return fail(GI8_ERR_INVALID_ARGUMENT, "scale arrays of 2^31 or more elements are not supported");
+    if (int rc = check_block_scales(sa, ld_sa, sw, ld_sw, M, N, K)) return rc;
     BlockwiseParams p{};
     p.x = x, p.y = y;
     p.out = out, p.sa = sa, p.sw = sw, p.status = st->status, p.ldo = N, p.ld_sa = ld_sa, p.ld_sw = ld_sw;
@@ -1315,13 +1331,22 @@ int gi8_matmul_blockwise(const int8_t* x, const int8_t* y, const float* sa, int6
 int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale, int64_t ld_sw, const void* bias, int blockwise,
                int64_t had_block, int8_t* xq, float* xs, void* out, int64_t M, int64_t N, int64_t K, void* stream)
 {
-    // Everything that the GEMM refuses is refused before the quantiser is launched.
+    // Everything that the quantiser or the GEMM refuses is refused before the quantiser is launched: after a refusal nothing is
+    // under way that writes xq and xs.  (An empty problem with a bad rotation block is refused as the quantiser refuses it.)
     if (int rc = check_common(xq, w, out, M, N, K, 2)) return rc;
     if (int rc = check_quant(x, x_dtype, xq, xs, M, K)) return rc;
     if (had_block && !blockwise) return fail(GI8_ERR_INVALID_ARGUMENT, "a rotation needs block scales");
+    if (had_block)
+        if (int rc = check_rotation(had_block, K)) return rc;
     if (reinterpret_cast<uintptr_t>(bias) % 2) return fail(GI8_ERR_MISALIGNED, "bias must be 2-byte aligned");
     if (M == 0 || N == 0) return GI8_OK;
     if (K == 0 && bias) return fail(GI8_ERR_UNSUPPORTED_SHAPE, "K must be positive for a product with a bias");
+    const int64_t ld_xs = (K + kBK - 1) / kBK;
+    if (!blockwise) {
+        if (int rc = check_scale_pointers(xs, w_scale)) return rc;
+    } else if (K > 0) {
+        if (int rc = check_block_scales(xs, ld_xs, w_scale, ld_sw, M, N, K)) return rc;
+    }
     if (!blockwise && g_forced_variant == VAR_SMALLM)
         return fail(GI8_ERR_WORKSPACE, "the scratch variant needs a workspace; call the quantiser and gi8_matmul_scaled");
     const uint16_t* b = static_cast<const uint16_t*>(bias);
@@ -1332,7 +1357,7 @@ int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale
     if (int rc = had_block ? gi8_hadamard_quantize_token_block(x, x_dtype, xq, xs, M, K, had_block, stream)
                            : gi8_quantize_token_block(x, x_dtype, xq, xs, M, K, stream))
         return rc;
-    return blockwise_dispatch(xq, w, xs, (K + 127) / 128, w_scale, ld_sw, out, M, N, K, stream, b, K > 0);
+    return blockwise_dispatch(xq, w, xs, ld_xs, w_scale, ld_sw, out, M, N, K, stream, b, K > 0);
 }
 
 int gi8_matmul_blockwise_f32(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw,

@@ -89,6 +89,36 @@ def test_host_side_validation_without_gpu():
     assert C.gi8_peer_alloc(None, 16) == 1 and C.gi8_peer_export(None, None) == 1 and C.gi8_peer_import(None, None) == 1
 
 
+@pytest.mark.parametrize("blockwise", [0, 1])
+def test_linear_refuses_before_it_launches(blockwise):
+    """What the product of a linear layer refuses is refused before its quantiser is queued: without a device the first launch
+    fails with GI8_ERR_CUDA, so any other status was given in front of it."""
+    import gemm_int8_b200 as g
+
+    C = g._C
+    buf = ctypes.create_string_buffer(8192 + 64)
+    base = (ctypes.addressof(buf) + 63) & ~63
+    p = ctypes.c_void_p
+
+    def status(w_scale=base, ld=2, bias=None, had=0, xq=base, xs=base, M=8, N=8, K=256):
+        return C.gi8_linear(p(base), 1, p(base), p(w_scale), ld, p(bias), blockwise, had, p(xq), p(xs), p(base), M, N, K, None)
+
+    assert status(w_scale=None) == 1 and b"null scale" in C.gi8_last_error()
+    assert status(w_scale=base + 2) == 3
+    assert status(bias=base + 1) == 3
+    assert status(xq=base + 8) == 3 and status(xs=base + 2) == 3
+    assert status(K=0, bias=base) == 2
+    assert status(M=0) == 0 and status(N=0) == 0
+    if blockwise:
+        assert status(ld=1) == 1 and b"row strides" in C.gi8_last_error()
+        assert status(ld=1 << 31) == 1 and b"2^31" in C.gi8_last_error()
+        assert status(had=384) == 2 and status(had=512) == 2
+        # an empty batch does not excuse a rotation block that the quantiser refuses
+        assert status(had=384, M=0) == 2 and status(had=384, N=0) == 2
+    else:
+        assert status(had=128) == 1
+
+
 def test_ops_registered_under_reference_names():
     import gemm_int8  # noqa: F401  (the drop-in package name)
 
