@@ -67,10 +67,11 @@ class Int8Linear(torch.nn.Module):
             x2 = x2.to(torch.bfloat16)
         weight, bias = self.weight_q, self.bias
         # The bias goes into the product's epilogue where it is the plain vector of a layer.  One that broadcasts in some
-        # other way, that is differentiated, or K = 0 takes the tensor addition.
+        # other way, that is differentiated (a Parameter while gradients are recorded, forward mode), or K = 0 takes the
+        # tensor addition.
         fused = bias
-        if bias is not None and (bias.shape != weight.shape[:1] or bias.requires_grad or weight.shape[1] == 0
-                                 or forward_ad._current_level >= 0):
+        if bias is not None and (bias.shape != weight.shape[:1] or (bias.requires_grad and torch.is_grad_enabled())
+                                 or weight.shape[1] == 0 or forward_ad._current_level >= 0):
             fused = None
         out = torch.ops.gemm_int8_CUDA.int8_linear(x2, weight, self.weight_scale, fused, self.mode == "blockwise", self.hadamard_block)
         if bias is not None and fused is None:
