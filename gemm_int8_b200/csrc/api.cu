@@ -563,18 +563,22 @@ TailPlan plan_tail(int64_t M, int64_t N, int64_t K, bool pair, double form_cycle
 }
 
 // The automatic choice for the dense entry points: tile form, and whether (part of) its grid goes to the split-K kernel.
-// A narrow-tile choice (few tiles) is also weighed against splitting the whole one-CTA 256-wide grid.
+// A narrow-tile choice (few tiles) is also weighed against splitting the whole one-CTA 256-wide grid.  The split-K kernel writes
+// bf16 in 8-byte pieces: without can_split (int32 results, rows that are not 16-byte aligned) the tile form runs by itself, and a
+// thin grid must keep its narrow tiles.  (Taking the wide form for a split that then could not run cost 200 x 4097 x 28672 86.7
+// instead of 55.6 us, 100 x 1001 x 8192 24.3 instead of 18.0, and 128 x 1000 x 28672 as int32 74.2 instead of 54.3.)
 struct DenseChoice {
     int bn;
     bool pair;
     TailPlan tail;
 };
 
-DenseChoice choose_dense(int64_t M, int64_t N, int64_t K, int sms)
+DenseChoice choose_dense(int64_t M, int64_t N, int64_t K, int sms, bool can_split)
 {
     DenseChoice c{};
     double cost = 0.0;
     c.bn = pick_bn(M, N, K, sms, false, &c.pair, &cost);
+    if (!can_split) return c;
     if (c.bn == 256) {
         c.tail = plan_tail(M, N, K, c.pair, c.pair ? kDenseForms[0].kblock_cycles : kDenseForms[1].kblock_cycles, sms);
     } else {
@@ -598,7 +602,7 @@ int dispatch_dense(DeviceState* st, const int8_t* x, const int8_t* y, DenseParam
         case VAR_DENSE_BN128: bn = 128; break;
         case VAR_DENSE_BN64: bn = 64; break;
         default: {
-            const DenseChoice c = choose_dense(p.M, p.N, p.K, st->sm_count);
+            const DenseChoice c = choose_dense(p.M, p.N, p.K, st->sm_count, EPI != EPI_RAW_I32 && p.vec_ok);
             bn = c.bn, pair = c.pair, t = c.tail;
         }
     }
@@ -880,7 +884,7 @@ const char* gi8_pick_variant(int kind, int64_t M, int64_t N, int64_t K)
         if (c.split.use) return c.split.bn_tail == 128 ? "blockwise_bn256+columns_bn128" : "blockwise_bn256+columns_bn64";
         return pair ? "blockwise_pair" : bn == 256 ? "blockwise_bn256" : bn == 128 ? "blockwise_bn128" : "blockwise_bn64";
     }
-    const DenseChoice c = choose_dense(M, N, K, sms);
+    const DenseChoice c = choose_dense(M, N, K, sms, N % 8 == 0);  // (of an output that is 16-byte aligned)
     const bool pair = c.pair;
     const int bn = c.bn;
     if (c.tail.use) {
