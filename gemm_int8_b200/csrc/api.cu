@@ -24,6 +24,7 @@ using namespace gi8;
 
 constexpr int kMaxDevices = 64;
 constexpr int64_t kMaxK = 131072;  // |acc| <= 128*128*K must stay below 2^31 (no saturation modelled)
+constexpr int kSmallMMaxM = 64;  // the automatic dispatch sends M <= 64 to the small-M kernel
 
 thread_local char g_err[512] = "";
 
@@ -432,6 +433,26 @@ int launch(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t stre
     return GI8_OK;
 }
 
+// When a launch lets the next one start: as soon as its CTAs have waited (early), or as they end (late).  Early, the next grid's CTAs
+// sit down wherever an SM is free and in the order in which SMs become free; late, they find the machine empty and take the
+// hardware's own order.  The difference is where neighbouring tiles, which read the same rows, run, and it shows most where rows
+// are not whole 32-byte sectors (K % 32 != 0), because then every 128-byte piece of a row lies in two lines.  So one-CTA tiles
+// release early where the next grid fits beside this one and late where it does not.  us a call, back to back, operands beyond L2,
+// ordinary launches / early / late:
+//   100 x 5003 x 6992 dense 21.0 / 23.8 / 19.4, blockwise 22.7 / 25.7 / 20.4 (79 tiles); 100 x 13952 x 6992 dense 31.1 / 32.5 / 28.9 (109);
+//   100 x 28672 x 4096 blockwise 30.5 / 28.6 / 27.4 (112); waves: 3000 x 13952 x 6992 blockwise 415 / 430 / 412;
+//   but 64 tiles, which fit twice: 20 x 4096 x 4096 blockwise 18.5 / 15.5 / 16.3.
+// Early stay: aligned rows in several waves (1500 x 13952 x 7040 blockwise 195 / 189 / 193) and dense tiles in several waves (777 x 28672 x
+// 4112 141 / 140 / 139); dense and narrow blockwise tiles behind the quantiser of a layer (777 x 5003 x 6992 with its quantiser early 50.9,
+// late 54.3; 4 x 13952 x 14352 blockwise 68 / 69, in another run 74 / 80); two-CTA tiles (1500 x 13952 x 6992 dense 161 / 144 / 156, one wave
+// within 2.5 %); split-K grids (level); the first of two launches of one product, whose second is to start as SMs free up.
+// A quantiser releases late in front of several waves of one-CTA 256-wide tiles over rows that are not whole sectors, where the order
+// is worth more than the overlap; with the quantiser, ordinary / early / late: 777 x 13952 x 6992 blockwise 131 / 139 / 126, 300 x 13952 x
+// 6992 78 / 81 / 74, 777 x 28672 x 4112 per channel 142 / 141 / 139.  In front of narrow tiles it is not (300 x 4096 x 6992 blockwise
+// 34.3 / 30.0 / 31.2), nor where K % 32 == 0 (2048 x 11008 x 4096 119 / 114 / 114), nor in front of two-CTA tiles (3000 x 4096 x 6992 per channel
+// 113 / 106 / 109).
+bool release_late(int64_t ctas, int sms) { return ctas > sms / 2; }
+
 // Tensor map over the bf16 output [M, N] (row stride ldo elements) for the epilogue's TMA stores: boxes of 32 rows x
 // box_cols columns, 64-byte swizzle (32 columns) or 128-byte swizzle (64 columns).
 int make_output_map(CUtensorMap* map, void* out, int64_t M, int64_t N, int64_t ldo, int box_cols = 32)
@@ -463,6 +484,7 @@ int launch_dense(DeviceState* st, int slot, const int8_t* x, const int8_t* y, De
     p.group_m = pick_group_m(p.K);
     const int64_t tiles = p.tile_end > 0 ? p.tile_end : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
     const int grid = static_cast<int>(tiles < st->sm_count ? tiles : st->sm_count);
+    p.release_late = p.tile_end == 0 && !p.after_quant && tiles <= st->sm_count && release_late(tiles, st->sm_count);
     return launch(kernel, dim3(grid), kDenseThreads, smem, stream, dim3(1), p.dependent, mx, my, mo, p);
 }
 
@@ -495,7 +517,7 @@ int launch_dense_pair(DeviceState* st, int slot, const int8_t* x, const int8_t* 
 // Split-K launch for tiles [tile_begin, tile_begin + units / halves) of the grid described by p (tiles_m, tiles_n,
 // group_m as the main launch set them).
 template <int EPI>
-int launch_dense_splitk(DeviceState* st, int slot, const int8_t* x, const int8_t* y, const DenseParams& p,
+int launch_dense_splitk(DeviceState* st, int slot, const int8_t* x, const int8_t* y, DenseParams p,
                         const SplitKParams& q, cudaStream_t stream)
 {
     constexpr size_t smem = static_cast<size_t>(kSplitKStages) * (kBM + kSplitKBN) * kBK + 1024;
@@ -504,6 +526,11 @@ int launch_dense_splitk(DeviceState* st, int slot, const int8_t* x, const int8_t
     CUtensorMap mx, my;
     if (int rc = make_operand_map(&mx, x, p.M, p.K, kBM)) return rc;
     if (int rc = make_operand_map(&my, y, p.N, p.K, kSplitKBN)) return rc;
+    // A lone grid in two splits over rows that are not whole sectors is an ordinary launch unless its quantiser is in front: its place
+    // in the machine (see release_late) counts for more than the overlap.  us, ordinary / dependent: 100 x 13952 x 14352 51.0 / 53.5,
+    // 70 x 14336 x 16400 53.3 / 55.4; but 20 x 13952 x 14352 49.5 / 48.0, with its quantiser 100 x 13952 x 14352 66.6 / 63.8, K a multiple of 32
+    // 100 x 13952 x 14336 47.3 / 45.1, and four splits 200 x 4096 x 14352 31.6 / 28.3.
+    if (q.splits == 2 && p.K % 32 != 0 && p.M > kSmallMMaxM && !p.after_quant) p.dependent = 0;
     return launch(kernel, dim3(q.units * q.splits), kDenseThreads, smem, stream, dim3(q.splits), q.after_main || p.dependent, mx, my, p, q);
 }
 
@@ -662,8 +689,6 @@ struct SmallMPlan {
     int64_t scratch_bytes, total_bytes;
 };
 
-constexpr int kSmallMMaxM = 64;  // the automatic dispatch sends M <= 64 to the small-M kernel
-
 SmallMPlan plan_smallm(int64_t M, int64_t N, int64_t K, int sms, bool forced, int max_splits = 1 << 30)
 {
     SmallMPlan pl{};
@@ -816,11 +841,11 @@ __global__ void sum_parts_bf16_kernel(const float* __restrict__ parts, int n_par
 }
 
 template <typename T>
-static int launch_quant_row(const T* in, int8_t* q, float* scales, int64_t M, int K, int blocks, cudaStream_t s)
+static int launch_quant_row(const T* in, int8_t* q, float* scales, int64_t M, int K, int blocks, bool late, cudaStream_t s)
 {
     const int64_t loads = (static_cast<int64_t>(K) * sizeof(T) + kQuantThreads * 16 - 1) / (kQuantThreads * 16);
     auto kernel = loads <= 2 ? quantize_token_row_kernel<T, 2> : loads <= 4 ? quantize_token_row_kernel<T, 4> : quantize_token_row_kernel<T, 8>;
-    return launch(kernel, dim3(blocks), kQuantThreads, 0, s, dim3(1), knobs().pdl, in, q, scales, M, K);
+    return launch(kernel, dim3(blocks), kQuantThreads, 0, s, dim3(1), knobs().pdl, in, q, scales, M, K, late);
 }
 
 template <typename T, int LOGH>
@@ -1065,6 +1090,7 @@ static int scaled_impl(const int8_t* x, const int8_t* y, const float* sx, const 
     p.vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (N % 8 == 0);
     p.pair_ok = (reinterpret_cast<uintptr_t>(out) % 4 == 0) && (N % 2 == 0);
     p.bias = bias, p.bias_vec = reinterpret_cast<uintptr_t>(bias) % 16 == 0;
+    p.after_quant = after_quant;
     return dispatch_dense<EPI_ROWCOL_BF16>(st, x, y, p, s);
 }
 
@@ -1136,7 +1162,8 @@ static int check_rotation(int64_t had_block, int64_t K)
     return GI8_OK;
 }
 
-int gi8_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream)
+// waves_behind (of both quantisers): the product behind runs in several waves of one-CTA 256-wide tiles (see release_late).
+static int quantize_token_block(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream, bool waves_behind)
 {
     if (int rc = check_quant(in, in_dtype, q, scales, M, K)) return rc;
     if (M == 0 || K == 0) return GI8_OK;
@@ -1151,11 +1178,18 @@ int gi8_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* sca
     int64_t blocks = (warps + kQuantThreads / 32 - 1) / (kQuantThreads / 32);
     const int64_t cap = static_cast<int64_t>(st->sm_count) * 16;
     if (blocks > cap) blocks = cap;
+    const bool late = waves_behind && K % 32 != 0 && release_late(blocks, st->sm_count);
     if (in_dtype == 0)
         return launch(quantize_token_block_kernel<float>, dim3(static_cast<int>(blocks)), kQuantThreads, 0, s, dim3(1), knobs().pdl,
-                      static_cast<const float*>(in), q, scales, M, static_cast<int>(K), KB);
+                      static_cast<const float*>(in), q, scales, M, static_cast<int>(K), KB, late);
     return launch(quantize_token_block_kernel<__nv_bfloat16>, dim3(static_cast<int>(blocks)), kQuantThreads, 0, s, dim3(1), knobs().pdl,
-                  static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), KB);
+                  static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), KB, late);
+}
+
+int gi8_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream)
+{
+    // (what follows is not known here; K decides between one- and two-CTA tiles of a long grid)
+    return quantize_token_block(in, in_dtype, q, scales, M, K, stream, (K + kBK - 1) / kBK < kBlockwiseForms[0].min_kb);
 }
 
 int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K,
@@ -1171,7 +1205,7 @@ int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, f
     return launch_hadamard_quant(static_cast<const __nv_bfloat16*>(in), q, scales, M * K, static_cast<int>(had_block), s);
 }
 
-int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream)
+static int quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream, bool waves_behind)
 {
     if (int rc = check_quant(in, in_dtype, q, scales, M, K)) return rc;
     if (M == 0 || K == 0) return GI8_OK;
@@ -1181,8 +1215,15 @@ int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, i
     int64_t blocks = M;
     const int64_t cap = static_cast<int64_t>(st->sm_count) * 8;
     if (blocks > cap) blocks = cap;
-    if (in_dtype == 0) return launch_quant_row(static_cast<const float*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
-    return launch_quant_row(static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), s);
+    const bool late = waves_behind && K % 32 != 0 && release_late(blocks, st->sm_count);
+    if (in_dtype == 0) return launch_quant_row(static_cast<const float*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), late, s);
+    return launch_quant_row(static_cast<const __nv_bfloat16*>(in), q, scales, M, static_cast<int>(K), static_cast<int>(blocks), late, s);
+}
+
+int gi8_quantize_token(const void* in, int in_dtype, int8_t* q, float* scales, int64_t M, int64_t K, void* stream)
+{
+    // (what follows is not known here; most products of many rows run on two-CTA tiles)
+    return quantize_token(in, in_dtype, q, scales, M, K, stream, false);
 }
 
 // gather != nullptr: the N-sharded form.  This GEMM's [M,N] result is columns [col0, col0 + N) of an [M, n_total]
@@ -1247,6 +1288,8 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     const int64_t tiles = static_cast<int64_t>(p.tiles_m) * p.tiles_n;
     const int slots = pair ? st->sm_count / 2 : st->sm_count;
     const int grid = static_cast<int>(tiles < slots ? tiles : slots) * (pair ? 2 : 1);
+    p.release_late = !pair && force_bn == 0 && !(p.after_quant && bn < 256) && (tiles <= st->sm_count || K % 32 != 0) &&
+                     release_late(tiles, st->sm_count);
     OutputMaps mo{};
     if (scatter) {
         // one fp32 map per rank over its receive area [n_out * R, N], boxes of 32 rows x 32 columns
@@ -1354,12 +1397,19 @@ int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale
     if (!blockwise && g_forced_variant == VAR_SMALLM)
         return fail(GI8_ERR_WORKSPACE, "the scratch variant needs a workspace; call the quantiser and gi8_matmul_scaled");
     const uint16_t* b = static_cast<const uint16_t*>(bias);
+    bool waves = false;  // several waves of one-CTA 256-wide tiles (asked only where the quantiser's rule looks at it)
+    if (K % 32 != 0) {
+        DeviceState* st;
+        if (int rc = get_device_state(&st)) return rc;
+        bool pair = false;
+        waves = ((M + kBM - 1) / kBM) * ((N + 255) / 256) > st->sm_count && pick_bn(M, N, K, st->sm_count, blockwise, &pair) == 256 && !pair;
+    }
     if (!blockwise) {
-        if (int rc = gi8_quantize_token(x, x_dtype, xq, xs, M, K, stream)) return rc;
+        if (int rc = quantize_token(x, x_dtype, xq, xs, M, K, stream, waves)) return rc;
         return scaled_impl(xq, w, xs, w_scale, out, M, N, K, nullptr, 0, stream, b, K > 0);
     }
     if (int rc = had_block ? gi8_hadamard_quantize_token_block(x, x_dtype, xq, xs, M, K, had_block, stream)
-                           : gi8_quantize_token_block(x, x_dtype, xq, xs, M, K, stream))
+                           : quantize_token_block(x, x_dtype, xq, xs, M, K, stream, waves))
         return rc;
     return blockwise_dispatch(xq, w, xs, ld_xs, w_scale, ld_sw, out, M, N, K, stream, b, K > 0);
 }

@@ -109,6 +109,7 @@ struct BlockwiseParams {
     const uint16_t* bias;  // bf16 [N] added to the rounded result (BIAS kernels)
     int bias_vec;   // bias is 16-byte aligned
     int after_quant;  // launched as the programmatic dependent of the quantiser that writes x and sa (and of nothing else)
+    int release_late; // do not let the next launch start before the CTAs have ended (see the host's release_late)
     int out_f32;    // store the fp32 accumulators themselves (out is float [M,N]) instead of their bf16 cast; the
                     // partial results of a K-sharded GEMM, and the bit-exact check of the accumulation order
 };
@@ -367,7 +368,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     // What follows in the stream may start as SMs free up, once this CTA has waited: the second of two launches, and a small-M
     // kernel with static weights, read before they wait themselves.  The thread is one of warp 1, which has waited in every
     // case; warp 0 has not where it requests weights early.
-    if (p.pdl_role != 2 && threadIdx.x == 32) pdl_launch_dependents();
+    if (p.pdl_role != 2 && !p.release_late && threadIdx.x == 32) pdl_launch_dependents();
 
     if (warp < 4) {
         setmaxnreg_dec<kControlRegs>();

@@ -54,6 +54,8 @@ struct DenseParams {
     float alpha;
     const uint16_t* bias; // bf16 [N] added to the rounded result, or null (EPI_ROWCOL_BF16)
     int bias_vec;         // bias is 16-byte aligned
+    int release_late;     // do not let the next launch start before the CTAs have ended (see the host's release_late)
+    int after_quant;      // (host) the launch in front is the quantiser that writes x and sx
     int dependent;        // launched as a programmatic dependent: wait for the kernel in front before the first access
 };
 
@@ -239,7 +241,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if (p.dependent) pdl_wait();
     // What follows in the stream may start as SMs free up.  Only after that wait: a split-K launch over the last tiles of this
     // grid reads x and y without waiting for anything itself.
-    if (threadIdx.x == 0) pdl_launch_dependents();
+    if (threadIdx.x == 0 && !p.release_late) pdl_launch_dependents();
 
     // The producer and the MMA issuer run their loops with the WHOLE warp (uniform control flow) and elect one lane
     // only around the TMA / MMA / commit instructions.  Inside an `if (lane == 0)` region the compiler treats

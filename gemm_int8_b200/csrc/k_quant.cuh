@@ -16,10 +16,11 @@ constexpr int kQuantThreads = 256;
 // First statement of every quantiser: it may have been started while the kernel before it was still running, so nothing
 // is read or written before that kernel has ended.  Only then may a dependent kernel start: the GEMM behind a quantiser
 // reads its weights without waiting for the quantiser, and must find what the kernel before the quantiser wrote.
-GI8_DEVICE void quant_dependency()
+// release_late: it may start only as the CTAs end (see the host's release_late).
+GI8_DEVICE void quant_dependency(bool release_late = false)
 {
     pdl_wait();
-    pdl_launch_dependents();
+    if (!release_late) pdl_launch_dependents();
 }
 
 GI8_DEVICE float warp_max(float v)
@@ -204,9 +205,9 @@ constexpr int kQuantBlocksPerItem = 8;  // 128-wide blocks per warp and iteratio
 template <typename T>
 __global__ void __launch_bounds__(kQuantThreads, 4)
 quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K,
-                            int KB)
+                            int KB, bool release_late)
 {
-    quant_dependency();
+    quant_dependency(release_late);
     constexpr int EPL = 16 / sizeof(T);   // elements per lane and load
     constexpr int LPB = 128 / EPL;        // lanes per 128-wide block
     constexpr int BPL = 32 / LPB;         // blocks per warp and load
@@ -263,9 +264,10 @@ quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, flo
 // a short row leaves unused would cost resident CTAs.
 template <typename T, int LOADS>
 __global__ void __launch_bounds__(kQuantThreads)
-quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K)
+quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K,
+                          bool release_late)
 {
-    quant_dependency();
+    quant_dependency(release_late);
     constexpr int EPL = 16 / sizeof(T);
     constexpr int kStep = kQuantThreads * EPL;
     __shared__ float warp_amax[2][kQuantThreads / 32];
