@@ -42,8 +42,26 @@ def _stale(target: str, sources: list[str]) -> bool:
     return any(os.path.exists(f) and os.path.getmtime(f) > t for f in sources)
 
 
+def _ops_tag() -> str:
+    """What the operator library is tied to besides its sources: it is compiled against one torch and one Python ABI."""
+    import sysconfig
+
+    import torch
+
+    return f"torch {torch.__version__} abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} {sysconfig.get_config_var('SOABI')}"
+
+
+def _built_for_other_torch() -> bool:
+    with open(OPS_PATH, "rb") as f:
+        return _ops_tag().encode() + b"\0" not in f.read()  # gi8_torch_ops_built_for of torch_ops.cpp
+
+
+def _ops_stale() -> bool:
+    return _stale(OPS_PATH, [OPS_SOURCE, HEADERS[-1]]) or _built_for_other_torch()
+
+
 def is_stale() -> bool:
-    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(OPS_PATH, [OPS_SOURCE, HEADERS[-1]])
+    return _stale(LIB_PATH, SOURCES + HEADERS) or _ops_stale()
 
 
 def _run(cmd: list[str], verbose: bool) -> None:
@@ -64,16 +82,17 @@ def _build_ops(verbose: bool) -> None:
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{d}" for d in include),
-          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", OPS_PATH, OPS_SOURCE,
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DGI8_BUILT_FOR="{_ops_tag()}"', "-o", OPS_PATH, OPS_SOURCE,
           f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
           f"-L{_PKG}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"], verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile both libraries if they are missing or older than their sources; returns the path of the first."""
+    """Compile both libraries if they are missing or older than their sources, the operators also if the installed torch or
+    Python is another one; returns the path of the first."""
     if force or _stale(LIB_PATH, SOURCES + HEADERS):
         _run([_nvcc(), *(["-Xptxas", "-v"] if verbose else []), *NVCC_FLAGS, "-o", LIB_PATH, *SOURCES], verbose)
-    if force or _stale(OPS_PATH, [OPS_SOURCE, HEADERS[-1]]):
+    if force or _ops_stale():
         _build_ops(verbose)
     return LIB_PATH
 

@@ -13,6 +13,12 @@
 
 #include "../../include/gemm_int8_b200.h"
 
+// The torch and Python this library was compiled against; _build.py compares it with what is installed.
+extern "C" {
+extern const char gi8_torch_ops_built_for[];
+const char gi8_torch_ops_built_for[] = GI8_BUILT_FOR;
+}
+
 namespace {
 
 constexpr int64_t kBlock = 128;

@@ -119,6 +119,15 @@ def test_linear_refuses_before_it_launches(blockwise):
         assert status(had=128) == 1
 
 
+def test_operator_library_is_stale_for_another_torch(monkeypatch):
+    """The operator library is tied to the installed torch's ABI: an upgrade must rebuild it although no source is newer."""
+    from gemm_int8_b200 import _build
+
+    assert not _build._built_for_other_torch()
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert _build._ops_stale()
+
+
 def test_ops_registered_under_reference_names():
     import gemm_int8  # noqa: F401  (the drop-in package name)
 
