@@ -194,13 +194,6 @@ GI8_DEVICE float chain_from_global(const int8_t* x, const int8_t* y, const float
     return acc;
 }
 
-GI8_DEVICE uint64_t splat_f32x2(float t)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(t));
-    return r;
-}
-
 // a * b (fp32, round to nearest) as a volatile statement: it keeps its place among the other volatile statements
 // (tensor-memory loads, conversions).  The scales are loaded two K blocks before their use; written as plain C++ the
 // compiler hoists the product up to the loads to save a register, and the warp then waits out the L2 latency right
@@ -227,16 +220,11 @@ GI8_DEVICE float mul_in_place(float a, float b)
     return r;
 }
 
-GI8_DEVICE void unpack_f32x2(uint64_t v, float& lo, float& hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // Two packed pairs (four consecutive columns) -> two bf16x2 words.
 GI8_DEVICE uint32_t pack_bf16x2_of(uint64_t pair)
 {
     float lo, hi;
-    unpack_f32x2(pair, lo, hi);
+    f32x2_split(pair, lo, hi);
     return pack_bf16x2(lo, hi);
 }
 
@@ -534,8 +522,8 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         // lay under that arithmetic.  Otherwise the bounded wait runs; the branch is taken on a vote, which makes it
         // warp-uniform.
         bool polled = false;
-        [[maybe_unused]] const uint64_t unbias_c2 = splat_f32x2(0x1p127f);
-        [[maybe_unused]] const uint64_t unbias_b2 = splat_f32x2(-static_cast<float>(kPartialBias) * 0x1p-22f);
+        [[maybe_unused]] const uint64_t unbias_c2 = f32x2(0x1p127f, 0x1p127f);
+        [[maybe_unused]] const uint64_t unbias_b2 = f32x2(-static_cast<float>(kPartialBias) * 0x1p-22f, -static_cast<float>(kPartialBias) * 0x1p-22f);
         // (so, sp): byte offset of the stage's barrier in its ring and the parity awaited there.
         auto wait_partial = [&](int h, uint32_t so, uint32_t sp) {
             if (!__all_sync(0xffffffffu, polled)) {
@@ -632,7 +620,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 for (int h = 0; h < SPLIT; ++h) {
                     if (!wait_partial(h, so, sp)) return false;
                     const float ts = BIASED ? t[h] * 0x1p22f : t[h];
-                    const uint64_t t2 = splat_f32x2(ts);
+                    const uint64_t t2 = f32x2(ts, ts);
                     const uint32_t taddr = tm_warp + bc + h * NSUB;
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
@@ -756,10 +744,10 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                         for (int j = 0; j < CW / 2; ++j) {
                             float lo, hi;
-                            unpack_f32x2(acc[j], lo, hi);
+                            f32x2_split(acc[j], lo, hi);
                             if (c == 2 * j) lo = r;
                             if (c == 2 * j + 1) hi = r;
-                            asm("mov.b64 %0, {%1, %2};" : "=l"(acc[j]) : "f"(lo), "f"(hi));
+                            acc[j] = f32x2(lo, hi);
                         }
                     }
                     __syncwarp();
@@ -871,7 +859,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                             for (int j = 0; j < SEGW / 2; ++j) {
                                 float lo, hi;
-                                unpack_f32x2(a[j], lo, hi);
+                                f32x2_split(a[j], lo, hi);
                                 if (c0 + 2 * j < p.N) dst[2 * j] = lo;
                                 if (c0 + 2 * j + 1 < p.N) dst[2 * j + 1] = hi;
                             }

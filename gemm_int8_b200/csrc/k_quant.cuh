@@ -49,15 +49,7 @@ GI8_DEVICE QuantScale make_quant_scale(float amax)
     return qs;
 }
 
-// Packed fp32 pairs (element 0 in the low half): one instruction for two elements; each half rounds like the scalar
-// instruction.
-GI8_DEVICE uint64_t f32x2(float lo, float hi)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-GI8_DEVICE void f32x2_split(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+// Arithmetic on packed fp32 pairs: one instruction for two elements; each half rounds like the scalar instruction.
 GI8_DEVICE uint64_t add2(uint64_t a, uint64_t b)
 {
     uint64_t r;

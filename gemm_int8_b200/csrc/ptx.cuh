@@ -341,6 +341,15 @@ GI8_DEVICE uint32_t pack_bf16x2(float lo, float hi)
 }
 
 
+// A pair of fp32 values in one 64-bit register (element 0 in the low half), as the packed instructions take them.
+GI8_DEVICE uint64_t f32x2(float lo, float hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+GI8_DEVICE void f32x2_split(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+
 // max(|a|, |b|, |c|): ignoring NaN, and propagating it.
 GI8_DEVICE float max3_abs(float a, float b, float c)
 {
