@@ -55,8 +55,8 @@ std::atomic<int> g_forced_variant{VAR_AUTO};
 // read once, when the library is first used, and again only when gi8_reload_env() is called: nothing on the launch
 // path calls getenv.
 //   GEMM_INT8_GROUP_M    = 1..64   row-blocks per rasterisation band (default: fitted to K)
-//   GEMM_INT8_TMA_STORE  = 0       bf16 epilogues store from registers instead of through shared memory + TMA
-//   GEMM_INT8_PDL        = 0       no programmatic dependent launch anywhere (small-M kernels, second launches of a GEMM)
+//   GEMM_INT8_TMA_STORE  = 0       bf16 blocks staged in shared memory are written row by row instead of by TMA stores
+//   GEMM_INT8_PDL        = 0       ordinary, fully ordered launches everywhere (quantisers and products)
 //   GEMM_INT8_SPLITS     = n       small-M kernels: number of K splits
 //   GEMM_INT8_BW_HALVES  = 1 | 2   blockwise 256-wide tile: MMAs with N = 256, or two column halves with N = 128 (default)
 //   GEMM_INT8_BW_ISSUERS = 1 | 2   blockwise kernel without column halves: MMA-issuing threads (default: one for the
@@ -65,8 +65,8 @@ std::atomic<int> g_forced_variant{VAR_AUTO};
 //                                  of a tile grid to a second launch: the split-K kernel (dense entry points; also a whole
 //                                  thin grid), narrower tiles over the remaining columns (blockwise entry point)
 // and one promise by the host rather than a knob:
-//   GEMM_INT8_STATIC_WEIGHTS = 1   the weight operand of the small-M path is not written by the work that directly
-//                                  precedes the call in its stream: its first tiles may be requested early
+//   GEMM_INT8_STATIC_WEIGHTS = 1   the weight operand of the scaled product is not written by the work that directly precedes
+//                                  the call in its stream: the small-M kernel may request its first tiles early
 struct Knobs {
     int group_m = 0;
     bool tma_store = true;
@@ -74,8 +74,8 @@ struct Knobs {
     int splits = 0;
     int bw_halves = 0;   // 0: column halves
     int bw_issuers = 0;  // 0: one for the 256-wide tile, two for the narrower ones
-    // The caller promises that the weight operand of the small-M path is not written by the kernel that precedes the
-    // call in its stream (weights quantised ahead of time): its first tiles are then requested before that kernel ends.
+    // The caller promises that the weights of the scaled product are not written by the kernel that precedes the call in its
+    // stream (quantised ahead of time): the small-M kernel then requests its first tiles before that kernel ends.
     bool static_weights = false;
     int tail_split = 1;  // dense kernels: 0 never split K, 1 when the model says it pays, 2 whenever it is possible
 };
@@ -268,13 +268,17 @@ int check_block_scales(const float* sa, int64_t ld_sa, const float* sw, int64_t 
 // form's cycles per K block, fitted on B200 from device-timed runs (8192^3, 2048 x 11008 x 4096, 128..512 x 8192 x
 // 8192 and the reference benchmark's layer shapes, timed back to back):
 //   dense      256 x 256 two-CTA tile (74 slots) 580 | 128 x 256: 655 | 128 x 128: 465 | 128 x 64: 330
-//   blockwise  128 x 256: 950 | 256 x 256 two-CTA tile: 920 | (fitted when both converted their partials; without conversions
-//              both take 3 to 6 % less, the order stands).  The two-CTA tile gains by fewer operand bytes per MAC, which counts
-//              the longer the run and the longer K: 0.15 s of back-to-back calls, one-CTA against two-CTA, 2048 x 8192 x
-//              28672 577 -> 549 us, 4096 x 4096 x 14336 285 -> 275, 700 x 9000 x 12288 115 -> 111, 1024 x 4096 x 14336 72.5 ->
-//              70.9, 2048 x 11008 x 4096 110.1 -> 107.9; in short bursts, below the power cap, level up to 8192^3.  Hence its
-//              minimum: twenty waves, or 96 K blocks
-//              | 128 x 128: 650 | 128 x 64: 490
+//   blockwise  128 x 256: 950 | 256 x 256 two-CTA tile: 920 | 128 x 128: 650 | 128 x 64: 490 (fitted when the wide forms still converted
+//              their partials; us per wave and K block between K = 4096 and 16384 since then: 0.56 | 0.56 | 0.37 | 0.27 on full
+//              waves, 0.44 | 0.44 | 0.30 | 0.22 on 32 to 128 CTAs: the same ranking).
+//              The two-CTA tile gains by fewer operand bytes per MAC, which counts the longer the run and the longer K.  0.12 s of
+//              back-to-back calls, one-CTA / two-CTA us, for K = 4096, 6144, 8192, 10240, 12288, 16384:
+//                512 x 8192    23.1/24.2  32.5/33.8  42.8/43.1  52.6/52.6  62.3/62.1  81.2/81.1
+//                1024 x 4096   21.9/22.8  31.7/32.7  41.2/41.7  50.8/50.7  60.6/60.0  79.2/78.8
+//                2048 x 8192   82.7/82.8  120/119    157/154    197/194    235/232    312/307
+//                2048 x 11008  107/106    154/153    200/199    257/250    306/305    414/404
+//              In short bursts, below the power cap, it is level or up to 1 % behind at all of them.  Hence its minimum: twenty
+//              waves, or 96 K blocks, from which on it is not behind on any of these grids in a long run.
 // The table is data: kDenseForms / kBlockwiseForms below.  The narrow tiles cost more per column (the tensor-core instruction is issue
 // bound below N = 128, and the per-K-block hand-overs do not shrink with the tile) and only pay when the wide tile
 // would leave most SMs without work.
@@ -327,14 +331,15 @@ int pick_group_m(int64_t K)
     return static_cast<int>(g);
 }
 
-// A blockwise tile cannot split K (the accumulation order is part of the result), so a grid of W full waves plus a few
+// Blockwise tiles do not split K (their fp32 chain runs in K order across the whole K), so a grid of W full waves plus a few
 // tiles would pay W + 1 waves.  Where the full waves are whole column bands (W x SMs divisible by the row-block count),
 // the columns are split instead: the first launch covers the columns of the W full waves with 128 x 256 tiles, a second
 // launch covers the rest with the widest narrower tile that fits one wave -- more CTAs, each costing less per K block
 // (cycles of kBlockwiseForms).  The second launch reads nothing the first writes, so it is released as the first one's
 // CTAs leave (programmatic dependent launch without a wait before its work; it waits before it ends, see
 // BlockwiseParams::pdl_role).  kColumnSplitFixedCycles: set-up and epilogue of the second kernel's CTAs.  Measured on
-// B200, L2-cold: 512 x 10240 x 8192 (160 tiles) 75.8 -> 66.6 us, 512 x 57344 x 8192 256 -> 243, 2048 x 10240 x 8192 204 -> 196.
+// B200, back to back: 512 x 10240 x 8192 (160 tiles) 75.5 -> 60.1 us, 512 x 10240 x 16384 148 -> 112, 512 x 57344 x 8192 302 -> 277,
+// 2048 x 10240 x 8192 202 -> 192.
 constexpr double kColumnSplitFixedCycles = 10000.0;  // measured: a lone 64-wide launch of 64 K blocks takes 5 us more than its K blocks
 struct ColumnSplit {
     bool use;
@@ -435,9 +440,10 @@ int launch(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t stre
 
 // When a launch lets the next one start: as soon as its CTAs have waited (early), or as they end (late).  Early, the next grid's CTAs
 // sit down wherever an SM is free and in the order in which SMs become free; late, they find the machine empty and take the
-// hardware's own order.  The difference is where neighbouring tiles, which read the same rows, run, and it shows most where rows
-// are not whole 32-byte sectors (K % 32 != 0), because then every 128-byte piece of a row lies in two lines.  So one-CTA tiles
-// release early where the next grid fits beside this one and late where it does not.  us a call, back to back, operands beyond L2,
+// hardware's own order.  What differs is only where neighbouring tiles, which read the same rows, run; it shows most where rows
+// are not whole 32-byte sectors (K % 32 != 0), so that every 128-byte piece of a row lies in two lines (staggered starts of
+// the CTAs changed nothing, a release at a CTA's last load half as much; the traffic itself was not measured).  So one-CTA tiles release
+// early where the next grid fits beside this one and late where it does not.  us a call, back to back, operands beyond L2,
 // ordinary launches / early / late:
 //   100 x 5003 x 6992 dense 21.0 / 23.8 / 19.4, blockwise 22.7 / 25.7 / 20.4 (79 tiles); 100 x 13952 x 6992 dense 31.1 / 32.5 / 28.9 (109);
 //   100 x 28672 x 4096 blockwise 30.5 / 28.6 / 27.4 (112); waves: 3000 x 13952 x 6992 blockwise 415 / 430 / 412;
@@ -719,7 +725,9 @@ constexpr int kMaxClusterSplits = 8;  // portable thread-block cluster size
 // beyond L2, dense against small-M): always up to 16 tokens (16 x 4096 x 14336 29.8 -> 12.3 us, 16 x 14336 x 4096 20.6 -> 13.7,
 // 16 x 57344 x 14336 135 -> 123, 16 x 1000 x 1024 4.5 -> 3.4); above, where K is long and cut into eight splits, or seven (64 x 4096 x 14336
 // 30.0 -> 15.1, 64 x 4096 x 4096 10.8 -> 9.1, 64 x 1000 x 4096 9.9 -> 6.4).  Elsewhere the reduction, or the wider token tile, costs more
-// than it gains (64 x 4096 x 1024 4.7 -> 7.6, 64 x 14336 x 4096 13.7 -> 18.1).
+// than it gains (64 x 4096 x 1024 4.7 -> 7.6, 64 x 14336 x 4096 13.7 -> 18.1).  The line at K = 4096 lies on the safe side: with up to 4096
+// columns the small-M kernel is ahead from 3072 on (64 x 4096 x 3072 8.8 -> 8.1, 64 x 1000 x 3072 8.6 -> 6.3), at 2048 it depends on the
+// columns (64 x 4096 x 2048 6.9 -> 7.4, 64 x 1000 x 2048 6.7 -> 5.9), at 1024 it is behind (64 x 1000 x 1024 4.4 -> 6.7).
 SmallMPlan plan_smallm_plain(int64_t M, int64_t N, int64_t K, int sms)
 {
     SmallMPlan pl = plan_smallm(M, N, K, sms, false, kMaxClusterSplits);

@@ -24,11 +24,11 @@
 //   SPLIT == 1 (narrow tiles): two cvt.rn.f32.s32 and one fma.rn.f32x2 per pair (promote_pair).
 // Conversions take the half-rate integer pipe two cycles each, and they, the multiply-adds and the tensor-memory loads of
 // a scheduler do not overlap as freely as their pipes would allow: with conversions alone or multiply-adds alone the
-// kernel ran at the speed of its MMAs, with both a third slower.  Measured, conversions -> bias (one MMA in four more included):
-// 2048 x 11008 x 4096 98.9 -> 96.1 us, 512 x 8192 x 8192 53.4 -> 51.0, 8192^3 615 -> 589, 2048 x 8192 x 28672 594 -> 568,
-// 16384 x 57344 x 8192 8.64 -> 8.16 ms (back to back, so the long ones under the power cap).  A fixed mixture (half of the
-// columns converted) was slower than either, and so was a branch for the scale products the trick does not cover inside
-// the K loop (15-20 %): they are looked for once per tile.
+// kernel ran at the speed of its MMAs, with both a third slower.  Measured in one build, N = 256 MMAs with conversions
+// (GEMM_INT8_BW_HALVES=1) -> column halves with the bias (one MMA in four more included): 2048 x 11008 x 4096 115 -> 107 us, 512 x 8192 x
+// 8192 46.6 -> 42.9, 8192^3 630 -> 582, 16384 x 57344 x 8192 9.15 -> 7.93 ms (back to back, so the long ones under the power cap).  A
+// fixed mixture (half of the columns converted) was slower than either, and so was a branch for the scale products the trick
+// does not cover inside the K loop (15-20 %): they are looked for once per tile.
 //
 // Why eight fat warps (measured on B200 with a stand-alone loop of the same instructions, cycles per 128 x 256
 // K block, tensor core busy in the background): a tcgen05.ld costs about one cycle per 32-lane column whatever its
@@ -36,11 +36,11 @@
 // counts is instructions issued.  16 warps x 64 columns with 16-column loads and a biased accumulator written
 // back with tcgen05.st: 860-920.  8 warps x 128 columns, 32-column loads: biased accumulator with write-back 665-685
 // (the stores alone cost 140), cvt + fma.f32x2 without any write-back 545-580, against 512 for the MMAs.
-// The same was measured in this kernel itself, with the column groups made a template parameter: twelve promotion
+// The same was measured in this kernel itself (with conversions), the column groups made a template parameter: twelve promotion
 // warps (three per scheduler) on a 128 x 192 tile ran 15-20 % slower than eight on 128 x 256, sixteen (four per
 // scheduler, 112 registers each, 16-column loads) 40-50 % slower -- every warp repeats the per-K-block bookkeeping
 // (barrier test, hand-back, scale product, counters), and those instructions share the half-rate integer pipe
-// with the conversions, which is the busiest unit (two cycles per cvt.rn.f32.s32: 512 of the K block's cycles).
+// with the conversions, which was the busiest unit (two cycles per cvt.rn.f32.s32: 512 of the K block's cycles).
 //
 // Barrier protocol (every wait is a parity wait, so it must hold that a barrier cannot complete a second phase
 // before the waiter has consumed the first; the comment at each barrier says what gates its next phase):

@@ -1,8 +1,8 @@
 // Activation quantisers: the step that feeds the W8A8 GEMMs.  The reference ships none (its benchmark only rounds
 // and clamps, benchmark.py:17-18); these follow the package's torch quantisers bit for bit:
 //     s = amax / 127  (s = 1 where the block is all zero),  q = clamp(rint(v / s), -127, 127)
-// with IEEE division and round-half-even.  Both kernels are HBM-bound streams (5 bytes per fp32 element,
-// 3 per bf16 element): every element is read once with 16-byte loads and written once.
+// with IEEE division and round-half-even.  Every element is read once with 16-byte loads and written once (5 bytes per fp32
+// element, 3 per bf16 element; the row quantiser reads what does not fit its registers twice).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -188,8 +188,9 @@ GI8_DEVICE void group_scales(float (&m)[U], float (&s)[U], float (&r)[U])
 // quarter of the copy bandwidth).  The loaded 16 bytes stay in registers as they came (four registers per load whatever
 // the type) and are unpacked at each use: a byte in flight costs a register byte.  fp32 input takes eight loads per lane,
 // bf16 input, which is closer to the bound of instruction issue, four.
-// Bound: HBM for fp32 (16384 x 8192: 121 -> 111 us, 6.0 TB/s), instruction issue for bf16 (103 -> 90.5 us, 4.4 TB/s), in both
-// with the packed arithmetic and one division per lane instead of one or two per block and lane (group_scales).
+// Bound: HBM for fp32 (16384 x 8192: 128 -> 113 us, 6.0 TB/s, 0.91 of the copy bandwidth); for bf16 (103 -> 88 us, 4.6 TB/s, 0.71) no
+// single unit: 16 instructions an element issue on 68 % of the cycles, the integer pipe is at 54 %, and warps wait for their
+// loads.  Both with the packed arithmetic and one division per lane instead of one or two per block and lane (group_scales).
 // a [M,K] (K % EPL == 0, rows 16-byte aligned) -> q int8 [M,K], s fp32 [M, ceil(K/128)].
 constexpr int kQuantBlocksPerItem = 8;  // 128-wide blocks per warp and iteration, whatever the type (1 x 8 or 2 x 4)
 
@@ -254,6 +255,8 @@ quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, flo
 // the maximum and the quantisation, so that the row is read once; what lies beyond them is read again (it hits L1 or L2).
 // The host takes the smallest of 2, 4 and 8 that holds the row (eight: 16384 bf16 or 8192 fp32 elements): registers that
 // a short row leaves unused would cost resident CTAs.
+// 16384 x 8192, row read twice -> held in registers: fp32 149 -> 102 us (6.6 TB/s), bf16 126 -> 88.5 (4.5 TB/s; issue 60 %, the rest waits
+// for loads and the barrier of a row).  Beyond the registers the second read stays: 8192 x 28672 bf16 211 -> 209 us (3.4 TB/s), fp32 322 -> 246.
 template <typename T, int LOADS>
 __global__ void __launch_bounds__(kQuantThreads)
 quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K,
@@ -321,9 +324,10 @@ quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float
 // Stages on bits 0-2 run in L, the middle ones in M, the top ones back in L: four shared-memory accesses an element,
 // where a chain of five shuffle stages and up to three shared-memory stages took up to eleven, each with its selects.
 // Words are padded and bit 2 of the word index is flipped by bit 5, which makes both arrangements free of bank conflicts.
-// Measured, before and after: 2048 x 28672 bf16, H = 4096, 118 -> 60 us (2.9 TB/s); 499 x 8192 fp32, H = 8192, 18.5 -> 11.3 us;
-// 4096 x 8192 bf16, H = 128, 140 -> 35 us.  What bounds it now is instruction issue and the shared-memory passes: 13 packed
-// additions, four shared-memory accesses and about ten instructions of quantisation for 3 or 5 bytes.
+// Measured, before and after: 2048 x 28672 bf16, H = 4096, 115 -> 56 us (3.1 TB/s); 499 x 8192 fp32, H = 8192, 18.4 -> 8.9 us;
+// 4096 x 8192 bf16, H = 128, 137 -> 32 us.  What bounds it now is no single unit either: at 8192 x 8192 bf16 and H = 8192 23
+// instructions an element issue on 62 % of the cycles, the load-store pipe (shared memory above all, 3 % of its accesses in conflict) is
+// at 46 %, and 96 registers allow five CTAs of four warps.
 template <int LOGH>
 struct HadamardShape {
     static constexpr int LOGU = LOGH < 11 ? 11 : LOGH;

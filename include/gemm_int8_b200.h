@@ -205,11 +205,11 @@ int gi8_hadamard_quantize_token_block(const void* in, int in_dtype, int8_t* q, f
  *   had_block  0, or the rotation block of gi8_hadamard_quantize_token_block (blockwise 1 only)
  *   xq, xs   scratch that receives the quantised activations and their scales: int8 [M,K] (16-byte aligned) and fp32 [M] or
  *            [M, ceil(K/128)]
- * Results are those of the quantiser, gi8_matmul_scaled or gi8_matmul_blockwise, and a bf16 addition, bit for bit.
+ * Results are those of the quantiser, gi8_matmul_scaled or gi8_matmul_blockwise, and a bf16 addition, bit for bit.  Whatever either
+ * step refuses is refused before the first launch.
  */
 int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale, int64_t ld_sw, const void* bias_bf16, int blockwise,
                int64_t had_block, int8_t* xq, float* xs, void* out_bf16, int64_t M, int64_t N, int64_t K, void* stream);
-
 
 /*
  * Forces a kernel variant for the calling process (tuning and tests); NULL or "" restores the fitted
@@ -225,7 +225,7 @@ int gi8_force_variant(const char* name);
  * read "blockwise_bn256", "blockwise_bn128", "blockwise_bn64", "blockwise_pair", and "blockwise_bn256+columns_bnW" where
  * the columns of the thin last wave go to a second launch with W-wide tiles).  For the dense kernels "+splitkS"
  * after a form's name means that the tiles of its last wave go to the split-K kernel with S splits, and "splitkS" alone
- * that the whole grid does. */
+ * that the whole grid does (an output that is 16-byte aligned is assumed). */
 const char* gi8_pick_variant(int kind, int64_t M, int64_t N, int64_t K);
 
 /*
@@ -258,7 +258,8 @@ int gi8_selftest_wait_timeout(void* stream);
  * GEMM_INT8_STATIC_WEIGHTS=1 (default 0) is a promise rather than a tuning: the weight operand of gi8_matmul_scaled's
  * small-M path is not written by the work that directly precedes the call in its stream (weights quantised ahead of
  * time), so the kernel may request its first weight tiles while that work is still finishing.  Activations, scales
- * and the output are touched only after it has ended, whatever the setting.
+ * and the output are touched only after it has ended, whatever the setting; so are both operands of gi8_matmul.  Weights written
+ * further back in the stream are safe.
  * No reference counterpart (its tuning is compile-time, CMakeLists.txt:49-51).
  */
 int gi8_reload_env(void);

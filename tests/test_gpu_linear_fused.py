@@ -89,8 +89,9 @@ def test_what_is_not_fused_and_what_is_refused(g):
 
 @pytest.mark.parametrize("mode", ["channel", "blockwise"])
 def test_fused_sees_what_was_just_written(g, mode):
-    """Weights, scales and activations written by the kernels directly in front, on a side stream and in a captured graph: the
-    product may request weights before its quantiser has ended, but never before their writer has."""
+    """Weights, scales, bias and activations replaced by device copies between the calls, on a side stream and in a captured graph.
+    (Copies order what follows them, so this is about nothing being kept from one call to the next; the order behind kernels that
+    let the next one start early is tested in test_gpu_launch_ordering.py.)"""
     gen = torch.Generator(device="cuda").manual_seed(11)
     a, b = (_layer(g, 2048, 4096, mode, None, True, gen) for _ in range(2))
     live = _layer(g, 2048, 4096, mode, None, True, gen)

@@ -241,7 +241,8 @@ def test_config3_decode_shapes(g, oracle, K, N):
 def test_smallm_static_weights_option(g, oracle, monkeypatch):
     """GEMM_INT8_STATIC_WEIGHTS=1 lets the small-M kernel request its first weight tiles before the preceding
     kernel has ended; activations and scales are still read after it.  Here the activations of every call are
-    written by a kernel directly before it (a device copy), back to back, and the bits must stay the oracle's."""
+    replaced by device copies in front of it, back to back, and the bits must stay the oracle's.  (Copies do not let the
+    next kernel start early; producers that do are in test_gpu_static_weights.py.)"""
     from gemm_int8_b200 import workloads
 
     monkeypatch.setenv("GEMM_INT8_STATIC_WEIGHTS", "1")
