@@ -88,6 +88,28 @@ GI8_DEVICE float amax_pairs(const uint64_t* v)
     return m;
 }
 
+// Largest magnitude of 16 loaded bytes (NaN ignored).  bf16: on the packed pairs as they came, one instruction for two elements.
+template <typename T>
+GI8_DEVICE float amax16(const uint4& u);
+
+template <>
+GI8_DEVICE float amax16<float>(const uint4& u)
+{
+    return max3_abs(__uint_as_float(u.x), __uint_as_float(u.y), max3_abs(__uint_as_float(u.z), __uint_as_float(u.w), 0.0f));
+}
+
+template <>
+GI8_DEVICE float amax16<__nv_bfloat16>(const uint4& u)
+{
+    // (the magnitudes' maximum with the product of the signs, which the last step drops; it starts at zero, so that two NaN do not meet)
+    uint32_t m = 0u;
+    asm("max.xorsign.abs.bf16x2 %0, %0, %1;\n\tmax.xorsign.abs.bf16x2 %0, %0, %2;\n\tmax.xorsign.abs.bf16x2 %0, %0, %3;\n\t"
+        "max.xorsign.abs.bf16x2 %0, %0, %4;"
+        : "+r"(m)
+        : "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w));
+    return max3_abs(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u), 0.0f);
+}
+
 // The exact rule for one element.
 GI8_DEVICE int quant_exact(float v, float s)
 {
@@ -102,18 +124,18 @@ GI8_DEVICE uint32_t pack_i8x4(int a, int b, int c, int d)
            ((static_cast<uint32_t>(c) & 0xff) << 16) | ((static_cast<uint32_t>(d) & 0xff) << 24);
 }
 
-// Four elements (two pairs) -> four packed int8.  Fast path, full-rate instructions only: t = v * r; adding 1.5 * 2^23
-// rounds t to the nearest-even integer n in the low mantissa bits, whose low byte is the int8 result; subtracting
-// the constant again gives n as a float for the half-integer test.  |n| <= 127 because |v| <= amax, so no clamp.
+// Four elements (two pairs) -> four packed int8.  Fast path, full-rate instructions only: v * r + 1.5 * 2^23 in one rounding
+// leaves the nearest integer n of v * r in the low mantissa bits, whose low byte is the int8 result; the constant minus that
+// is -n as a float, and v * r - n, again in one rounding, the distance for the half-integer test.  |n| <= 127 because
+// |v| <= amax, so no clamp.
 // The largest of the four distances decides (a NaN among them fails the test): packed arithmetic and three-operand
 // maxima make that about 3.5 instructions an element, where scalar ones with a comparison each took seven.
 GI8_DEVICE uint32_t quant_pack4(uint64_t v0, uint64_t v1, const QuantScale& qs)
 {
     const uint64_t magic = f32x2(12582912.0f, 12582912.0f);
     const uint64_t r2 = f32x2(qs.r, qs.r);
-    const uint64_t t0 = mul2(v0, r2), t1 = mul2(v1, r2);
-    const uint64_t u0 = add2(t0, magic), u1 = add2(t1, magic);
-    const uint64_t d0 = sub2(t0, sub2(u0, magic)), d1 = sub2(t1, sub2(u1, magic));
+    const uint64_t u0 = fma2(v0, r2, magic), u1 = fma2(v1, r2, magic);
+    const uint64_t d0 = fma2(v0, r2, sub2(magic, u0)), d1 = fma2(v1, r2, sub2(magic, u1));
     float a, b, c, d;
     f32x2_split(d0, a, b), f32x2_split(d1, c, d);
     if (max3_abs_nan(max3_abs_nan(a, b, c), d, 0.0f) <= 0.49993f) {
@@ -189,8 +211,8 @@ GI8_DEVICE void group_scales(float (&m)[U], float (&s)[U], float (&r)[U])
 // the type) and are unpacked at each use: a byte in flight costs a register byte.  fp32 input takes eight loads per lane,
 // bf16 input, which is closer to the bound of instruction issue, four.
 // Bound: HBM for fp32 (16384 x 8192: 128 -> 113 us, 6.0 TB/s, 0.91 of the copy bandwidth); for bf16 (103 -> 88 us, 4.6 TB/s, 0.71) no
-// single unit: 16 instructions an element issue on 68 % of the cycles, the integer pipe is at 54 %, and warps wait for their
-// loads.  Both with the packed arithmetic and one division per lane instead of one or two per block and lane (group_scales).
+// single unit; fewer instructions help: maxima on packed bf16 and quant_pack4 with two packed multiply-adds 90.4 -> 85.4 us (another
+// box), 4096 x 14336 40.7 -> 38.6.  Both with the packed arithmetic and one division per lane instead of one or two per block and lane (group_scales).
 // a [M,K] (K % EPL == 0, rows 16-byte aligned) -> q int8 [M,K], s fp32 [M, ceil(K/128)].
 constexpr int kQuantBlocksPerItem = 8;  // 128-wide blocks per warp and iteration, whatever the type (1 x 8 or 2 x 4)
 
@@ -228,9 +250,7 @@ quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, flo
         float m[kQuantUnroll], sc[kQuantUnroll], rc[kQuantUnroll];
 #pragma unroll
         for (int u = 0; u < kQuantUnroll; ++u) {
-            uint64_t v[EPL / 2];
-            unpack16<T>(raw[u], v);
-            m[u] = amax_pairs<EPL / 2>(v);
+            m[u] = amax16<T>(raw[u]);
         }
         group_scales<kQuantUnroll, LPB>(m, sc, rc);
 #pragma unroll
@@ -255,10 +275,13 @@ quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, flo
 // the maximum and the quantisation, so that the row is read once; what lies beyond them is read again (it hits L1 or L2).
 // The host takes the smallest of 2, 4 and 8 that holds the row (eight: 16384 bf16 or 8192 fp32 elements): registers that
 // a short row leaves unused would cost resident CTAs.
-// 16384 x 8192, row read twice -> held in registers: fp32 149 -> 102 us (6.6 TB/s), bf16 126 -> 88.5 (4.5 TB/s; issue 60 %, the rest waits
-// for loads and the barrier of a row).  Beyond the registers the second read stays: 8192 x 28672 bf16 211 -> 209 us (3.4 TB/s), fp32 322 -> 246.
+// 16384 x 8192, row read twice -> held in registers: fp32 149 -> 102 us (6.6 TB/s), bf16 126 -> 88.5 (on another box 74.6, since then 73).
+// Beyond the registers the second read stays: 8192 x 28672 fp32 322 -> 246 us.
+// Four CTAs per SM even with eight loads, which the maximum on packed bf16 makes room for (64 registers; unbounded it takes 72 and three
+// fit): bf16 4096 x 14336 36.7 -> 33.5 us (unbounded 35.8), 8192 x 28672 184 -> 131 us (unbounded 151), with the shorter
+// quant_pack4 included.
 template <typename T, int LOADS>
-__global__ void __launch_bounds__(kQuantThreads)
+__global__ void __launch_bounds__(kQuantThreads, LOADS == 8 ? 4 : LOADS == 4 ? 5 : 6)
 quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K,
                           bool release_late)
 {
@@ -276,16 +299,9 @@ quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float
             raw[u] = col0 + u * kStep < K ? __ldg(reinterpret_cast<const uint4*>(src + col0 + u * kStep)) : make_uint4(0u, 0u, 0u, 0u);
         float amax = 0.0f;
 #pragma unroll
-        for (int u = 0; u < LOADS; ++u) {
-            uint64_t v[EPL / 2];
-            unpack16<T>(raw[u], v);
-            amax = fmaxf(amax, amax_pairs<EPL / 2>(v));
-        }
-        for (int col = col0 + LOADS * kStep; col < K; col += kStep) {
-            uint64_t v[EPL / 2];
-            unpack16<T>(__ldg(reinterpret_cast<const uint4*>(src + col)), v);
-            amax = fmaxf(amax, amax_pairs<EPL / 2>(v));
-        }
+        for (int u = 0; u < LOADS; ++u) amax = fmaxf(amax, amax16<T>(raw[u]));
+        for (int col = col0 + LOADS * kStep; col < K; col += kStep)
+            amax = fmaxf(amax, amax16<T>(__ldg(reinterpret_cast<const uint4*>(src + col))));
         amax = warp_max(amax);
         // (two sets of slots in turn: one barrier per row is enough)
         if ((threadIdx.x & 31) == 0) warp_amax[parity][threadIdx.x >> 5] = amax;
