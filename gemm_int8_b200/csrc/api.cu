@@ -1333,13 +1333,13 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     const bool two = knobs().bw_issuers == 2 || (knobs().bw_issuers == 0 && bn < 256);
     const bool halves = knobs().bw_halves != 1;
     if (bias) {  // (the knobs below choose among forms without one)
-        if (pair) GI8_LAUNCH_BW(256, 4, 2, 2, true, true, 28);
+        if (pair) GI8_LAUNCH_BW(256, 6, 2, 2, true, true, 28);
         if (bn == 256) GI8_LAUNCH_BW(256, 4, 2, 2, false, true, 29);
         if (bn == 128) GI8_LAUNCH_BW(128, 6, 1, 2, false, true, 30);
         GI8_LAUNCH_BW(64, 8, 1, 2, false, true, 31);
     }
     if (pair) {
-        if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, true, false, 21);
+        if (halves) GI8_LAUNCH_BW(256, 6, 2, 2, true, false, 21);
         else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, true, false, 22);
         else GI8_LAUNCH_BW(256, 4, 1, 1, true, false, 23);
     } else if (bn == 256) {

@@ -8,13 +8,13 @@
 //   warpgroup 0 control (setmaxnreg.dec): warp 0 TMA producer (as in the dense kernel); warp 1 (and warp 3 when
 //               NISS == 2, taking alternate K blocks) MMA issuer -- per K block four tcgen05.mma kind::i8 with N = BN
 //               (or 2 x 4 with N = 128 when SPLIT == 2) that overwrite one of NBUF = 512 / BN tensor-memory partial
-//               buffers, then ONE commit per column half that both frees the pipeline stage and publishes the
-//               partial; warp 2 allocates tensor memory.
+//               buffers, then a commit that both frees the pipeline stage and publishes the partial (with column halves one
+//               commit for either); warp 2 allocates tensor memory.
 //   warps 4..11 promotion (setmaxnreg.inc): warp w owns TMEM lane quarter (w % 4) and BN/2 of the tile's columns
 //               (with column halves: 64 columns of each half), i.e. 32 rows x BN/2 columns, whose fp32
 //               accumulators it keeps in registers (as f32x2 pairs).  Per K block and half: tcgen05.ld the int32
-//               partial in 32-column chunks, hand the half back after the last load, and accumulate it with the
-//               block's scale.  A warp's segment never straddles a 128-wide weight-scale block.  At the end of the
+//               partial in chunks of 32 columns (column halves: 16, the next chunk's load running under the arithmetic of this
+//               one), hand the half back after the last load, and accumulate it with the block's scale.  A warp's segment never straddles a 128-wide weight-scale block.  At the end of the
 //               tile the same warps cast to bf16 and store through swizzled shared memory and TMA.
 //
 // Two ways to accumulate, both one rounding per K block and element, the same bits:
@@ -42,19 +42,34 @@
 // (barrier test, hand-back, scale product, counters), and those instructions share the half-rate integer pipe
 // with the conversions, which was the busiest unit (two cycles per cvt.rn.f32.s32: 512 of the K block's cycles).
 //
+// What bounds the column halves (two-CTA form, cycles per K block at 1.6 GHz, which is what the chip holds under this load; copies of
+// the kernel with parts left out): all 826; without the bias MMA 810; without arithmetic 710; without both 626; without MMAs
+// 800; one multiply-add instead of two 842.  Neither pipe alone: a K block's two hand-overs, during which the eight warps
+// do the same thing at the same time, lie between stretches of arithmetic (the loop without hand-overs takes 554).  Partial
+// buffers with barriers of their own (their ring positions are compile-time constants whatever the stage count), six stages
+// instead of four in the two-CTA form (four starved it: 1.5 us a round trip), loads one chunk ahead and a warp-uniform issue loop, all
+// together: 2048 x 11008 x 4096 95.6 -> 93.3 us, 8192^3 511 -> 492 (two-CTA 492 -> 478), 512 x 9472 x 16384 74.6 -> 73.9 (two-CTA 73.9 -> 72.1).
+// Tried on top of that, us at 2048 x 11008 x 4096 (two-CTA): sixteen promotion warps, four a scheduler, 121; one issuer for both
+// halves 103; one lane instead of the warp at the barriers 132; N = 256 MMAs with one hand-over a K block 102; loads of 32 columns
+// one chunk ahead 119 (spills).
+//
 // Barrier protocol (every wait is a parity wait, so it must hold that a barrier cannot complete a second phase
 // before the waiter has consumed the first; the comment at each barrier says what gates its next phase):
 //   bar_full[s]        completed by the TMA bytes of K block `it` (s = it % STAGES).  Waiter: the issuer of K block
 //                      `it` (with column halves: both issuers, each of which visits every K block).  Next phase
-//                      needs the producer to refill stage s, which needs bar_done[h][s] of K block `it` for every
-//                      half h, i.e. every waiting issuer's own commit: gated by each waiter.
-//   bar_done[h][s]     completed by the issuer's commit for column half h of K block `it`.  Waiters: the producer
-//                      (before refilling s; the next completion needs its own refill: gated) and all promotion
-//                      warps (the next completion is K block it + STAGES, whose MMAs need half h of partial buffer
+//                      needs the producer to refill stage s, which needs bar_done[s] of K block `it`, i.e. every waiting
+//                      issuer's own commit: gated by each waiter.
+//   bar_done[s]        completed by the issuer's commit for K block `it` (with column halves by both issuers').  Waiters: the
+//                      producer (before refilling s; the next completion needs its own refill: gated) and, without column
+//                      halves, all promotion warps (the next completion is K block it + STAGES, whose MMAs need partial buffer
 //                      (it + STAGES) % NBUF handed back by every warp for K block it + STAGES - NBUF >= it: gated).
+//   bar_part_full[h][b]   column halves: completed by the commit of half h of a K block in buffer b.  Waiters: the promotion warps;
+//                      the next completion needs MMAs into that half, which need its hand-back by each of them: gated.
 //   bar_part_empty[h][b]  completed by the arrivals of all eight promotion warps after their last load of half h of
 //                      a K block in buffer b.  Waiter: the issuer of half h of the next K block that uses b; the
 //                      completion after that needs this issuer's MMAs: gated.
+//   With column halves the buffer is the parity of the K block inside its tile: a tile of an odd count of K blocks ends and the next
+//   one begins with buffer 0, and each buffer's phase is counted by itself (issuers and promotion warps do the same).
 //   Without column halves and with two issuers, issuer j takes K blocks it % 2 == j, hence stages s % 2 == j and
 //   buffers b % 2 == j (STAGES and NBUF are even): every barrier still has exactly one issuing waiter, which sees
 //   all its phases.
@@ -237,6 +252,9 @@ GI8_DEVICE int rotate_tile(int tile, int rot, int n)
 
 // Makes a 32-bit value opaque to the optimiser at this point, so that later uses read the register instead of
 // recomputing the value.
+GI8_DEVICE void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_32x32b_x16(taddr, r); }
+GI8_DEVICE void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32b_x32(taddr, r); }
+
 #define GI8_PIN(v) asm volatile("" : "+r"(v))
 
 // SPLIT = 2 (BN = 256 only): the MMAs of a K block are issued as two column halves (N = 128 each), each half by its
@@ -250,8 +268,7 @@ GI8_DEVICE int rotate_tile(int tile, int rot, int n)
 // PAIR: two CTAs on neighbouring SMs (a 2 x 1 x 1 cluster) share one 256 x BN tile, as in the dense kernel: the
 // leader's issuers run tcgen05.mma.cta_group::2 (M = 256), each CTA loads its own 128 rows of x and HALF of the BN
 // rows of y, keeps the partials of its 128 rows in its own tensor memory and promotes them with its own eight warps.
-// Per SM that is a third fewer operand bytes per K block (32 KB instead of 48 KB; four stages are used, six would fit
-// and measured the same) and half the MMA instructions.  It matters because the 1-CTA kernel is bound by bytes in flight: with four
+// Per SM that is a third fewer operand bytes per K block (32 KB instead of 48 KB; six stages) and half the MMA instructions.  It matters because the 1-CTA kernel is bound by bytes in flight: with four
 // 48 KB stages, one of them being read by the tensor core, 144 KB are in flight against an L2 latency of about 2000
 // cycles under load -- 72 bytes per cycle, i.e. 670 cycles per 48 KB K block where the tensor core needs 512.  TMA
 // loads are unicast into the issuing CTA's shared memory and signal the leader's barrier; the commits are two
@@ -274,16 +291,16 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     constexpr int NSUB = BN / SPLIT;     // N of one MMA = columns of one half
     constexpr int CW = BN / 2;           // columns per promotion warp (128, 64 or 32) ...
     constexpr int SEGW = CW / SPLIT;     // ... as SPLIT segments of SEGW columns, one in each half
-    constexpr int CHW = 32;              // columns per tensor-memory load (64 was measured: no gain)
+    constexpr int CHW = SPLIT == 2 ? 16 : 32;  // columns per tensor-memory load
     constexpr int NC = SEGW / CHW;       // loads per segment
     constexpr int STORE_W = blockwise_store_cols(BN);
     static_assert(SEGW % STORE_W == 0 && SEGW % 32 == 0, "segments are whole store boxes and whole loads");
     // SPLIT == 1: each issuer must own the stages and the partial buffers of its K blocks (see the protocol above):
     // with an odd count an issuer would meet a barrier only every second phase, which a parity wait cannot tell apart.
     static_assert(SPLIT == 2 || (STAGES % NISS == 0 && NBUF % NISS == 0), "issuers must own their stages and partial buffers");
-    // A promotion warp's parity wait on bar_done is safe only if the commit STAGES K blocks later needs a partial
-    // buffer that the same warp hands back after the awaited K block (see the protocol above).
-    static_assert(STAGES >= NBUF, "the stage ring must be at least as deep as the partial-buffer ring");
+    // Without column halves a promotion warp's parity wait on bar_done is safe only if the commit STAGES K blocks later needs a
+    // partial buffer that the same warp hands back after the awaited K block (see the protocol above).
+    static_assert(SPLIT == 2 || STAGES >= NBUF, "the stage ring must be at least as deep as the partial-buffer ring");
     static_assert(!PAIR || BN == 256, "two-CTA tiles are 256 wide");
     constexpr bool BIASED = SPLIT == 2;
     constexpr int kTileM = PAIR ? 2 * kBM : kBM;  // rows of the (pair's) tile
@@ -302,7 +319,8 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
     __shared__ __align__(8) uint64_t bar_full[STAGES];
-    __shared__ __align__(8) uint64_t bar_done[SPLIT][STAGES];
+    __shared__ __align__(8) uint64_t bar_done[STAGES];
+    __shared__ __align__(8) uint64_t bar_part_full[SPLIT][NBUF];  // column halves only
     __shared__ __align__(8) uint64_t bar_part_empty[SPLIT][NBUF];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile uint32_t abort_flag;
@@ -321,10 +339,13 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&bar_full[s], 1);
-            for (int h = 0; h < SPLIT; ++h) mbar_init(&bar_done[h][s], 1);
+            mbar_init(&bar_done[s], SPLIT);
         }
         for (int b = 0; b < NBUF; ++b) {
-            for (int h = 0; h < SPLIT; ++h) mbar_init(&bar_part_empty[h][b], PAIR ? 2 * kPromoWarps : kPromoWarps);
+            for (int h = 0; h < SPLIT; ++h) {
+                mbar_init(&bar_part_full[h][b], 1);
+                mbar_init(&bar_part_empty[h][b], PAIR ? 2 * kPromoWarps : kPromoWarps);
+            }
         }
         fence_barrier_init();
         prefetch_tensormap(&map_x);
@@ -399,9 +420,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 int mb, nb;
                 tile_coords(rotate_tile(tile, p.tile_rot, num_tiles), p.tiles_m, p.tiles_n, mb, nb, p.group_m);
                 for (int kb = tile == first_tile ? kb_early : 0; kb < num_kb; ++kb) {
-                    bool freed = wait_or_abort(&bar_done[0][s], ph ^ 1, &abort_flag);
-                    if (SPLIT == 2 && freed) freed = wait_or_abort(&bar_done[SPLIT - 1][s], ph ^ 1, &abort_flag);
-                    if (!freed) {
+                    if (!wait_or_abort(&bar_done[s], ph ^ 1, &abort_flag)) {
                         if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_PRODUCER);
                         ok = false;
                         break;
@@ -440,8 +459,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         } else if ((warp == 1 || (NISS == 2 && warp == 3)) && rank == 0) {
             // -------------------------------------------------------------- MMA issuer(s) (PAIR: the leader's)
             const uint32_t me = warp == 1 ? 0u : 1u;
-            // SPLIT == 2: issuer `me` issues column half `me` of EVERY K block.  SPLIT == 1: issuer `me` issues the
-            // K blocks with it % NISS == me.
+            // Column halves: issuer `me` issues half `me` of every K block.  Otherwise issuer `me` takes the K blocks with it % NISS == me.
             constexpr uint32_t kStep = SPLIT == 2 ? 1u : static_cast<uint32_t>(NISS);
             const uint32_t first = SPLIT == 2 ? 0u : me;
             const uint32_t h = SPLIT == 2 ? me : 0u;
@@ -450,48 +468,62 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             const uint32_t total = static_cast<uint32_t>(my_tiles) * static_cast<uint32_t>(num_kb);
             // stage / partial buffer of K block `it` and their phase parities, stepped without divisions
             uint32_t s = first, ph = 0, buf = first, bph = 0;
-            uint64_t* const done_h = &bar_done[h][0];
-            uint64_t* const empty_h = &bar_part_empty[h][0];
+            // column halves: the buffer is the parity of the K block inside its tile, bit b of bph the phase of buffer b
+            [[maybe_unused]] int kb_in_tile = 0;
             [[maybe_unused]] const uint64_t d_ones = make_smem_desc_ones(smem_u32(ones_tile));
+            // Half h: rows h * NSUB.. of the weight tile (PAIR: rows h * NSUB / 2.. of each CTA's half of it) into columns h * NSUB..
+            // of the partial buffer.
+            const uint32_t da_0 = smem_desc_lo(smem_u32(smem)), db_0 = smem_desc_lo(smem_u32(smem) + kBytesA + h * (PAIR ? NSUB / 2 : NSUB) * kBK);
+            const uint32_t full_0 = smem_u32(&bar_full[0]), done_0 = smem_u32(&bar_done[0]);
+            const uint32_t empty_0 = smem_u32(&bar_part_empty[h][0]), part_0 = smem_u32(&bar_part_full[h][0]);
             for (uint32_t it = first; it < total; it += kStep) {
                 // The operands first (they land long before the partial buffer is free), so that nothing but the
                 // MMAs stands between the buffer hand-back and the tensor core.
-                bool issued = wait_or_abort(&bar_full[s], ph, &abort_flag);
-                // Half h: rows h * NSUB.. of the weight tile (PAIR: rows h * NSUB / 2.. of each CTA's half of it) into
-                // columns h * NSUB.. of the partial buffer.
-                const uint32_t tmem_d = tmem_base + buf * BN + h * NSUB;
-                const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
-                const uint64_t da = make_smem_desc_k128(a_addr);
-                const uint64_t db = make_smem_desc_k128(a_addr + kBytesA + h * (PAIR ? NSUB / 2 : NSUB) * kBK);
-                issued = issued && wait_or_abort(&empty_h[buf], bph ^ 1, &abort_flag);
+                bool issued = wait_or_abort_addr(full_0 + 8 * s, ph, &abort_flag);
+                issued = issued && wait_or_abort_addr(empty_0 + 8 * buf, (SPLIT == 2 ? (bph >> buf) & 1u : bph) ^ 1, &abort_flag);
+                // (the vote keeps the loop, and with it the descriptors below, warp-uniform; the narrow tiles do not gain by it)
+                if constexpr (SPLIT == 2) issued = __all_sync(0xffffffffu, issued);
                 if (!issued) {
                     if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
                     break;
                 }
+                const uint32_t tmem_d = tmem_base + buf * BN + h * NSUB;
+                const uint32_t da = da_0 + s * (kStageBytes / 16), db = db_0 + s * (kStageBytes / 16);
                 tcgen05_fence_after_sync();
                 if (elect_one()) {
                     // The first K step overwrites the buffer.
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k) {
-                        if constexpr (PAIR) umma_i8_pair(tmem_d, da + 2 * k, db + 2 * k, kIdesc, k != 0 ? 1u : 0u);
-                        else umma_i8(tmem_d, da + 2 * k, db + 2 * k, kIdesc, k != 0 ? 1u : 0u);
+                        if constexpr (PAIR) umma_i8_pair(tmem_d, smem_desc_k128_of(da + 2 * k), smem_desc_k128_of(db + 2 * k), kIdesc, k != 0 ? 1u : 0u);
+                        else umma_i8(tmem_d, smem_desc_k128_of(da + 2 * k), smem_desc_k128_of(db + 2 * k), kIdesc, k != 0 ? 1u : 0u);
                     }
                     if constexpr (BIASED) {
                         if constexpr (PAIR) umma_i8_pair(tmem_d, d_ones, d_ones, make_idesc_u8(kTileM, NSUB), 1u);
                         else umma_i8(tmem_d, d_ones, d_ones, make_idesc_u8(kTileM, NSUB), 1u);
                     }
                     if constexpr (PAIR) {
-                        umma_commit_pair(map_to_cta(smem_u32(&done_h[s]), 0));
-                        umma_commit_pair(map_to_cta(smem_u32(&done_h[s]), 1));
+                        if constexpr (SPLIT == 2) {
+                            umma_commit_pair(map_to_cta(part_0 + 8 * buf, 0));
+                            umma_commit_pair(map_to_cta(part_0 + 8 * buf, 1));
+                        }
+                        umma_commit_pair(map_to_cta(done_0 + 8 * s, 0));
+                        umma_commit_pair(map_to_cta(done_0 + 8 * s, 1));
                     } else {
-                        umma_commit(&done_h[s]);
+                        if constexpr (SPLIT == 2) umma_commit(&bar_part_full[h][buf]);
+                        umma_commit(&bar_done[s]);
                     }
                 }
                 __syncwarp();
                 s += kStep;
                 if (s >= STAGES) s -= STAGES, ph ^= 1;
-                buf += kStep;
-                if (buf >= NBUF) buf -= NBUF, bph ^= 1;
+                if constexpr (SPLIT == 2) {
+                    bph ^= 1u << buf;
+                    buf ^= 1u;
+                    if (++kb_in_tile == num_kb) kb_in_tile = 0, buf = 0;
+                } else {
+                    buf += kStep;
+                    if (buf >= NBUF) buf -= NBUF, bph ^= 1;
+                }
             }
         }
     } else {
@@ -505,48 +537,35 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         // issue.
         uint32_t tm_warp = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(cg * SEGW);
         GI8_PIN(tm_warp);
-        uint32_t bar_done_0 = smem_u32(&bar_done[0][0]);
+        uint32_t bar_part_0 = SPLIT == 2 ? smem_u32(&bar_part_full[0][0]) : smem_u32(&bar_done[0]);
         // (PAIR: the hand-back barriers are the leader's, addressed through the cluster window)
         uint32_t bar_empty_0 = PAIR ? map_to_cta(smem_u32(&bar_part_empty[0][0]), 0) : smem_u32(&bar_part_empty[0][0]);
-        GI8_PIN(bar_done_0);
+        GI8_PIN(bar_part_0);
         GI8_PIN(bar_empty_0);
-        // Stage, partial buffer and barrier phase of the running K block (as in the MMA issuer), stepped without
-        // divisions: byte offset of the stage's barrier, its parity, byte offset of the buffer's barrier, the
-        // buffer's first column.
-        uint32_t st_off = 0, st_par = 0, buf_off = 0, buf_col = 0;
+        // Narrow tiles: stage, partial buffer and barrier phase of the running K block (as in the MMA issuer), stepped without
+        // divisions: byte offset of the stage's barrier, its parity, byte offset of the buffer's barrier, the buffer's first
+        // column.
+        [[maybe_unused]] uint32_t st_off = 0, st_par = 0, buf_off = 0, buf_col = 0;
+        // Column halves: bit b is the phase of partial buffer b.
+        [[maybe_unused]] uint32_t buf_par = 0;
         bool ok = true;
 
-        // Waits for half h of the partial of the running K block; false on every lane if any lane gave up.  The
-        // barrier was already tested once, without blocking, before the arithmetic of the previous chunk
-        // (`polled`, see poll_next): in the steady state the MMAs are ahead, the test has succeeded and its latency
-        // lay under that arithmetic.  Otherwise the bounded wait runs; the branch is taken on a vote, which makes it
-        // warp-uniform.
+        // Waits for the partial whose barrier is `bar`; false on every lane if any lane gave up.  The barrier was already tested
+        // once, without blocking, some arithmetic earlier (`polled`): in the steady state the MMAs are ahead, the test has
+        // succeeded and its latency lay under that arithmetic.  Otherwise the bounded wait runs; the branch is taken on a vote,
+        // which makes it warp-uniform.
         bool polled = false;
         [[maybe_unused]] const uint64_t unbias_c2 = f32x2(0x1p127f, 0x1p127f);
         [[maybe_unused]] const uint64_t unbias_b2 = f32x2(-static_cast<float>(kPartialBias) * 0x1p-22f, -static_cast<float>(kPartialBias) * 0x1p-22f);
-        // (so, sp): byte offset of the stage's barrier in its ring and the parity awaited there.
-        auto wait_partial = [&](int h, uint32_t so, uint32_t sp) {
+        auto wait_partial = [&](uint32_t bar, uint32_t parity) {
             if (!__all_sync(0xffffffffu, polled)) {
-                const uint32_t bar = bar_done_0 + h * (STAGES * 8) + so;
-                bool got = wait_or_abort_addr(bar, sp, &abort_flag);
+                bool got = wait_or_abort_addr(bar, parity, &abort_flag);
                 if (!got && lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
                 got = __all_sync(0xffffffffu, got);
                 if (!got) return false;
             }
             tcgen05_fence_after_sync();
             return true;
-        };
-        // Tests the barrier of the partial that follows half h of the K block at (so, sp): the other half of the same
-        // K block, or half 0 of the next K block (the stage ring runs on across tiles; after the last K block of the
-        // last tile the test simply fails and is never looked at).
-        auto poll_next = [&](int h, uint32_t so, uint32_t sp) {
-            int hn = h + 1;
-            if (hn == SPLIT) {
-                hn = 0;
-                so += 8;
-                if (so == STAGES * 8) so = 0, sp ^= 1;
-            }
-            polled = mbar_test_wait_addr(bar_done_0 + hn * (STAGES * 8) + so, sp);
         };
         // This warp's columns of half h of the K block in the partial buffer whose barrier lies at byte offset bo are
         // in registers: one of the arrivals that hand the half back to its MMA issuer.
@@ -559,19 +578,6 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 mbar_arrive_elected_addr(bar_empty_0 + h * (NBUF * 8) + bo);
             }
         };
-        auto next_k_block = [&]() {
-            st_off += 8;
-            if (st_off == STAGES * 8) st_off = 0, st_par ^= 1;
-            buf_off += 8, buf_col += BN;
-            if (buf_off == NBUF * 8) buf_off = 0, buf_col = 0;
-        };
-        // With four stages, two partial buffers and K blocks handled four at a time (the vector-scale path, whose K
-        // block count is a multiple of four), every tile starts at stage 0 and buffer 0: the ring positions of the four
-        // K blocks of a group are compile-time constants and only the parity, flipped once per group, lives in a
-        // register.  That removes the counter arithmetic (about ten instructions per warp and K block on the integer
-        // pipe, which the conversions keep busiest).
-        constexpr bool kStaticRing = STAGES == 4 && NBUF == 2;
-
         for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
             int mb, nb;
             tile_coords(rotate_tile(tile, p.tile_rot, num_tiles), p.tiles_m, p.tiles_n, mb, nb, p.group_m);
@@ -598,53 +604,86 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j) acc[j] = 0ull;
 
-            // One K block with the scale products t[h] of its column halves: per half wait for the partial, then per
-            // 32-column chunk load, (after the half's last load) hand the half back, convert and accumulate.
-            // (Issuing the next chunk's load before this chunk's arithmetic was tried with 32- and with 16-column
-            // chunks: no gain, the 32-column form spills.  64-column loads: no gain.  Sending a third of the pairs
-            // through an integer multiply-add on the other pipe instead of cvt: no gain.  Leaving the grouping of
-            // conversions and multiply-adds to the compiler (non-volatile statements): the same cycle count.  Writing
-            // the conversions one to sixteen pairs ahead of their multiply-adds: the same times to within the run-to-run
-            // spread -- the assembler schedules the block itself.  Sending every third to eighth pair through
-            // multiply-add-pipe instructions only (integer multiply-add with the bias 0x4B400000, packed subtract,
-            // packed fma), measured again after the barrier latencies had been hidden: 15-45 % slower on the one-CTA
-            // form, 2-4 % faster on the two-CTA form with column halves.)
-            // J >= 0: K block J of a group of four under kStaticRing; J < 0: the running counters.
-            auto k_block = [&](const float (&t)[SPLIT], auto jc) -> bool {
-                constexpr int J = decltype(jc)::value;
-                const uint32_t so = J >= 0 ? static_cast<uint32_t>(J * 8) : st_off;
-                const uint32_t sp = st_par;
-                const uint32_t bo = J >= 0 ? static_cast<uint32_t>((J & 1) * 8) : buf_off;
-                const uint32_t bc = J >= 0 ? static_cast<uint32_t>((J & 1) * BN) : buf_col;
+            // Narrow tiles, one K block with scale product t: wait for the partial, then per 32-column chunk load, (after the last load)
+            // hand the buffer back, convert and accumulate.
+            [[maybe_unused]] auto k_block_narrow = [&](float t) -> bool {
+                if (!wait_partial(bar_part_0 + st_off, st_par)) return false;
+                const uint64_t t2 = f32x2(t, t);
 #pragma unroll
-                for (int h = 0; h < SPLIT; ++h) {
-                    if (!wait_partial(h, so, sp)) return false;
-                    const float ts = BIASED ? t[h] * 0x1p22f : t[h];
-                    const uint64_t t2 = f32x2(ts, ts);
-                    const uint32_t taddr = tm_warp + bc + h * NSUB;
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        uint32_t v[CHW];
-                        tmem_ld_32x32b_x32(taddr + c * CHW, v);
-                        tmem_ld_wait();
-                        if (c + 1 == NC) {
-                            release_partial(h, bo);
-                            poll_next(h, so, sp);
-                        }
-#pragma unroll
-                        for (int q = 0; q < CHW / 2; ++q) {
-                            uint64_t& a = acc[h * (SEGW / 2) + c * (CHW / 2) + q];
-                            if constexpr (BIASED) promote_pair_biased(a, v[2 * q], v[2 * q + 1], unbias_c2, unbias_b2, t2);
-                            else promote_pair(a, v[2 * q], v[2 * q + 1], t2);
-                        }
+                for (int c = 0; c < NC; ++c) {
+                    uint32_t v[CHW];
+                    tmem_ld(tm_warp + buf_col + c * CHW, v);
+                    tmem_ld_wait();
+                    if (c + 1 == NC) {
+                        release_partial(0, buf_off);
+                        // (the stage ring runs on across tiles; behind the last K block the test fails and is never looked at)
+                        uint32_t so = st_off + 8, sp = st_par;
+                        if (so == STAGES * 8) so = 0, sp ^= 1;
+                        polled = mbar_test_wait_addr(bar_part_0 + so, sp);
                     }
+#pragma unroll
+                    for (int q = 0; q < CHW / 2; ++q) promote_pair(acc[c * (CHW / 2) + q], v[2 * q], v[2 * q + 1], t2);
                 }
-                if constexpr (J < 0) next_k_block();
-                else if constexpr (J == 3) st_par ^= 1;
+                st_off += 8;
+                if (st_off == STAGES * 8) st_off = 0, st_par ^= 1;
+                buf_off += 8, buf_col += BN;
+                if (buf_off == NBUF * 8) buf_off = 0, buf_col = 0;
                 return true;
             };
-            using Dyn = std::integral_constant<int, -1>;
+            // Column halves, one K block with the scale products t[h], whose partials lie in buffer B; its first chunk is on the
+            // way into v[0].  Per chunk: wait for its load, (after a half's last load) hand the half back, start the load of
+            // the next chunk, which may lie in the other half or in the next K block, and accumulate this one under that load.
+            // A half's barrier is tested one chunk's arithmetic before the load that needs it.
+            [[maybe_unused]] uint32_t v[2][CHW];
+            [[maybe_unused]] auto wait_half = [&](int h, int b) { return wait_partial(bar_part_0 + (h * NBUF + b) * 8, (buf_par >> b) & 1u); };
+            [[maybe_unused]] auto load_chunk = [&](int h, int b, int c, uint32_t (&r)[CHW]) { tmem_ld(tm_warp + b * BN + h * NSUB + c * CHW, r); };
+            auto k_block = [&](const float (&t)[SPLIT], auto buffer, bool has_next) -> bool {
+                [[maybe_unused]] constexpr int B = decltype(buffer)::value;
+                if constexpr (SPLIT == 1) {
+                    return k_block_narrow(t[0]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float ts = t[h] * 0x1p22f;
+                        const uint64_t t2 = f32x2(ts, ts);
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            const int cur = (h * NC + c) & 1;
+                            tmem_ld_wait();
+                            if (c + 1 < NC) {
+                                load_chunk(h, B, c + 1, v[cur ^ 1]);
+                            } else {
+                                release_partial(h, B * 8);
+                                if (h == 0) {
+                                    if (!wait_half(1, B)) return false;
+                                    buf_par ^= 1u << B;
+                                    load_chunk(1, B, 0, v[cur ^ 1]);
+                                } else if (has_next) {
+                                    if (!wait_half(0, B ^ 1)) return false;
+                                    load_chunk(0, B ^ 1, 0, v[cur ^ 1]);
+                                }
+                            }
+                            if (c + 2 == NC) {
+                                const int hn = h ^ 1, bn = h == 0 ? B : B ^ 1;
+                                polled = mbar_test_wait_addr(bar_part_0 + (hn * NBUF + bn) * 8, (buf_par >> bn) & 1u);
+                            }
+#pragma unroll
+                            for (int q = 0; q < CHW / 2; ++q)
+                                promote_pair_biased(acc[h * (SEGW / 2) + c * (CHW / 2) + q], v[cur][2 * q], v[cur][2 * q + 1], unbias_c2, unbias_b2, t2);
+                        }
+                    }
+                    return true;
+                }
+            };
+            using Buffer0 = std::integral_constant<int, 0>;
+            using Buffer1 = std::integral_constant<int, 1>;
 
+            if constexpr (SPLIT == 2) {
+                static_assert(NC >= 2 && NC % 2 == 0, "a half's barrier is tested one chunk ahead; a K block is an even number of chunks");
+                polled = false;
+                if (!wait_half(0, 0)) break;
+                load_chunk(0, 0, 0, v[0]);
+            }
             if (p.scale_vec) {
                 // Scales of four K blocks per load (16 bytes per row): a quarter of the load instructions and of
                 // the sectors touched (a token's scales of eight consecutive K blocks share one 32-byte sector, and
@@ -670,16 +709,16 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     float t[SPLIT];
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.x, sw_c[h].x);
-                    ok = k_block(t, std::integral_constant<int, kStaticRing ? 0 : -1>{});
+                    ok = k_block(t, Buffer0{}, true);
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.y, sw_c[h].y);
-                    ok = ok && k_block(t, std::integral_constant<int, kStaticRing ? 1 : -1>{});
+                    ok = ok && k_block(t, Buffer1{}, true);
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.z, sw_c[h].z);
-                    ok = ok && k_block(t, std::integral_constant<int, kStaticRing ? 2 : -1>{});
+                    ok = ok && k_block(t, Buffer0{}, true);
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.w, sw_c[h].w);
-                    ok = ok && k_block(t, std::integral_constant<int, kStaticRing ? 3 : -1>{});
+                    ok = ok && k_block(t, Buffer1{}, kb + 4 < num_kb);
                     sa_c = sa_n;
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) sw_c[h] = sw_n[h];
@@ -713,7 +752,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                         for (int h = 0; h < SPLIT; ++h) sw_q[j][h] = ldg_in_place(p.sw + (sw_off[h] + kb + 2));
                     }
-                    return k_block(t, Dyn{});
+                    return j == 0 ? k_block(t, Buffer0{}, kb + 1 < num_kb) : k_block(t, Buffer1{}, kb + 1 < num_kb);
                 };
                 for (int kb = 0; kb < num_kb && ok; kb += 2) {
                     ok = k_block_scalar(kb, 0);

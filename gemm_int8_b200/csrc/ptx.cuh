@@ -249,6 +249,16 @@ GI8_DEVICE uint64_t make_smem_desc_k128(uint32_t smem_addr)
     return d;
 }
 
+// The same in two halves: the low word of the descriptor of a tile, to which a byte offset (>> 4) is added, and the descriptor of a
+// low word.
+GI8_DEVICE uint32_t smem_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3ffff) >> 4) | (1u << 16); }
+GI8_DEVICE uint64_t smem_desc_k128_of(uint32_t lo)
+{
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((1024u >> 4) | (1u << 14) | (2u << 29)));
+    return d;
+}
+
 // Instruction descriptor for kind::i8: D = int32 (format 2 at bits [4,6)), A and B signed 8-bit
 // (1 at bits [7,10) and [10,13)), both K-major (bits 15, 16 clear), N >> 3 at [17,23),
 // M >> 4 at [24,29).  Bit 3 selects a saturating accumulator.
