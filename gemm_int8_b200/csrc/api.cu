@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "k_blockwise.cuh"
+#include "k_blockwise_smallm.cuh"
 #include "k_dense.cuh"
 #include "k_quant.cuh"
 #include "k_smallm.cuh"
@@ -735,6 +736,24 @@ SmallMPlan plan_smallm_plain(int64_t M, int64_t N, int64_t K, int sms)
     return pl;
 }
 
+// Block-scaled products of up to sixteen tokens run on blockwise_smallm_kernel whatever N and K (its header has both sides of the line).
+// Four stages let two CTAs share an SM, which grids of more than one CTA per SM need (16 x 14336 x 4096 14.6 us, with six stages 19.4);
+// where every CTA has an SM to itself six put more bytes in flight (16 x 8192 x 8192 and 16 x 4096 x 14336 with four: 17.7 and 23.8 against 17.8
+// and 26.0 us in one build, 17.5 and 25.5 with six in another: level).
+bool use_blockwise_smallm(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= kBwSmallTokens && N > 0 && K > 0; }
+
+template <int STAGES>
+int launch_blockwise_smallm(DeviceState* st, int slot, const int8_t* x, const int8_t* w, const BlockwiseSmallMParams& p, cudaStream_t stream)
+{
+    using S = BlockwiseSmallM<STAGES>;
+    auto kernel = blockwise_smallm_kernel<STAGES>;
+    if (int rc = ensure_smem(st, slot, kernel, S::SMEM)) return rc;
+    CUtensorMap mw, mx;
+    if (int rc = make_operand_map(&mw, w, p.N, p.K, kBwSmallTileN)) return rc;
+    if (int rc = make_operand_map(&mx, x, p.M, p.K, kBwSmallTokens)) return rc;
+    return launch(kernel, dim3((p.N + kBwSmallTileN - 1) / kBwSmallTileN), S::THREADS, S::SMEM, stream, dim3(1), knobs().pdl, mw, mx, p);
+}
+
 template <int MT, int STAGES>
 int launch_smallm(DeviceState* st, int slot, const int8_t* x, const int8_t* w, SmallMParams p, const SmallMPlan& pl,
                   cudaStream_t stream)
@@ -911,6 +930,7 @@ const char* gi8_pick_variant(int kind, int64_t M, int64_t N, int64_t K)
     if (forced != VAR_AUTO) return kVariantNames[forced];
     if ((kind == 1 && plan_smallm(M, N, K, sms, false).use) || (kind == 0 && plan_smallm_plain(M, N, K, sms).use)) return "smallm_cluster";
     if (kind == 2) {
+        if (use_blockwise_smallm(M, N, K)) return "blockwise_bn64";  // (the small-M form of it: 64 columns, the tokens on the narrow side)
         const BlockwiseChoice c = choose_blockwise(M, N, K, sms);
         const int bn = c.bn;
         const bool pair = c.pair;
@@ -1360,6 +1380,19 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
 static int blockwise_dispatch(const int8_t* x, const int8_t* y, const float* sa, int64_t ld_sa, const float* sw, int64_t ld_sw, void* out,
                               int64_t M, int64_t N, int64_t K, void* stream, const uint16_t* bias, bool after_quant)
 {
+    if (g_forced_variant == VAR_AUTO && use_blockwise_smallm(M, N, K)) {
+        if (int rc = check_common(x, y, out, M, N, K, 2)) return rc;
+        DeviceState* st;
+        if (int rc = get_device_state(&st)) return rc;
+        if (int rc = check_block_scales(sa, ld_sa, sw, ld_sw, M, N, K)) return rc;
+        BlockwiseSmallMParams q{};
+        q.out = static_cast<uint16_t*>(out), q.sa = sa, q.sw = sw, q.bias = bias, q.status = st->status;
+        q.ldo = N, q.ld_sa = ld_sa, q.ld_sw = ld_sw, q.M = (int)M, q.N = (int)N, q.K = (int)K;
+        q.after_quant = after_quant && knobs().pdl;
+        cudaStream_t s = static_cast<cudaStream_t>(stream);
+        if (N <= static_cast<int64_t>(kBwSmallTileN) * st->sm_count) return launch_blockwise_smallm<6>(st, 33, x, y, q, s);
+        return launch_blockwise_smallm<4>(st, 32, x, y, q, s);
+    }
     if (g_forced_variant == VAR_AUTO && M > 0 && N > 0 && K > 0 && out && reinterpret_cast<uintptr_t>(out) % 16 == 0 && N % 8 == 0) {
         DeviceState* st;
         if (int rc = get_device_state(&st)) return rc;

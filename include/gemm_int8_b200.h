@@ -222,7 +222,8 @@ int gi8_linear(const void* x, int x_dtype, const int8_t* w, const float* w_scale
 int gi8_force_variant(const char* name);
 
 /* Name of the variant the dispatch would pick for (kind, M, N, K); kind: 0 plain, 1 scaled, 2 blockwise (whose names
- * read "blockwise_bn256", "blockwise_bn128", "blockwise_bn64", "blockwise_pair", and "blockwise_bn256+columns_bnW" where
+ * read "blockwise_bn256", "blockwise_bn128", "blockwise_bn64" (up to 16 tokens: its small-M form, which only the automatic dispatch
+ * runs), "blockwise_pair", and "blockwise_bn256+columns_bnW" where
  * the columns of the thin last wave go to a second launch with W-wide tiles).  For the dense kernels "+splitkS"
  * after a form's name means that the tiles of its last wave go to the split-K kernel with S splits, and "splitkS" alone
  * that the whole grid does (an output that is 16-byte aligned is assumed). */
