@@ -469,10 +469,19 @@ int make_output_map(CUtensorMap* map, void* out, int64_t M, int64_t N, int64_t l
     return cached_map(map, key);
 }
 
+// Threads of a dense launch: eight epilogue warps where the epilogue stands alone at the end of the grid's only wave (or of two, if the
+// rows have to be written without TMA, which takes several times as long); four where it runs under the next tile's MMAs, where
+// eight only disturb them.  us a call with four / eight: 1024 x 4096 x 4096 17.4 / 16.8, 777 x 5003 x 3088 22.8 / 21.5, 1500 x 5003 x 3088 (two waves)
+// 31.1 / 30.1, 100 x 1001 x 8192 19.2 / 18.8, 512 x 4096 x 4096 14.1 / 14.0; but 8192^3 320.5 / 325.5, 2048 x 11003 x 4096 (five waves) 62.7 / 63.6.
+int dense_threads(int64_t tiles, int64_t slots, bool tma_rows)
+{
+    return tiles <= (tma_rows ? slots : 2 * slots) ? kDenseThreads : kDenseThreads - 32 * (kDenseEpilogueWarps / 2);
+}
+
 template <int BN, int STAGES, int EPI>
 int launch_dense(DeviceState* st, int slot, const int8_t* x, const int8_t* y, DenseParams p, cudaStream_t stream)
 {
-    constexpr size_t kStoreStage = 4 * 2 * 2048;  // four epilogue warps x two 32 x 64-byte blocks
+    constexpr size_t kStoreStage = kDenseEpilogueWarps * 2 * 2048;  // per epilogue warp two 32 x 64-byte blocks
     constexpr size_t smem = static_cast<size_t>(STAGES) * (kBM + BN) * kBK + kStoreStage + 1024;
     auto kernel = dense_gemm_kernel<BN, STAGES, EPI>;
     if (int rc = ensure_smem(st, slot, kernel, smem)) return rc;
@@ -492,7 +501,7 @@ int launch_dense(DeviceState* st, int slot, const int8_t* x, const int8_t* y, De
     const int64_t tiles = p.tile_end > 0 ? p.tile_end : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
     const int grid = static_cast<int>(tiles < st->sm_count ? tiles : st->sm_count);
     p.release_late = p.tile_end == 0 && !p.after_quant && tiles <= st->sm_count && release_late(tiles, st->sm_count);
-    return launch(kernel, dim3(grid), kDenseThreads, smem, stream, dim3(1), p.dependent, mx, my, mo, p);
+    return launch(kernel, dim3(grid), dense_threads(tiles, st->sm_count, EPI == EPI_RAW_I32 || p.tma_store), smem, stream, dim3(1), p.dependent, mx, my, mo, p);
 }
 
 // Two-CTA form of the dense kernel: 256 x 256 tiles, one CTA pair (2 x 1 x 1 cluster) per tile.
@@ -500,7 +509,7 @@ template <int EPI>
 int launch_dense_pair(DeviceState* st, int slot, const int8_t* x, const int8_t* y, DenseParams p, cudaStream_t stream)
 {
     constexpr int BN = 256, STAGES = 6;
-    constexpr size_t kStoreStage = 4 * 2 * 2048;
+    constexpr size_t kStoreStage = kDenseEpilogueWarps * 2 * 2048;
     constexpr size_t smem = static_cast<size_t>(STAGES) * (kBM + BN / 2) * kBK + kStoreStage + 1024;
     auto kernel = dense_gemm_kernel<BN, STAGES, EPI, true>;
     if (int rc = ensure_smem(st, slot, kernel, smem)) return rc;
@@ -518,7 +527,7 @@ int launch_dense_pair(DeviceState* st, int slot, const int8_t* x, const int8_t* 
     p.group_m = pick_group_m(p.K) / 2 > 0 ? pick_group_m(p.K) / 2 : 1;
     const int64_t tiles = p.tile_end > 0 ? p.tile_end : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
     const int pairs = static_cast<int>(tiles < st->sm_count / 2 ? tiles : st->sm_count / 2);
-    return launch(kernel, dim3(2 * pairs), kDenseThreads, smem, stream, dim3(2), p.dependent, mx, my, mo, p);
+    return launch(kernel, dim3(2 * pairs), dense_threads(tiles, st->sm_count / 2, EPI == EPI_RAW_I32 || p.tma_store), smem, stream, dim3(2), p.dependent, mx, my, mo, p);
 }
 
 // Split-K launch for tiles [tile_begin, tile_begin + units / halves) of the grid described by p (tiles_m, tiles_n,
@@ -538,7 +547,7 @@ int launch_dense_splitk(DeviceState* st, int slot, const int8_t* x, const int8_t
     // 70 x 14336 x 16400 53.3 / 55.4; but 20 x 13952 x 14352 49.5 / 48.0, with its quantiser 100 x 13952 x 14352 66.6 / 63.8, K a multiple of 32
     // 100 x 13952 x 14336 47.3 / 45.1, and four splits 200 x 4096 x 14352 31.6 / 28.3.
     if (q.splits == 2 && p.K % 32 != 0 && p.M > kSmallMMaxM && !p.after_quant) p.dependent = 0;
-    return launch(kernel, dim3(q.units * q.splits), kDenseThreads, smem, stream, dim3(q.splits), q.after_main || p.dependent, mx, my, p, q);
+    return launch(kernel, dim3(q.units * q.splits), kSplitKThreads, smem, stream, dim3(q.splits), q.after_main || p.dependent, mx, my, p, q);
 }
 
 // The last wave of a persistent grid costs as much as a full one however few tiles it holds.  When it is thin -- or

@@ -9,8 +9,8 @@
 //   warp 1      MMA issuer: one thread issues tcgen05.mma kind::i8 (128 x BN x 32 per instruction),
 //               int32 accumulators live in tensor memory; two accumulator buffers so the epilogue of
 //               tile i overlaps the main loop of tile i+1.
-//   warps 2..5  epilogue: tcgen05.ld the accumulator (each warp owns the 32-lane quarter warp_id % 4),
-//               apply the epilogue in registers, store to global.
+//   warps 2..5 or 2..9  epilogue: tcgen05.ld the accumulator (a warp owns the 32-lane quarter warp_id % 4, and with eight warps half
+//               of the columns), apply the epilogue in registers, store to global.
 // Every mbarrier wait is bounded; on expiry the CTA records an error code and drains.
 #pragma once
 
@@ -21,7 +21,8 @@ namespace gi8 {
 constexpr int kBM = 128;       // rows of X per tile = UMMA M
 constexpr int kBK = 128;       // int8 elements (= bytes) of K per pipeline stage = one swizzle row
 constexpr int kUmmaK = 32;     // K per tcgen05.mma kind::i8
-constexpr int kDenseThreads = 192;
+constexpr int kDenseEpilogueWarps = 8;  // at most: the launch has four or eight (see the host's epilogue_warps)
+constexpr int kDenseThreads = 64 + 32 * kDenseEpilogueWarps;
 
 enum Epilogue : int {
     EPI_ALPHA_BF16 = 0,   // bf16( fp32(acc) * alpha )                       reference semantics
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1)
 dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                   const __grid_constant__ CUtensorMap map_out, const DenseParams p)
 {
-    static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "BN must be a multiple of 32 up to 256");
+    static_assert(BN == 64 || BN == 128 || BN == 256, "BN must be 64, 128 or 256");
     constexpr uint32_t kBytesA = kBM * kBK;
     constexpr int kTileM = PAIR ? 2 * kBM : kBM;       // rows of the (pair's) tile
     constexpr int kRowsB = PAIR ? BN / 2 : BN;         // rows of y this CTA loads
@@ -217,7 +218,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bar_acc_full[b], 1);
-            mbar_init(&bar_acc_empty[b], PAIR ? 8 : 4);
+            mbar_init(&bar_acc_empty[b], (PAIR ? 2 : 1) * (blockDim.x / 32 - 2));
         }
         fence_barrier_init();
         prefetch_tensormap(&map_x);
@@ -351,6 +352,9 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     } else {
         // ------------------------------------------------------------------ epilogue warps
         const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter + 32)
+        // All columns of the tile with four warps, half of them with eight.
+        const int c_count = blockDim.x == kDenseThreads ? BN / 2 : BN;
+        const int c_begin = ((warp - 2) >> 2) * c_count;
         uint32_t local_tile = 0;
         bool ok = true;
         for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
@@ -371,7 +375,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             if constexpr (EPI == EPI_ROWCOL_BF16) row_scale = row_ok ? __ldg(p.sx + row) : 0.0f;
 
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
+            for (int c = c_begin; c < c_begin + c_count; c += 32) {
                 uint32_t v[32];
                 __syncwarp();  // tcgen05.ld is warp-collective: reconverge after the predicated stores
                 tmem_ld_32x32b_x32(taddr + c, v);

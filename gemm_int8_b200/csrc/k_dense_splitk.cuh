@@ -24,6 +24,7 @@ namespace gi8 {
 
 constexpr int kSplitKBN = 256;
 constexpr int kSplitKStages = 4;
+constexpr int kSplitKThreads = 192;
 
 struct SplitKParams {
     int tile_begin;     // first tile (in the numbering of the main launch's tile grid) this launch covers
@@ -42,7 +43,7 @@ GI8_DEVICE void st_dsmem_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint3
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(kDenseThreads, 1)
+__global__ void __launch_bounds__(kSplitKThreads, 1)
 dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const DenseParams p, const SplitKParams q)
 {
