@@ -60,8 +60,8 @@
 //                      needs the producer to refill stage s, which needs bar_done[s] of K block `it`, i.e. every waiting
 //                      issuer's own commit: gated by each waiter.
 //   bar_done[s]        completed by the issuer's commit for K block `it` (with column halves by both issuers').  Waiters: the
-//                      producer (before refilling s; the next completion needs its own refill: gated) and, without column
-//                      halves, all promotion warps (the next completion is K block it + STAGES, whose MMAs need partial buffer
+//                      producer (before refilling s, and at its end for the stages not refilled; the next completion needs its own
+//                      refill: gated) and, without column halves, all promotion warps (the next completion is K block it + STAGES, whose MMAs need partial buffer
 //                      (it + STAGES) % NBUF handed back by every warp for K block it + STAGES - NBUF >= it: gated).
 //   bar_part_full[h][b]   column halves: completed by the commit of half h of a K block in buffer b.  Waiters: the promotion warps;
 //                      the next completion needs MMAs into that half, which need its hand-back by each of them: gated.
@@ -444,18 +444,9 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     if (++s == STAGES) s = 0, ph ^= 1;
                 }
             }
-            // Drain: every armed stage must have landed before the CTA may exit (PAIR: the leader's barriers complete
-            // only when both CTAs' bytes have landed; the peer leaves through the final cluster barrier).  (s, ph) is
-            // the slot after the last armed one; walk backwards over the armed stages.
-            if (PAIR && rank != 0) armed = 0;
-            for (uint32_t j = 0; j < armed; ++j) {
-                if (s == 0) s = STAGES, ph ^= 1;
-                --s;
-                if (!mbar_wait(&bar_full[s], ph)) {
-                    if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_DRAIN);
-                    break;
-                }
-            }
+            // (PAIR: as in the dense kernel.  With column halves the promotion warps wait for bar_part_full, whose commit comes
+            // before the one onto bar_done: this is the only wait for the last arrivals on bar_done.)
+            drain_stages<STAGES>(PAIR && rank != 0 ? nullptr : bar_full, bar_done, s, ph, armed, p.status, &abort_flag);
         } else if ((warp == 1 || (NISS == 2 && warp == 3)) && rank == 0) {
             // -------------------------------------------------------------- MMA issuer(s) (PAIR: the leader's)
             const uint32_t me = warp == 1 ? 0u : 1u;

@@ -149,14 +149,7 @@ blockwise_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             __syncwarp();
             if (++s == STAGES) s = 0, ph ^= 1;
         }
-        // Drain: what was requested must have landed before the CTA may exit.
-        for (int j = 1; j <= min(issued, STAGES); ++j) {
-            const int i = issued - j;
-            if (!mbar_wait(&bar_full[i % STAGES], (i / STAGES) & 1)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_DRAIN);
-                break;
-            }
-        }
+        drain_stages<STAGES>(bar_full, bar_done, issued % STAGES, (issued / STAGES) & 1, min(issued, STAGES), p.status, &abort_flag);
     } else if (warp == 3 || warp == 7) {
         // ---------------------------------------------------------------------------------- MMA issuers
         // The MMAs of the two K blocks of a stage alternate: each accumulates onto the one before the last, not onto the last.

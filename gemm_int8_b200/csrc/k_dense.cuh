@@ -89,6 +89,27 @@ GI8_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile uint32_t*
     return wait_or_abort_addr(smem_u32(bar), parity, abort_flag, limit_ns);
 }
 
+// End of a producer (whole warp): before the CTA may exit, every stage that it armed must have landed (bar_full, null where another
+// CTA's barriers count the bytes) AND have been handed back by the issuer's commit (bar_done, which this CTA has to itself).  The
+// second implies the first unless a role has aborted; nobody else waits for the last commits onto bar_done, and an arrival that
+// is still on its way when the CTA exits lands in shared memory that belongs to another CTA by then: completion of a later
+// commit (the accumulator's) does not say that the arrivals of the earlier ones have been made.  (s, ph) is the slot after
+// the last armed one; the walk is backwards.
+template <int STAGES>
+GI8_DEVICE void drain_stages(uint64_t* bar_full, uint64_t* bar_done, uint32_t s, uint32_t ph, uint32_t armed, uint32_t* status,
+                             volatile uint32_t* abort_flag)
+{
+    for (uint32_t j = 0; j < armed; ++j) {
+        if (s == 0) s = STAGES, ph ^= 1;
+        --s;
+        const bool landed = __all_sync(0xffffffffu, !bar_full || mbar_wait(&bar_full[s], ph));
+        const bool done = __all_sync(0xffffffffu, wait_or_abort(&bar_done[s], ph, abort_flag));
+        if (landed && done) continue;
+        if ((threadIdx.x & 31) == 0) raise_error(status, abort_flag, ERR_TIMEOUT_DRAIN);
+        if (!landed) return;
+    }
+}
+
 // Maps a linear tile index to (m block, n block).  Tiles are walked in bands of kGroupM row-blocks so
 // that the tiles resident at one time share X rows and Y rows in L2.
 GI8_DEVICE void tile_coords(int tile, int tiles_m, int tiles_n, int& mb, int& nb, int kGroupM = 8)
@@ -283,18 +304,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 if (++s == STAGES) s = 0, ph ^= 1;
             }
         }
-        // Drain: every armed stage must have landed before the CTA may exit (PAIR: the leader's barriers complete
-        // only when both CTAs' bytes have landed; the peer leaves through the final cluster barrier).  (s, ph) is the
-        // slot after the last armed one; walk backwards.
-        if (PAIR && rank != 0) armed = 0;
-        for (uint32_t j = 0; j < armed; ++j) {
-            if (s == 0) s = STAGES, ph ^= 1;
-            --s;
-            if (!mbar_wait(&bar_full[s], ph)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_DRAIN);
-                break;
-            }
-        }
+        // (PAIR: the leader's bar_full complete only when both CTAs' bytes have landed; the peer's own are never used)
+        drain_stages<STAGES>(PAIR && rank != 0 ? nullptr : bar_full, bar_empty, s, ph, armed, p.status, &abort_flag);
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         if (rank == 0) {

@@ -133,15 +133,8 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             issued = i + 1;
             if (++s == STAGES) s = 0, ph ^= 1;
         }
-        // Drain: every armed stage must have landed before the buffers are reused or the CTA exits.
-        const int armed = issued < STAGES ? issued : STAGES;
-        for (int j = 0; j < armed; ++j) {
-            const int i2 = issued - 1 - j;
-            if (!mbar_wait(&bar_full[i2 % STAGES], (i2 / STAGES) & 1)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_DRAIN);
-                break;
-            }
-        }
+        // (also before the buffers are used again)
+        drain_stages<STAGES>(bar_full, bar_empty, s, ph, min(issued, STAGES), p.status, &abort_flag);
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         uint32_t s = 0, ph = 0;

@@ -108,6 +108,7 @@ smallm_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (remaining stages)
+        int armed_to = 0;
         if (lane == 0) {
             const uint64_t pol_w = l2_policy_evict_first();
             const uint64_t pol_x = l2_policy_evict_last();
@@ -125,15 +126,10 @@ smallm_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 tma_load_2d_hint(sw_tile + kBytesW, &map_x, &bar_full[s], (kb_begin + i * kb_step) * kBK, 0, pol_x);
                 issued = i + 1;
             }
-            const int armed = issued < STAGES ? issued : STAGES;
-            for (int j = 0; j < armed; ++j) {
-                const int i2 = issued - 1 - j;
-                if (!mbar_wait(&bar_full[i2 % STAGES], (i2 / STAGES) & 1)) {
-                    raise_error(p.status, &abort_flag, ERR_TIMEOUT_DRAIN);
-                    break;
-                }
-            }
+            armed_to = issued;
         }
+        armed_to = __shfl_sync(0xffffffffu, armed_to, 0);
+        drain_stages<STAGES>(bar_full, bar_empty, armed_to % STAGES, (armed_to / STAGES) & 1, min(armed_to, STAGES), p.status, &abort_flag);
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         if (lane == 0 && num_kb > 0) {
@@ -365,14 +361,7 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             issued = i + 1;
             if (++s == STAGES) s = 0, ph ^= 1;
         }
-        const int armed = issued < STAGES ? issued : STAGES;
-        for (int j = 0; j < armed; ++j) {
-            const int i2 = issued - 1 - j;
-            if (!mbar_wait(&bar_full[i2 % STAGES], (i2 / STAGES) & 1)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_DRAIN);
-                break;
-            }
-        }
+        drain_stages<STAGES>(bar_full, bar_empty, issued % STAGES, (issued / STAGES) & 1, min(issued, STAGES), p.status, &abort_flag);
     } else if (warp == 1) {
         bool ok = num_kb > 0;
         uint32_t s = 0, ph = 0;

@@ -1,0 +1,38 @@
+"""Waits that the kernels must not miss, read from their sources: what they guard against (an arrival in shared memory that belongs to
+another CTA by then, a warp whose lanes part) shows in no result, and provoking it would hang or corrupt a GPU."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gemm_int8_b200", "csrc")
+
+
+def _kernels():
+    """(name, body) of every kernel that issues tensor-core work, comments removed."""
+    found = []
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith(".cuh"):
+            continue
+        with open(os.path.join(CSRC, f)) as fh:
+            text = re.sub(r"//[^\n]*", "", fh.read())
+        for m in re.finditer(r"__global__[^;{]*?\n(\w+)\(const __grid_constant__", text):
+            body = text[m.end():text.index("\n}\n", m.end())]
+            if "umma_commit" in body:
+                found.append(pytest.param(body, id=m.group(1)))
+    return found
+
+
+def test_all_kernels_are_seen():
+    names = {p.id for p in _kernels()}
+    assert names == {"dense_gemm_kernel", "dense_splitk_kernel", "smallm_gemm_kernel", "smallm_cluster_kernel", "blockwise_gemm_kernel",
+                     "blockwise_smallm_kernel"}
+
+
+@pytest.mark.parametrize("body", _kernels())
+def test_last_commits_are_awaited(body):
+    """The barrier that the issuer's commits hand a stage back on is waited for to the last of them, by the producer of each CTA."""
+    ring = "bar_done" if re.search(r"\bbar_done\[", body) else "bar_empty"
+    assert re.search(r"umma_commit\(&%s\[|umma_commit_pair\(map_to_cta\((smem_u32\(&%s\[|done_0)" % (ring, ring), body)
+    drains = re.findall(r"drain_stages<STAGES>\(([^;]*)\);", body)
+    assert len(drains) == 1 and re.search(r"bar_full, %s, " % ring, drains[0])
