@@ -367,6 +367,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const int c_count = blockDim.x == kDenseThreads ? BN / 2 : BN;
         const int c_begin = ((warp - 2) >> 2) * c_count;
         uint32_t local_tile = 0;
+        uint32_t staged = 0;  // chunks that this warp has staged, over all its tiles: its two blocks alternate whatever a tile's count of chunks
         bool ok = true;
         for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
             int mb, nb;
@@ -423,7 +424,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                     // the rows, the warp writes them out row by row.
                     const int row0 = mb * kTileM + static_cast<int>(rank) * kBM + quarter * 32;
                     if (row0 >= p.M) continue;  // warp-uniform
-                    uint8_t* stg = store_stage + ((warp - 2) * 2 + ((c >> 5) & 1)) * 2048;
+                    uint8_t* stg = store_stage + ((warp - 2) * 2 + (staged++ & 1)) * 2048;
                     if (p.tma_store && lane == 0) tma_store_wait_read<1>();  // the block staged two chunks ago has been read
                     __syncwarp();
 #pragma unroll

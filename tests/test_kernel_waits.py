@@ -36,3 +36,13 @@ def test_last_commits_are_awaited(body):
     assert re.search(r"umma_commit\(&%s\[|umma_commit_pair\(map_to_cta\((smem_u32\(&%s\[|done_0)" % (ring, ring), body)
     drains = re.findall(r"drain_stages<STAGES>\(([^;]*)\);", body)
     assert len(drains) == 1 and re.search(r"bar_full, %s, " % ring, drains[0])
+
+
+def test_staging_blocks_alternate_from_store_to_store():
+    """tma_store_wait_read<1> leaves the warp's latest store unread: the block staged next must be the other one, also when the latest store was
+    the last of an odd number in its tile.  So the dense kernel picks it by a count of its stores and not by the column."""
+    body = {p.id: p.values[0] for p in _kernels()}["dense_gemm_kernel"]
+    assert "tma_store_wait_read<1>" in body
+    pick = re.search(r"stg = store_stage \+ ([^;]*);", body).group(1)
+    assert "staged++" in pick and not re.search(r"\bc\b", pick)
+    assert "staged = 0" not in body.split("for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {")[-1]
