@@ -825,8 +825,8 @@ int get_static_scratch(void** out)
 
 }  // namespace
 
-// Exercises the bounded-wait error path without faulting or hanging anything: warp 1 waits (1 ms limit) on a barrier
-// that nobody ever arrives on, gives up, records ERR_TIMEOUT_EPILOGUE and raises the CTA's abort flag; warp 0 waits
+// Exercises the bounded-wait error path without faulting or hanging anything: half of warp 1 waits (1 ms limit) on a barrier
+// that nobody ever arrives on, the warp gives up, records ERR_TIMEOUT_EPILOGUE and raises the CTA's abort flag; warp 0 waits
 // on a second such barrier with the ordinary limit and must leave early because of the flag.  The kernel then
 // returns normally and the context stays usable.
 __global__ void wait_timeout_selftest_kernel(uint32_t* status)
@@ -840,9 +840,10 @@ __global__ void wait_timeout_selftest_kernel(uint32_t* status)
         gi8::fence_barrier_init();
     }
     __syncthreads();
-    if (threadIdx.x == 32) {
-        if (!gi8::wait_or_abort(&bar_never[0], 0, &abort_flag, 1000000ull))
-            gi8::raise_error(status, &abort_flag, gi8::ERR_TIMEOUT_EPILOGUE);
+    if (threadIdx.x >= 32) {
+        // A wait whose lanes end differently: the lower half's phase (the one before the first) is over, the upper half's never ends.
+        // The warp gives up as one, and its error is recorded.
+        gi8::warp_agrees(gi8::wait_or_abort(&bar_never[0], threadIdx.x < 48 ? 1u : 0u, &abort_flag, 1000000ull), status, &abort_flag, gi8::ERR_TIMEOUT_EPILOGUE);
     } else if (threadIdx.x == 0) {
         // returns false within microseconds of the flag being raised, long before its own 250 ms limit
         if (gi8::wait_or_abort(&bar_never[1], 0, &abort_flag)) gi8::raise_error(status, &abort_flag, gi8::ERR_TIMEOUT_PRODUCER);

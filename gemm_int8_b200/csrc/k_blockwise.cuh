@@ -420,8 +420,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 int mb, nb;
                 tile_coords(rotate_tile(tile, p.tile_rot, num_tiles), p.tiles_m, p.tiles_n, mb, nb, p.group_m);
                 for (int kb = tile == first_tile ? kb_early : 0; kb < num_kb; ++kb) {
-                    if (!wait_or_abort(&bar_done[s], ph ^ 1, &abort_flag)) {
-                        if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_PRODUCER);
+                    if (!warp_agrees(wait_or_abort(&bar_done[s], ph ^ 1, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) {
                         ok = false;
                         break;
                     }
@@ -470,14 +469,10 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             for (uint32_t it = first; it < total; it += kStep) {
                 // The operands first (they land long before the partial buffer is free), so that nothing but the
                 // MMAs stands between the buffer hand-back and the tensor core.
-                bool issued = wait_or_abort_addr(full_0 + 8 * s, ph, &abort_flag);
-                issued = issued && wait_or_abort_addr(empty_0 + 8 * buf, (SPLIT == 2 ? (bph >> buf) & 1u : bph) ^ 1, &abort_flag);
-                // (the vote keeps the loop, and with it the descriptors below, warp-uniform; the narrow tiles do not gain by it)
-                if constexpr (SPLIT == 2) issued = __all_sync(0xffffffffu, issued);
-                if (!issued) {
-                    if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
-                    break;
-                }
+                const bool ready = wait_or_abort_addr(full_0 + 8 * s, ph, &abort_flag) &&
+                                   wait_or_abort_addr(empty_0 + 8 * buf, (SPLIT == 2 ? (bph >> buf) & 1u : bph) ^ 1, &abort_flag);
+                // (the vote also keeps the loop, and with it the descriptors below, warp-uniform)
+                if (!warp_agrees(ready, p.status, &abort_flag, ERR_TIMEOUT_MMA)) break;
                 const uint32_t tmem_d = tmem_base + buf * BN + h * NSUB;
                 const uint32_t da = da_0 + s * (kStageBytes / 16), db = db_0 + s * (kStageBytes / 16);
                 tcgen05_fence_after_sync();
@@ -550,10 +545,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         [[maybe_unused]] const uint64_t unbias_b2 = f32x2(-static_cast<float>(kPartialBias) * 0x1p-22f, -static_cast<float>(kPartialBias) * 0x1p-22f);
         auto wait_partial = [&](uint32_t bar, uint32_t parity) {
             if (!__all_sync(0xffffffffu, polled)) {
-                bool got = wait_or_abort_addr(bar, parity, &abort_flag);
-                if (!got && lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
-                got = __all_sync(0xffffffffu, got);
-                if (!got) return false;
+                if (!warp_agrees(wait_or_abort_addr(bar, parity, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE)) return false;
             }
             tcgen05_fence_after_sync();
             return true;

@@ -138,10 +138,7 @@ blockwise_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         __syncwarp();
         int issued = first;
         for (uint32_t s = 0, ph = 0; issued < num_st; ++issued) {
-            if (!wait_or_abort(&bar_done[s], ph, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_PRODUCER);
-                break;
-            }
+            if (!warp_agrees(wait_or_abort(&bar_done[s], ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) break;
             if (elect_one()) {
                 load_w(issued, s);
                 load_x(issued, s);
@@ -157,12 +154,8 @@ blockwise_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         const uint32_t w_0 = smem_desc_lo(smem_u32(smem));
         uint32_t s = me, ph = 0;
         for (int i = me; i < num_st; i += 2) {
-            bool ready = wait_or_abort(&bar_full[s], ph, &abort_flag);
-            ready = ready && wait_or_abort(&bar_read[s], ph ^ 1, &abort_flag);
-            if (!__all_sync(0xffffffffu, ready)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
-                break;
-            }
+            const bool ready = wait_or_abort(&bar_full[s], ph, &abort_flag) && wait_or_abort(&bar_read[s], ph ^ 1, &abort_flag);
+            if (!warp_agrees(ready, p.status, &abort_flag, ERR_TIMEOUT_MMA)) break;
             tcgen05_fence_after_sync();
             const bool two = 2 * i + 1 < num_kb;
             const uint32_t dw = w_0 + s * (S::STAGE / 16), dw1 = dw + S::BYTES_W / 16;
@@ -210,10 +203,7 @@ blockwise_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         uint32_t s = 0, ph = 0;
         // Waits for the partials of stage (s, ph) and starts their load.
         auto fetch = [&](uint32_t (&r)[2][8]) {
-            bool ok = wait_or_abort(&bar_done[s], ph, &abort_flag);
-            if (!ok && lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads are warp-collective
-            if (!ok) return false;
+            if (!warp_agrees(wait_or_abort(&bar_done[s], ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE)) return false;
             tcgen05_fence_after_sync();
 #pragma unroll
             for (int j = 0; j < 2; ++j) tmem_ld_32x32b_x8(tm_warp + (s * 2 + j) * MT, r[j]);

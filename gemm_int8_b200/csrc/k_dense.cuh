@@ -89,6 +89,17 @@ GI8_DEVICE bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile uint32_t*
     return wait_or_abort_addr(smem_u32(bar), parity, abort_flag, limit_ns);
 }
 
+// Roles run their loops as whole warps, with full-mask instructions (elect.sync, __syncwarp, tcgen05.ld) behind every wait, which
+// have no limit of their own.  So the lanes decide together whether a bounded wait has failed: each looks at its own clock and
+// at the abort flag for itself, and one that left the loop alone would leave the others standing.  The error is
+// recorded whichever lane's wait it was.
+GI8_DEVICE bool warp_agrees(bool ok, uint32_t* status, volatile uint32_t* abort_flag, uint32_t code)
+{
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok && (threadIdx.x & 31) == 0) raise_error(status, abort_flag, code);
+    return ok;
+}
+
 // End of a producer (whole warp): before the CTA may exit, every stage that it armed must have landed (bar_full, null where another
 // CTA's barriers count the bytes) AND have been handed back by the issuer's commit (bar_done, which this CTA has to itself).  The
 // second implies the first unless a role has aborted; nobody else waits for the last commits onto bar_done, and an arrival that
@@ -103,10 +114,7 @@ GI8_DEVICE void drain_stages(uint64_t* bar_full, uint64_t* bar_done, uint32_t s,
         if (s == 0) s = STAGES, ph ^= 1;
         --s;
         const bool landed = __all_sync(0xffffffffu, !bar_full || mbar_wait(&bar_full[s], ph));
-        const bool done = __all_sync(0xffffffffu, wait_or_abort(&bar_done[s], ph, abort_flag));
-        if (landed && done) continue;
-        if ((threadIdx.x & 31) == 0) raise_error(status, abort_flag, ERR_TIMEOUT_DRAIN);
-        if (!landed) return;
+        if (!warp_agrees(landed && wait_or_abort(&bar_done[s], ph, abort_flag), status, abort_flag, ERR_TIMEOUT_DRAIN) && !landed) return;
     }
 }
 
@@ -279,8 +287,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             int mb, nb;
             tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb, p.group_m);
             for (int kb = 0; kb < num_kb; ++kb) {
-                if (!wait_or_abort(&bar_empty[s], ph ^ 1, &abort_flag)) {
-                    if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_PRODUCER);
+                if (!warp_agrees(wait_or_abort(&bar_empty[s], ph ^ 1, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) {
                     ok = false;
                     break;
                 }
@@ -315,15 +322,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
                 const uint32_t buf = local_tile & 1;
                 const uint32_t acc_ph = (local_tile >> 1) & 1;
-                if (!wait_or_abort(&bar_acc_empty[buf], acc_ph ^ 1, &abort_flag)) {
-                    if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
-                    break;
-                }
+                if (!warp_agrees(wait_or_abort(&bar_acc_empty[buf], acc_ph ^ 1, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_MMA)) break;
                 tcgen05_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + buf * BN;
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!wait_or_abort(&bar_full[s], ph, &abort_flag)) {
-                        if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
+                    if (!warp_agrees(wait_or_abort(&bar_full[s], ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_MMA)) {
                         ok = false;
                         break;
                     }
@@ -374,8 +377,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb, p.group_m);
             const uint32_t buf = local_tile & 1;
             const uint32_t acc_ph = (local_tile >> 1) & 1;
-            if (!wait_or_abort(&bar_acc_full[buf], acc_ph, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
+            if (!warp_agrees(wait_or_abort(&bar_acc_full[buf], acc_ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE)) {
                 ok = false;
                 break;
             }

@@ -119,10 +119,7 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         uint32_t s = 0, ph = 0;
         int issued = 0;
         for (int i = 0; i < num_kb; ++i) {
-            if (!wait_or_abort(&bar_empty[s], ph ^ 1, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_PRODUCER);
-                break;
-            }
+            if (!warp_agrees(wait_or_abort(&bar_empty[s], ph ^ 1, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) break;
             if (elect_one()) {
                 uint8_t* sa = smem + s * kStageBytes;
                 mbar_arrive_expect_tx(&bar_full[s], kStageBytes);
@@ -140,8 +137,7 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (int i = 0; i < num_kb; ++i) {
-            if (!wait_or_abort(&bar_full[s], ph, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
+            if (!warp_agrees(wait_or_abort(&bar_full[s], ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_MMA)) {
                 ok = false;
                 break;
             }
@@ -163,11 +159,9 @@ dense_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         // ------------------------------------------------------------------ epilogue warps: wait for the partial
         if (num_kb > 0) {
             // bar_acc_full completes only after every MMA has finished reading the pipeline buffers.
-            if (!wait_or_abort(&bar_acc_full, 0, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
+            if (!warp_agrees(wait_or_abort(&bar_acc_full, 0, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE)) {
                 acc_ok = false;
             }
-            acc_ok = __all_sync(0xffffffffu, acc_ok);  // the tensor-memory loads below are warp-collective
             tcgen05_fence_after_sync();
         }
     }

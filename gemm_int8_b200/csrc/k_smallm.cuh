@@ -162,12 +162,10 @@ smallm_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t v[MT];
         bool ok = true;
         if (num_kb > 0) {
-            if (!wait_or_abort(&bar_acc_full, 0, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
+            if (!warp_agrees(wait_or_abort(&bar_acc_full, 0, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE)) {
                 ok = false;
             }
             tcgen05_fence_after_sync();
-            __syncwarp();
             if (ok) {
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll
@@ -347,10 +345,7 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         int issued = min(num_kb, STAGES);
         uint32_t s = 0, ph = 0;
         for (int i = STAGES; i < num_kb; ++i) {
-            if (!wait_or_abort(&bar_empty[s], ph, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_PRODUCER);
-                break;
-            }
+            if (!warp_agrees(wait_or_abort(&bar_empty[s], ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) break;
             if (elect_one()) {
                 uint8_t* sw_tile = smem + s * kStageBytes;
                 mbar_arrive_expect_tx(&bar_full[s], kBytesW + kBytesX);
@@ -363,15 +358,10 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
         drain_stages<STAGES>(bar_full, bar_empty, issued % STAGES, (issued / STAGES) & 1, min(issued, STAGES), p.status, &abort_flag);
     } else if (warp == 1) {
-        bool ok = num_kb > 0;
         uint32_t s = 0, ph = 0;
         const uint32_t w_0 = smem_desc_lo(smem_u32(smem));
         for (int i = 0; i < num_kb; ++i) {
-            ok = __all_sync(0xffffffffu, wait_or_abort(&bar_full[s], ph, &abort_flag));
-            if (!ok) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_MMA);
-                break;
-            }
+            if (!warp_agrees(wait_or_abort(&bar_full[s], ph, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_MMA)) break;
             tcgen05_fence_after_sync();
             const uint32_t dw = w_0 + s * (kStageBytes / 16), dx = dw + kBytesW / 16;
             if (elect_one()) {
@@ -398,11 +388,9 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
         bool ok = true;
         if (num_kb > 0) {
-            if (!wait_or_abort(&bar_acc_full, 0, &abort_flag)) {
-                if (lane == 0) raise_error(p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE);
+            if (!warp_agrees(wait_or_abort(&bar_acc_full, 0, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_EPILOGUE)) {
                 ok = false;
             }
-            ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below are warp-collective
             tcgen05_fence_after_sync();
         }
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);

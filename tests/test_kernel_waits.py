@@ -46,3 +46,21 @@ def test_staging_blocks_alternate_from_store_to_store():
     pick = re.search(r"stg = store_stage \+ ([^;]*);", body).group(1)
     assert "staged++" in pick and not re.search(r"\bc\b", pick)
     assert "staged = 0" not in body.split("for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {")[-1]
+
+
+@pytest.mark.parametrize("body", _kernels())
+def test_lanes_of_a_warp_decide_together(body):
+    """Full-mask instructions stand behind every bounded wait, so whether it has failed is a vote (only the roles of a single thread do without)."""
+    waits = 0
+    for m in re.finditer(r"\bwait_or_abort(?:_addr)?\(", body):
+        start = max(body.rfind(c, 0, m.start()) for c in ";{}")
+        end = m.start() + re.search(r"[;{]", body[m.start():]).start()
+        statement = body[start + 1:end]
+        if "const bool ready =" in statement:
+            statement = body[start + 1:body.index(";", end + 1)]
+            assert "warp_agrees(ready," in statement
+        if "warp_agrees(" not in statement:
+            role = body[:start].rfind("if (lane == 0")
+            assert role > body[:start].rfind("} else if (warp == ") and "elect_one" not in body[role:start], statement
+        waits += 1
+    assert waits >= 3
