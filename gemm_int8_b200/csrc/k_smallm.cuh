@@ -241,7 +241,7 @@ smallm_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 // Cluster variant: the SPLITS CTAs that share one weight tile form a thread-block cluster (1 x SPLITS x 1,
 // SPLITS <= 8).  Token row m belongs to CTA m % SPLITS: every CTA sends its int32 partials of that row straight
 // from registers into the owner's receive area (remote shared-memory stores, which do not stall the sender);
-// after ONE cluster barrier each owner sums what it received from its own shared memory, applies the scales and
+// after a cluster barrier each owner sums what it received from its own shared memory, applies the scales and
 // stores bf16.  After that barrier nobody touches a peer's memory, so CTAs leave independently.  The receive
 // area lies behind the pipeline buffers (a fast peer may send while the owner is still streaming weights).
 // No global scratch, no atomics, and the sum is exact whatever the order.  The cluster barrier is a hardware
@@ -322,6 +322,9 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     tcgen05_fence_before_sync();
     __syncthreads();
     tcgen05_fence_after_sync();
+    // A CTA's shared memory may be written by its peers only once it has started: all threads arrive here, and the senders wait for that
+    // phase (long over by then) before their first remote store.
+    if (p.splits > 1) cluster_arrive_relaxed();
     pdl_wait();  // every thread: scales are read and the output is written only after the previous kernel is done
     // What follows in the stream may start as SMs free up, but only now: a dependent that requests its weights before its own
     // wait must find everything written in front of THIS kernel, not only what this kernel writes.
@@ -393,6 +396,7 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             }
             tcgen05_fence_after_sync();
         }
+        if (p.splits > 1) cluster_wait();  // every CTA of the cluster runs
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
         const uint32_t recv_mine = smem_u32(recv) + (my_rank * rows_per_owner * kSmallMTileN + n_local) * 4u;
         uint32_t owner = 0, row_local = 0;  // of token row c + j, kept incrementally
@@ -428,6 +432,7 @@ smallm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     tcgen05_fence_before_sync();
     if (p.splits > 1) {
+        if (warp < 2) cluster_wait();  // (the phase that the senders have waited for)
         cluster_sync_all();  // every partial has landed in its owner's receive area
         if (warp >= 2) {
             const int n_local = (warp & 3) * 32 + lane;

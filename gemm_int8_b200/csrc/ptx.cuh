@@ -428,6 +428,10 @@ GI8_DEVICE void cluster_sync_all()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The two halves of a cluster barrier whose phase says only that every thread of the cluster has got this far.
+GI8_DEVICE void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+GI8_DEVICE void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 GI8_DEVICE uint32_t cluster_cta_rank()
 {
     uint32_t r;

@@ -64,3 +64,11 @@ def test_lanes_of_a_warp_decide_together(body):
             assert role > body[:start].rfind("} else if (warp == ") and "elect_one" not in body[role:start], statement
         waits += 1
     assert waits >= 3
+
+
+def test_remote_stores_follow_a_barrier_of_the_cluster():
+    """A peer's shared memory may be written only once its CTA has started: some cluster barrier lies before the first remote store."""
+    for p in _kernels():
+        m = re.search(r"\bst_dsmem_\w+\(", p.values[0])
+        if m:
+            assert re.search(r"\bcluster_(sync_all|wait)\(\)", p.values[0][:m.start()]), p.id
