@@ -1306,9 +1306,6 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
         default: bn = pick_bn(M, N, K, st->sm_count, true, &pair);
     }
     if (force_bn) bn = force_bn, pair = false;
-    // The first of two launches over columns: its tiles fill whole waves, of CTA pairs too where the row blocks are even in number,
-    // and the pair gains most by six stages (a rotated fp32 layer of 499 x 10240 x 8192 with bias, us: one-CTA tiles 80.1-81.1, pairs 78.4-78.9).
-    if (force_bn == 256 && pdl_role == 0 && ((M + kBM - 1) / kBM) % 2 == 0) pair = true;
     if (scatter && bn == 64) bn = 128;  // a 32 x 32 fp32 box needs the 4 KB staging block of the wider tiles
     p.pdl_role = pdl_role;
     // The epilogue's TMA-store boxes are 64 columns wide for the 256- and 128-wide tiles and 32 for the 64-wide one.

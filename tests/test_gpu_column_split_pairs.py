@@ -1,5 +1,5 @@
-"""The first launch of a column split runs on CTA pairs where the row blocks are even in number and on one-CTA tiles where they are odd;
-against the 128-wide tiles (the same bits; those are compared with the oracle elsewhere)."""
+"""Column splits of even and of odd counts of row blocks (the first launch runs on one-CTA tiles for both), against the 128-wide tiles (the same
+bits; those are compared with the oracle elsewhere)."""
 import pytest
 import torch
 
