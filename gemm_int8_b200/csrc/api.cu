@@ -1349,10 +1349,10 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
         if (p.tma_store)
             if (int rc = make_output_map(&mo.m[0], out, M, N, N, box_cols)) return rc;
     }
-#define GI8_LAUNCH_BW(BN_, ST_, SPLIT_, NISS_, PAIR_, BIAS_, SLOT_)                           \
+#define GI8_LAUNCH_BW(BN_, ST_, SPLIT_, NISS_, PAIR_, BIAS_, AHEAD_, SLOT_)                   \
     do {                                                                                      \
         constexpr size_t smem = blockwise_smem_bytes(BN_, ST_, PAIR_);                        \
-        auto kernel = blockwise_gemm_kernel<BN_, ST_, SPLIT_, NISS_, PAIR_, BIAS_>;           \
+        auto kernel = blockwise_gemm_kernel<BN_, ST_, SPLIT_, NISS_, PAIR_, BIAS_, AHEAD_>;   \
         if (int rc = ensure_smem(st, SLOT_, kernel, smem)) return rc;                         \
         return launch(kernel, dim3(grid), kBlockwiseThreads, smem, s, dim3(PAIR_ ? 2 : 1), pdl, mx, my, mo, p); \
     } while (0)
@@ -1362,26 +1362,29 @@ static int blockwise_impl(const int8_t* x, const int8_t* y, const float* sa, int
     const bool pdl = knobs().pdl && !scatter && n_out == 1;
     const bool two = knobs().bw_issuers == 2 || (knobs().bw_issuers == 0 && bn < 256);
     const bool halves = knobs().bw_halves != 1;
+    const bool ahead = tiles > 2 * static_cast<int64_t>(st->sm_count);  // one-CTA column halves; both sides stand in the kernel's header
     if (bias) {  // (the knobs below choose among forms without one)
-        if (pair) GI8_LAUNCH_BW(256, 6, 2, 2, true, true, 28);
-        if (bn == 256) GI8_LAUNCH_BW(256, 4, 2, 2, false, true, 29);
-        if (bn == 128) GI8_LAUNCH_BW(128, 6, 1, 2, false, true, 30);
-        GI8_LAUNCH_BW(64, 8, 1, 2, false, true, 31);
+        if (pair) GI8_LAUNCH_BW(256, 6, 2, 2, true, true, true, 28);
+        if (bn == 256 && ahead) GI8_LAUNCH_BW(256, 4, 2, 2, false, true, true, 35);
+        if (bn == 256) GI8_LAUNCH_BW(256, 4, 2, 2, false, true, false, 29);
+        if (bn == 128) GI8_LAUNCH_BW(128, 6, 1, 2, false, true, false, 30);
+        GI8_LAUNCH_BW(64, 8, 1, 2, false, true, false, 31);
     }
     if (pair) {
-        if (halves) GI8_LAUNCH_BW(256, 6, 2, 2, true, false, 21);
-        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, true, false, 22);
-        else GI8_LAUNCH_BW(256, 4, 1, 1, true, false, 23);
+        if (halves) GI8_LAUNCH_BW(256, 6, 2, 2, true, false, true, 21);
+        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, true, false, false, 22);
+        else GI8_LAUNCH_BW(256, 4, 1, 1, true, false, false, 23);
     } else if (bn == 256) {
-        if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, false, false, 13);
-        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, false, false, 15);
-        else GI8_LAUNCH_BW(256, 4, 1, 1, false, false, 16);
+        if (halves && ahead) GI8_LAUNCH_BW(256, 4, 2, 2, false, false, true, 34);
+        else if (halves) GI8_LAUNCH_BW(256, 4, 2, 2, false, false, false, 13);
+        else if (two) GI8_LAUNCH_BW(256, 4, 1, 2, false, false, false, 15);
+        else GI8_LAUNCH_BW(256, 4, 1, 1, false, false, false, 16);
     } else if (bn == 128) {
-        if (two) GI8_LAUNCH_BW(128, 6, 1, 2, false, false, 17);
-        else GI8_LAUNCH_BW(128, 6, 1, 1, false, false, 18);
+        if (two) GI8_LAUNCH_BW(128, 6, 1, 2, false, false, false, 17);
+        else GI8_LAUNCH_BW(128, 6, 1, 1, false, false, false, 18);
     } else {
-        if (two) GI8_LAUNCH_BW(64, 8, 1, 2, false, false, 19);
-        else GI8_LAUNCH_BW(64, 8, 1, 1, false, false, 20);
+        if (two) GI8_LAUNCH_BW(64, 8, 1, 2, false, false, false, 19);
+        else GI8_LAUNCH_BW(64, 8, 1, 1, false, false, false, 20);
     }
 #undef GI8_LAUNCH_BW
 }

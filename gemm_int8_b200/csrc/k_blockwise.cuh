@@ -8,14 +8,15 @@
 //   warpgroup 0 control (setmaxnreg.dec): warp 0 TMA producer (as in the dense kernel); warp 1 (and warp 3 when
 //               NISS == 2, taking alternate K blocks) MMA issuer -- per K block four tcgen05.mma kind::i8 with N = BN
 //               (or 2 x 4 with N = 128 when SPLIT == 2) that overwrite one of NBUF = 512 / BN tensor-memory partial
-//               buffers, then a commit that both frees the pipeline stage and publishes the partial (with column halves one
-//               commit for either); warp 2 allocates tensor memory.
+//               buffers, then ONE commit per column half that both frees the pipeline stage and publishes the
+//               partial (DECOUPLED: one commit for either); warp 2 allocates tensor memory.
 //   warps 4..11 promotion (setmaxnreg.inc): warp w owns TMEM lane quarter (w % 4) and BN/2 of the tile's columns
 //               (with column halves: 64 columns of each half), i.e. 32 rows x BN/2 columns, whose fp32
 //               accumulators it keeps in registers (as f32x2 pairs).  Per K block and half: tcgen05.ld the int32
-//               partial in chunks of 32 columns (column halves: 16, the next chunk's load running under the arithmetic of this
-//               one), hand the half back after the last load, and accumulate it with the block's scale.  A warp's segment never straddles a 128-wide weight-scale block.  At the end of the
-//               tile the same warps cast to bf16 and store through swizzled shared memory and TMA.
+//               partial in chunks of 32 columns (DECOUPLED: 16, the next chunk's load running under the arithmetic of
+//               this one), hand the half back after the last load, and accumulate it with the block's scale.  A
+//               warp's segment never straddles a 128-wide weight-scale block.  At the end of the tile the same
+//               warps cast to bf16 and store through swizzled shared memory and TMA.
 //
 // Two ways to accumulate, both one rounding per K block and element, the same bits:
 //   column halves (SPLIT == 2; both 256-wide forms as dispatched): no conversion.  A fifth MMA per K block, unsigned 255 x 255,
@@ -47,8 +48,13 @@
 // 800; one multiply-add instead of two 842.  Neither pipe alone: a K block's two hand-overs, during which the eight warps
 // do the same thing at the same time, lie between stretches of arithmetic (the loop without hand-overs takes 554).  Partial
 // buffers with barriers of their own (their ring positions are compile-time constants whatever the stage count), six stages
-// instead of four in the two-CTA form (four starved it: 1.5 us a round trip), loads one chunk ahead and a warp-uniform issue loop, all
-// together: 2048 x 11008 x 4096 95.6 -> 93.3 us, 8192^3 511 -> 492 (two-CTA 492 -> 478), 512 x 9472 x 16384 74.6 -> 73.9 (two-CTA 73.9 -> 72.1).
+// instead of four in the two-CTA form (four starved it: 1.5 us a round trip), loads one chunk ahead and a warp-uniform issue
+// loop, all together (DECOUPLED, on column halves): 8192^3 511 -> 492 us, two-CTA 492 -> 478, 512 x 9472 x 16384 two-CTA 73.9 -> 72.1.
+// One-CTA tiles keep the coupled form (one commit per half, plain 32-column loads) on grids of up to two waves, where the other loses,
+// most where weights stream past few tokens, us coupled / decoupled: 64 x 28672 x 8192 46.9 / 49.1, 100 x 37888 x 4096 32.9 / 33.9, 128 x
+// 37888 x 8192 62.0 / 63.5, 384 x 12544 x 8192 46.6 / 47.2, 1024 x 4096 x 8192 level; 1.5 to 2 waves: 384 x 25088 x 4096 50.0 / 52.0, 32 x
+// 57344 x 8192 92.6 / 95.0; more: 896 x 12544 x 4096 64.4 / 64.3, 900 x 12040 x 4096 66.1 / 64.7, 2048 x 8192 x 4096 85.3 / 83.4, 4096 x
+// 8192 x 4096 152.5 / 148.5, 8192^3 599 / 582.
 // Tried on top of that, us at 2048 x 11008 x 4096 (two-CTA): sixteen promotion warps, four a scheduler, 121; one issuer for both
 // halves 103; one lane instead of the warp at the barriers 132; N = 256 MMAs with one hand-over a K block 102; loads of 32 columns
 // one chunk ahead 119 (spills).
@@ -59,16 +65,17 @@
 //                      `it` (with column halves: both issuers, each of which visits every K block).  Next phase
 //                      needs the producer to refill stage s, which needs bar_done[s] of K block `it`, i.e. every waiting
 //                      issuer's own commit: gated by each waiter.
-//   bar_done[s]        completed by the issuer's commit for K block `it` (with column halves by both issuers').  Waiters: the
-//                      producer (before refilling s, and at its end for the stages not refilled; the next completion needs its own
-//                      refill: gated) and, without column halves, all promotion warps (the next completion is K block it + STAGES, whose MMAs need partial buffer
+//   bar_done[h][s]     completed by the issuer's commit for column half h of K block `it`.  Waiters: the producer (before refilling s,
+//                      and at its end for the stages not refilled; the next completion needs its own refill: gated) and all
+//                      promotion warps (the next completion is K block it + STAGES, whose MMAs need half h of partial buffer
 //                      (it + STAGES) % NBUF handed back by every warp for K block it + STAGES - NBUF >= it: gated).
-//   bar_part_full[h][b]   column halves: completed by the commit of half h of a K block in buffer b.  Waiters: the promotion warps;
-//                      the next completion needs MMAs into that half, which need its hand-back by each of them: gated.
+//                      DECOUPLED: one ring, completed by both issuers' commits, and only the producer waits.
+//   bar_part_full[h][b]   DECOUPLED: completed by the commit of half h of a K block in buffer b.  Waiters: the promotion warps; the
+//                      next completion needs MMAs into that half, which need its hand-back by each of them: gated.
 //   bar_part_empty[h][b]  completed by the arrivals of all eight promotion warps after their last load of half h of
 //                      a K block in buffer b.  Waiter: the issuer of half h of the next K block that uses b; the
 //                      completion after that needs this issuer's MMAs: gated.
-//   With column halves the buffer is the parity of the K block inside its tile: a tile of an odd count of K blocks ends and the next
+//   DECOUPLED: the buffer is the parity of the K block inside its tile: a tile of an odd count of K blocks ends and the next
 //   one begins with buffer 0, and each buffer's phase is counted by itself (issuers and promotion warps do the same).
 //   Without column halves and with two issuers, issuer j takes K blocks it % 2 == j, hence stages s % 2 == j and
 //   buffers b % 2 == j (STAGES and NBUF are even): every barrier still has exactly one issuing waiter, which sees
@@ -250,11 +257,12 @@ GI8_DEVICE int rotate_tile(int tile, int rot, int n)
     return t >= n ? t - n : t;
 }
 
-// Makes a 32-bit value opaque to the optimiser at this point, so that later uses read the register instead of
-// recomputing the value.
+// Loads of 16 or 32 columns, by the array.
 GI8_DEVICE void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_32x32b_x16(taddr, r); }
 GI8_DEVICE void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32b_x32(taddr, r); }
 
+// Makes a 32-bit value opaque to the optimiser at this point, so that later uses read the register instead of
+// recomputing the value.
 #define GI8_PIN(v) asm volatile("" : "+r"(v))
 
 // SPLIT = 2 (BN = 256 only): the MMAs of a K block are issued as two column halves (N = 128 each), each half by its
@@ -278,7 +286,7 @@ GI8_DEVICE void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32b_x32(
 // tile columns cg * 128 + h * 64 .. (still contiguous and inside one weight-scale block).
 // BIAS: a bf16 vector is added to the rounded result.  A template parameter, not a branch: with the branch in the epilogue
 // the K loop of the 256-wide forms was compiled 6 % slower (2048 x 11008 x 4096: 97 -> 103 us).
-template <int BN, int STAGES, int SPLIT, int NISS, bool PAIR = false, bool BIAS = false>
+template <int BN, int STAGES, int SPLIT, int NISS, bool PAIR, bool BIAS, bool DECOUPLED>
 __global__ void __launch_bounds__(kBlockwiseThreads, 1)
 blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                       const __grid_constant__ OutputMaps outs, const BlockwiseParams p)
@@ -291,16 +299,18 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     constexpr int NSUB = BN / SPLIT;     // N of one MMA = columns of one half
     constexpr int CW = BN / 2;           // columns per promotion warp (128, 64 or 32) ...
     constexpr int SEGW = CW / SPLIT;     // ... as SPLIT segments of SEGW columns, one in each half
-    constexpr int CHW = SPLIT == 2 ? 16 : 32;  // columns per tensor-memory load
+    static_assert(DECOUPLED ? SPLIT == 2 : !(PAIR && SPLIT == 2), "two-CTA column halves are decoupled, one-CTA ones may be, others are not");
+    constexpr int DONE_RINGS = SPLIT == 2 && !DECOUPLED ? 2 : 1;  // a ring of bar_done for each column half, or one
+    constexpr int CHW = DECOUPLED ? 16 : 32;  // columns per tensor-memory load
     constexpr int NC = SEGW / CHW;       // loads per segment
     constexpr int STORE_W = blockwise_store_cols(BN);
     static_assert(SEGW % STORE_W == 0 && SEGW % 32 == 0, "segments are whole store boxes and whole loads");
     // SPLIT == 1: each issuer must own the stages and the partial buffers of its K blocks (see the protocol above):
     // with an odd count an issuer would meet a barrier only every second phase, which a parity wait cannot tell apart.
     static_assert(SPLIT == 2 || (STAGES % NISS == 0 && NBUF % NISS == 0), "issuers must own their stages and partial buffers");
-    // Without column halves a promotion warp's parity wait on bar_done is safe only if the commit STAGES K blocks later needs a
-    // partial buffer that the same warp hands back after the awaited K block (see the protocol above).
-    static_assert(SPLIT == 2 || STAGES >= NBUF, "the stage ring must be at least as deep as the partial-buffer ring");
+    // A promotion warp's parity wait on bar_done is safe only if the commit STAGES K blocks later needs a partial buffer that the
+    // same warp hands back after the awaited K block (see the protocol above).
+    static_assert(DECOUPLED || STAGES >= NBUF, "the stage ring must be at least as deep as the partial-buffer ring");
     static_assert(!PAIR || BN == 256, "two-CTA tiles are 256 wide");
     constexpr bool BIASED = SPLIT == 2;
     constexpr int kTileM = PAIR ? 2 * kBM : kBM;  // rows of the (pair's) tile
@@ -319,8 +329,8 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
     __shared__ __align__(8) uint64_t bar_full[STAGES];
-    __shared__ __align__(8) uint64_t bar_done[STAGES];
-    __shared__ __align__(8) uint64_t bar_part_full[SPLIT][NBUF];  // column halves only
+    __shared__ __align__(8) uint64_t bar_done[DONE_RINGS][STAGES];
+    __shared__ __align__(8) uint64_t bar_part_full[SPLIT][NBUF];  // DECOUPLED only
     __shared__ __align__(8) uint64_t bar_part_empty[SPLIT][NBUF];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile uint32_t abort_flag;
@@ -339,7 +349,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&bar_full[s], 1);
-            mbar_init(&bar_done[s], SPLIT);
+            for (int r = 0; r < DONE_RINGS; ++r) mbar_init(&bar_done[r][s], DECOUPLED ? SPLIT : 1);
         }
         for (int b = 0; b < NBUF; ++b) {
             for (int h = 0; h < SPLIT; ++h) {
@@ -420,7 +430,9 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 int mb, nb;
                 tile_coords(rotate_tile(tile, p.tile_rot, num_tiles), p.tiles_m, p.tiles_n, mb, nb, p.group_m);
                 for (int kb = tile == first_tile ? kb_early : 0; kb < num_kb; ++kb) {
-                    if (!warp_agrees(wait_or_abort(&bar_done[s], ph ^ 1, &abort_flag), p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) {
+                    const bool ready = wait_or_abort(&bar_done[0][s], ph ^ 1, &abort_flag) &&
+                                       (DONE_RINGS == 1 || wait_or_abort(&bar_done[DONE_RINGS - 1][s], ph ^ 1, &abort_flag));
+                    if (!warp_agrees(ready, p.status, &abort_flag, ERR_TIMEOUT_PRODUCER)) {
                         ok = false;
                         break;
                     }
@@ -443,9 +455,9 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     if (++s == STAGES) s = 0, ph ^= 1;
                 }
             }
-            // (PAIR: as in the dense kernel.  With column halves the promotion warps wait for bar_part_full, whose commit comes
-            // before the one onto bar_done: this is the only wait for the last arrivals on bar_done.)
-            drain_stages<STAGES>(PAIR && rank != 0 ? nullptr : bar_full, bar_done, s, ph, armed, p.status, &abort_flag);
+            // (PAIR: as in the dense kernel.  DECOUPLED: the promotion warps wait for bar_part_full, whose commit comes before the
+            // one onto bar_done: this is the only wait for the last arrivals on bar_done.)
+            drain_stages<STAGES, DONE_RINGS>(PAIR && rank != 0 ? nullptr : bar_full, bar_done[0], s, ph, armed, p.status, &abort_flag);
         } else if ((warp == 1 || (NISS == 2 && warp == 3)) && rank == 0) {
             // -------------------------------------------------------------- MMA issuer(s) (PAIR: the leader's)
             const uint32_t me = warp == 1 ? 0u : 1u;
@@ -458,19 +470,19 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             const uint32_t total = static_cast<uint32_t>(my_tiles) * static_cast<uint32_t>(num_kb);
             // stage / partial buffer of K block `it` and their phase parities, stepped without divisions
             uint32_t s = first, ph = 0, buf = first, bph = 0;
-            // column halves: the buffer is the parity of the K block inside its tile, bit b of bph the phase of buffer b
+            // DECOUPLED: the buffer is the parity of the K block inside its tile, bit b of bph the phase of buffer b
             [[maybe_unused]] int kb_in_tile = 0;
             [[maybe_unused]] const uint64_t d_ones = make_smem_desc_ones(smem_u32(ones_tile));
             // Half h: rows h * NSUB.. of the weight tile (PAIR: rows h * NSUB / 2.. of each CTA's half of it) into columns h * NSUB..
             // of the partial buffer.
             const uint32_t da_0 = smem_desc_lo(smem_u32(smem)), db_0 = smem_desc_lo(smem_u32(smem) + kBytesA + h * (PAIR ? NSUB / 2 : NSUB) * kBK);
-            const uint32_t full_0 = smem_u32(&bar_full[0]), done_0 = smem_u32(&bar_done[0]);
+            const uint32_t full_0 = smem_u32(&bar_full[0]), done_0 = smem_u32(&bar_done[0][0]);
             const uint32_t empty_0 = smem_u32(&bar_part_empty[h][0]), part_0 = smem_u32(&bar_part_full[h][0]);
             for (uint32_t it = first; it < total; it += kStep) {
                 // The operands first (they land long before the partial buffer is free), so that nothing but the
                 // MMAs stands between the buffer hand-back and the tensor core.
                 const bool ready = wait_or_abort_addr(full_0 + 8 * s, ph, &abort_flag) &&
-                                   wait_or_abort_addr(empty_0 + 8 * buf, (SPLIT == 2 ? (bph >> buf) & 1u : bph) ^ 1, &abort_flag);
+                                   wait_or_abort_addr(empty_0 + 8 * buf, (DECOUPLED ? (bph >> buf) & 1u : bph) ^ 1, &abort_flag);
                 // (the vote also keeps the loop, and with it the descriptors below, warp-uniform)
                 if (!warp_agrees(ready, p.status, &abort_flag, ERR_TIMEOUT_MMA)) break;
                 const uint32_t tmem_d = tmem_base + buf * BN + h * NSUB;
@@ -488,21 +500,21 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                         else umma_i8(tmem_d, d_ones, d_ones, make_idesc_u8(kTileM, NSUB), 1u);
                     }
                     if constexpr (PAIR) {
-                        if constexpr (SPLIT == 2) {
+                        if constexpr (DECOUPLED) {
                             umma_commit_pair(map_to_cta(part_0 + 8 * buf, 0));
                             umma_commit_pair(map_to_cta(part_0 + 8 * buf, 1));
                         }
                         umma_commit_pair(map_to_cta(done_0 + 8 * s, 0));
                         umma_commit_pair(map_to_cta(done_0 + 8 * s, 1));
                     } else {
-                        if constexpr (SPLIT == 2) umma_commit(&bar_part_full[h][buf]);
-                        umma_commit(&bar_done[s]);
+                        if constexpr (DECOUPLED) umma_commit(&bar_part_full[h][buf]);
+                        umma_commit(&bar_done[DONE_RINGS == 2 ? h : 0][s]);
                     }
                 }
                 __syncwarp();
                 s += kStep;
                 if (s >= STAGES) s -= STAGES, ph ^= 1;
-                if constexpr (SPLIT == 2) {
+                if constexpr (DECOUPLED) {
                     bph ^= 1u << buf;
                     buf ^= 1u;
                     if (++kb_in_tile == num_kb) kb_in_tile = 0, buf = 0;
@@ -523,16 +535,20 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         // issue.
         uint32_t tm_warp = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(cg * SEGW);
         GI8_PIN(tm_warp);
-        uint32_t bar_part_0 = SPLIT == 2 ? smem_u32(&bar_part_full[0][0]) : smem_u32(&bar_done[0]);
+        uint32_t bar_part_0 = DECOUPLED ? smem_u32(&bar_part_full[0][0]) : smem_u32(&bar_done[0][0]);
         // (PAIR: the hand-back barriers are the leader's, addressed through the cluster window)
         uint32_t bar_empty_0 = PAIR ? map_to_cta(smem_u32(&bar_part_empty[0][0]), 0) : smem_u32(&bar_part_empty[0][0]);
         GI8_PIN(bar_part_0);
         GI8_PIN(bar_empty_0);
-        // Narrow tiles: stage, partial buffer and barrier phase of the running K block (as in the MMA issuer), stepped without
-        // divisions: byte offset of the stage's barrier, its parity, byte offset of the buffer's barrier, the buffer's first
-        // column.
+        // Stage, partial buffer and barrier phase of the running K block (as in the MMA issuer), stepped without divisions: byte
+        // offset of the stage's barrier, its parity, byte offset of the buffer's barrier, the buffer's first column.
         [[maybe_unused]] uint32_t st_off = 0, st_par = 0, buf_off = 0, buf_col = 0;
-        // Column halves: bit b is the phase of partial buffer b.
+        // With four stages, two partial buffers and K blocks handled four at a time (the vector-scale path, whose K block count is
+        // a multiple of four), every tile starts at stage 0 and buffer 0: the ring positions of the four K blocks of a group are
+        // compile-time constants and only the parity, flipped once per group, lives in a register.  That removes the
+        // counter arithmetic (about ten instructions per warp and K block on the integer pipe).
+        constexpr bool kStaticRing = !DECOUPLED && STAGES == 4 && NBUF == 2;
+        // DECOUPLED: bit b is the phase of partial buffer b.
         [[maybe_unused]] uint32_t buf_par = 0;
         bool ok = true;
 
@@ -587,44 +603,65 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j) acc[j] = 0ull;
 
-            // Narrow tiles, one K block with scale product t: wait for the partial, then per 32-column chunk load, (after the last load)
-            // hand the buffer back, convert and accumulate.
-            [[maybe_unused]] auto k_block_narrow = [&](float t) -> bool {
-                if (!wait_partial(bar_part_0 + st_off, st_par)) return false;
-                const uint64_t t2 = f32x2(t, t);
+            // One K block with the scale products t[h] of its column halves: per half wait for the partial, then per 32-column chunk
+            // load, (after the half's last load) hand the half back, convert and accumulate.  The barrier that follows (the
+            // other half's, or half 0 of the next K block: the stage ring runs on across tiles; behind the last K block the test
+            // fails and is never looked at) is tested before the last chunk's arithmetic.
+            // J >= 0: K block J of a group of four under kStaticRing; J < 0: the running counters.
+            [[maybe_unused]] auto k_block_coupled = [&](const float (&t)[SPLIT], auto jc) -> bool {
+                constexpr int J = decltype(jc)::value;
+                const uint32_t so = J >= 0 ? static_cast<uint32_t>(J * 8) : st_off;
+                const uint32_t bo = J >= 0 ? static_cast<uint32_t>((J & 1) * 8) : buf_off;
+                const uint32_t bc = J >= 0 ? static_cast<uint32_t>((J & 1) * BN) : buf_col;
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    uint32_t v[CHW];
-                    tmem_ld(tm_warp + buf_col + c * CHW, v);
-                    tmem_ld_wait();
-                    if (c + 1 == NC) {
-                        release_partial(0, buf_off);
-                        // (the stage ring runs on across tiles; behind the last K block the test fails and is never looked at)
-                        uint32_t so = st_off + 8, sp = st_par;
-                        if (so == STAGES * 8) so = 0, sp ^= 1;
-                        polled = mbar_test_wait_addr(bar_part_0 + so, sp);
+                for (int h = 0; h < SPLIT; ++h) {
+                    if (!wait_partial(bar_part_0 + h * (STAGES * 8) + so, st_par)) return false;
+                    const float ts = BIASED ? t[h] * 0x1p22f : t[h];
+                    const uint64_t t2 = f32x2(ts, ts);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        uint32_t v[CHW];
+                        tmem_ld(tm_warp + bc + h * NSUB + c * CHW, v);
+                        tmem_ld_wait();
+                        if (c + 1 == NC) {
+                            release_partial(h, bo);
+                            uint32_t so_n = so, sp_n = st_par;
+                            if (h + 1 == SPLIT) {
+                                so_n += 8;
+                                if (so_n == STAGES * 8) so_n = 0, sp_n ^= 1;
+                            }
+                            polled = mbar_test_wait_addr(bar_part_0 + (h + 1) % SPLIT * (STAGES * 8) + so_n, sp_n);
+                        }
+#pragma unroll
+                        for (int q = 0; q < CHW / 2; ++q) {
+                            uint64_t& a = acc[h * (SEGW / 2) + c * (CHW / 2) + q];
+                            if constexpr (BIASED) promote_pair_biased(a, v[2 * q], v[2 * q + 1], unbias_c2, unbias_b2, t2);
+                            else promote_pair(a, v[2 * q], v[2 * q + 1], t2);
+                        }
                     }
-#pragma unroll
-                    for (int q = 0; q < CHW / 2; ++q) promote_pair(acc[c * (CHW / 2) + q], v[2 * q], v[2 * q + 1], t2);
                 }
-                st_off += 8;
-                if (st_off == STAGES * 8) st_off = 0, st_par ^= 1;
-                buf_off += 8, buf_col += BN;
-                if (buf_off == NBUF * 8) buf_off = 0, buf_col = 0;
+                if constexpr (J < 0) {
+                    st_off += 8;
+                    if (st_off == STAGES * 8) st_off = 0, st_par ^= 1;
+                    buf_off += 8, buf_col += BN;
+                    if (buf_off == NBUF * 8) buf_off = 0, buf_col = 0;
+                } else if constexpr (J == 3) {
+                    st_par ^= 1;
+                }
                 return true;
             };
-            // Column halves, one K block with the scale products t[h], whose partials lie in buffer B; its first chunk is on the
+            // DECOUPLED, one K block with the scale products t[h], whose partials lie in buffer B; its first chunk is on the
             // way into v[0].  Per chunk: wait for its load, (after a half's last load) hand the half back, start the load of
             // the next chunk, which may lie in the other half or in the next K block, and accumulate this one under that load.
             // A half's barrier is tested one chunk's arithmetic before the load that needs it.
             [[maybe_unused]] uint32_t v[2][CHW];
             [[maybe_unused]] auto wait_half = [&](int h, int b) { return wait_partial(bar_part_0 + (h * NBUF + b) * 8, (buf_par >> b) & 1u); };
             [[maybe_unused]] auto load_chunk = [&](int h, int b, int c, uint32_t (&r)[CHW]) { tmem_ld(tm_warp + b * BN + h * NSUB + c * CHW, r); };
-            auto k_block = [&](const float (&t)[SPLIT], auto buffer, bool has_next) -> bool {
-                [[maybe_unused]] constexpr int B = decltype(buffer)::value;
-                if constexpr (SPLIT == 1) {
-                    return k_block_narrow(t[0]);
+            auto k_block = [&](const float (&t)[SPLIT], auto jc, [[maybe_unused]] bool has_next) -> bool {
+                if constexpr (!DECOUPLED) {
+                    return k_block_coupled(t, jc);
                 } else {
+                    constexpr int B = decltype(jc)::value;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const float ts = t[h] * 0x1p22f;
@@ -658,10 +695,15 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     return true;
                 }
             };
-            using Buffer0 = std::integral_constant<int, 0>;
-            using Buffer1 = std::integral_constant<int, 1>;
+            // K block j of a group of four, and of a pair, as k_block wants them.
+            auto of_four = [](auto j) { return std::integral_constant<int, DECOUPLED ? decltype(j)::value & 1 : kStaticRing ? decltype(j)::value : -1>{}; };
+            auto of_two = [](auto j) { return std::integral_constant<int, DECOUPLED ? decltype(j)::value : -1>{}; };
+            using J0 = std::integral_constant<int, 0>;
+            using J1 = std::integral_constant<int, 1>;
+            using J2 = std::integral_constant<int, 2>;
+            using J3 = std::integral_constant<int, 3>;
 
-            if constexpr (SPLIT == 2) {
+            if constexpr (DECOUPLED) {
                 static_assert(NC >= 2 && NC % 2 == 0, "a half's barrier is tested one chunk ahead; a K block is an even number of chunks");
                 polled = false;
                 if (!wait_half(0, 0)) break;
@@ -692,16 +734,16 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     float t[SPLIT];
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.x, sw_c[h].x);
-                    ok = k_block(t, Buffer0{}, true);
+                    ok = k_block(t, of_four(J0{}), true);
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.y, sw_c[h].y);
-                    ok = ok && k_block(t, Buffer1{}, true);
+                    ok = ok && k_block(t, of_four(J1{}), true);
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.z, sw_c[h].z);
-                    ok = ok && k_block(t, Buffer0{}, true);
+                    ok = ok && k_block(t, of_four(J2{}), true);
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) t[h] = mul_in_place(sa_c.w, sw_c[h].w);
-                    ok = ok && k_block(t, Buffer1{}, kb + 4 < num_kb);
+                    ok = ok && k_block(t, of_four(J3{}), kb + 4 < num_kb);
                     sa_c = sa_n;
 #pragma unroll
                     for (int h = 0; h < SPLIT; ++h) sw_c[h] = sw_n[h];
@@ -735,7 +777,7 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                         for (int h = 0; h < SPLIT; ++h) sw_q[j][h] = ldg_in_place(p.sw + (sw_off[h] + kb + 2));
                     }
-                    return j == 0 ? k_block(t, Buffer0{}, kb + 1 < num_kb) : k_block(t, Buffer1{}, kb + 1 < num_kb);
+                    return j == 0 ? k_block(t, of_two(J0{}), kb + 1 < num_kb) : k_block(t, of_two(J1{}), kb + 1 < num_kb);
                 };
                 for (int kb = 0; kb < num_kb && ok; kb += 2) {
                     ok = k_block_scalar(kb, 0);

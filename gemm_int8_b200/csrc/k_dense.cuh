@@ -106,7 +106,8 @@ GI8_DEVICE bool warp_agrees(bool ok, uint32_t* status, volatile uint32_t* abort_
 // is still on its way when the CTA exits lands in shared memory that belongs to another CTA by then: completion of a later
 // commit (the accumulator's) does not say that the arrivals of the earlier ones have been made.  (s, ph) is the slot after
 // the last armed one; the walk is backwards.
-template <int STAGES>
+// RINGS: bar_done is that many rings of barriers, one after the other.
+template <int STAGES, int RINGS = 1>
 GI8_DEVICE void drain_stages(uint64_t* bar_full, uint64_t* bar_done, uint32_t s, uint32_t ph, uint32_t armed, uint32_t* status,
                              volatile uint32_t* abort_flag)
 {
@@ -114,7 +115,10 @@ GI8_DEVICE void drain_stages(uint64_t* bar_full, uint64_t* bar_done, uint32_t s,
         if (s == 0) s = STAGES, ph ^= 1;
         --s;
         const bool landed = __all_sync(0xffffffffu, !bar_full || mbar_wait(&bar_full[s], ph));
-        if (!warp_agrees(landed && wait_or_abort(&bar_done[s], ph, abort_flag), status, abort_flag, ERR_TIMEOUT_DRAIN) && !landed) return;
+        bool done = landed;
+#pragma unroll
+        for (int r = 0; r < RINGS; ++r) done = done && wait_or_abort(&bar_done[r * STAGES + s], ph, abort_flag);
+        if (!warp_agrees(done, status, abort_flag, ERR_TIMEOUT_DRAIN) && !landed) return;
     }
 }
 

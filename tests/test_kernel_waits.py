@@ -34,8 +34,8 @@ def test_last_commits_are_awaited(body):
     """The barrier that the issuer's commits hand a stage back on is waited for to the last of them, by the producer of each CTA."""
     ring = "bar_done" if re.search(r"\bbar_done\[", body) else "bar_empty"
     assert re.search(r"umma_commit\(&%s\[|umma_commit_pair\(map_to_cta\((smem_u32\(&%s\[|done_0)" % (ring, ring), body)
-    drains = re.findall(r"drain_stages<STAGES>\(([^;]*)\);", body)
-    assert len(drains) == 1 and re.search(r"bar_full, %s, " % ring, drains[0])
+    drains = re.findall(r"drain_stages<STAGES(?:, DONE_RINGS)?>\(([^;]*)\);", body)
+    assert len(drains) == 1 and re.search(r"bar_full, %s(\[0\])?, " % ring, drains[0])
 
 
 def test_staging_blocks_alternate_from_store_to_store():
