@@ -32,8 +32,9 @@ GI8_DEVICE float warp_max(float v)
 
 // q = clamp(rint(v / s)) with the IEEE quotient, at the price of a multiplication for all but one element in
 // several thousand: v * r, r an approximate 1/s (one unit in the last place), is within 2^-15 of the correctly rounded
-// quotient (|v / s| <= 127: 127 * (2^-23 of r, 2^-24 of the product, 2^-24 of the quotient) = 3.1e-5), so rounding it
-// gives the same integer unless it lies within 7e-5 of a half-integer -- only then is the division carried out.
+// quotient (|v / s| <= 127: 127 * (2^-23 of r, 2^-24 of the quotient) = 2.3e-5, and 2^-24 of the product where that is rounded
+// first, 3.1e-5), so rounding it gives the same integer unless it lies within 7e-5 of a half-integer -- only then is the
+// division carried out.
 // r is NaN for blocks whose scale is so small or large that 1/s overflows or loses accuracy: every comparison with it
 // then fails and all their elements take the division.
 struct QuantScale {
@@ -130,12 +131,21 @@ GI8_DEVICE uint32_t pack_i8x4(int a, int b, int c, int d)
 // |v| <= amax, so no clamp.
 // The largest of the four distances decides (a NaN among them fails the test): packed arithmetic and three-operand
 // maxima make that about 3.5 instructions an element, where scalar ones with a comparison each took seven.
+// FUSED = false: the product is rounded first, one packed instruction more for two elements (what the row quantiser takes: see there).
+template <bool FUSED = true>
 GI8_DEVICE uint32_t quant_pack4(uint64_t v0, uint64_t v1, const QuantScale& qs)
 {
     const uint64_t magic = f32x2(12582912.0f, 12582912.0f);
     const uint64_t r2 = f32x2(qs.r, qs.r);
-    const uint64_t u0 = fma2(v0, r2, magic), u1 = fma2(v1, r2, magic);
-    const uint64_t d0 = fma2(v0, r2, sub2(magic, u0)), d1 = fma2(v1, r2, sub2(magic, u1));
+    uint64_t u0, u1, d0, d1;
+    if constexpr (FUSED) {
+        u0 = fma2(v0, r2, magic), u1 = fma2(v1, r2, magic);
+        d0 = fma2(v0, r2, sub2(magic, u0)), d1 = fma2(v1, r2, sub2(magic, u1));
+    } else {
+        const uint64_t t0 = mul2(v0, r2), t1 = mul2(v1, r2);
+        u0 = add2(t0, magic), u1 = add2(t1, magic);
+        d0 = sub2(t0, sub2(u0, magic)), d1 = sub2(t1, sub2(u1, magic));
+    }
     float a, b, c, d;
     f32x2_split(d0, a, b), f32x2_split(d1, c, d);
     if (max3_abs_nan(max3_abs_nan(a, b, c), d, 0.0f) <= 0.49993f) {
@@ -275,13 +285,15 @@ quantize_token_block_kernel(const T* __restrict__ a, int8_t* __restrict__ q, flo
 // the maximum and the quantisation, so that the row is read once; what lies beyond them is read again (it hits L1 or L2).
 // The host takes the smallest of 2, 4 and 8 that holds the row (eight: 16384 bf16 or 8192 fp32 elements): registers that
 // a short row leaves unused would cost resident CTAs.
-// 16384 x 8192, row read twice -> held in registers: fp32 149 -> 102 us (6.6 TB/s), bf16 126 -> 88.5 (on another box 74.6, since then 73).
-// Beyond the registers the second read stays: 8192 x 28672 fp32 322 -> 246 us.
-// Four CTAs per SM even with eight loads, which the maximum on packed bf16 makes room for (64 registers; unbounded it takes 72 and three
-// fit): bf16 4096 x 14336 36.7 -> 33.5 us (unbounded 35.8), 8192 x 28672 184 -> 131 us (unbounded 151), with the shorter
-// quant_pack4 included.
+// 16384 x 8192, row read twice -> held in registers: fp32 149 -> 102 us (6.6 TB/s), bf16 126 -> 88.5, since then 85.
+// Beyond the registers the second read stays: 8192 x 28672 fp32 322 -> 240 us.
+// bf16 with eight loads: four CTAs per SM, which the maximum on packed bf16 makes room for (64 registers; without the bound 72 and three
+// fit): 4096 x 14336 43.6 -> 39.1 us, 8192 x 28672 208 -> 146.  fp32 with two loads: six (40 registers for 42), 2048 x 2048 6.9 -> 6.4.  The
+// other forms are left to the compiler, and fp32 keeps the plain maximum and all of them the rounded product (quant_pack4<false>): with
+// bounds everywhere, the nested maximum and the fused product fp32 8192 x 28672 took 250 us for 240, 4096 x 14336 58.0 for 55.8, 4096 x
+// 4096 16.7 for 16.1, bf16 4096 x 4096 16.3 for 15.6, 8192 x 28672 151 for 146 (a bound of one CTA per SM: fp32 380).
 template <typename T, int LOADS>
-__global__ void __launch_bounds__(kQuantThreads, LOADS == 8 ? 4 : LOADS == 4 ? 5 : 6)
+__global__ void __launch_bounds__(kQuantThreads, sizeof(T) == 2 ? (LOADS == 8 ? 4 : 0) : (LOADS == 2 ? 6 : 0))
 quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float* __restrict__ s, int64_t M, int K,
                           bool release_late)
 {
@@ -297,11 +309,19 @@ quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float
 #pragma unroll
         for (int u = 0; u < LOADS; ++u)
             raw[u] = col0 + u * kStep < K ? __ldg(reinterpret_cast<const uint4*>(src + col0 + u * kStep)) : make_uint4(0u, 0u, 0u, 0u);
+        auto amax_of = [](const uint4& u) {
+            if constexpr (sizeof(T) == 2) {
+                return amax16<T>(u);
+            } else {
+                uint64_t v[EPL / 2];
+                unpack16<T>(u, v);
+                return amax_pairs<EPL / 2>(v);
+            }
+        };
         float amax = 0.0f;
 #pragma unroll
-        for (int u = 0; u < LOADS; ++u) amax = fmaxf(amax, amax16<T>(raw[u]));
-        for (int col = col0 + LOADS * kStep; col < K; col += kStep)
-            amax = fmaxf(amax, amax16<T>(__ldg(reinterpret_cast<const uint4*>(src + col))));
+        for (int u = 0; u < LOADS; ++u) amax = fmaxf(amax, amax_of(raw[u]));
+        for (int col = col0 + LOADS * kStep; col < K; col += kStep) amax = fmaxf(amax, amax_of(__ldg(reinterpret_cast<const uint4*>(src + col))));
         amax = warp_max(amax);
         // (two sets of slots in turn: one barrier per row is enough)
         if ((threadIdx.x & 31) == 0) warp_amax[parity][threadIdx.x >> 5] = amax;
@@ -315,8 +335,8 @@ quantize_token_row_kernel(const T* __restrict__ a, int8_t* __restrict__ q, float
             uint64_t v[EPL / 2];
             unpack16<T>(u, v);
             int8_t* dst = q + row * K + col;
-            if constexpr (EPL == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(quant_pack4(v[0], v[1], sc), quant_pack4(v[2], v[3], sc));
-            else *reinterpret_cast<uint32_t*>(dst) = quant_pack4(v[0], v[1], sc);
+            if constexpr (EPL == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(quant_pack4<false>(v[0], v[1], sc), quant_pack4<false>(v[2], v[3], sc));
+            else *reinterpret_cast<uint32_t*>(dst) = quant_pack4<false>(v[0], v[1], sc);
         };
 #pragma unroll
         for (int u = 0; u < LOADS; ++u)
