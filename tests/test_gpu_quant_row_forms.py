@@ -22,7 +22,7 @@ def test_forms(dtype, loads, extra):
     q, s = g.quantize_per_token(a)
     v = a.float()
     amax = v.abs().amax(dim=1)
-    want_s = torch.where(amax > 0, amax / 127.0, torch.ones_like(amax))
+    want_s = torch.where(amax > 0, amax / torch.full_like(amax, 127.0), torch.ones_like(amax))
     assert torch.equal(s.flatten(), want_s)
     want = torch.round(v / want_s[:, None]).clamp(-127, 127).to(torch.int8)
     assert torch.equal(q, want)
