@@ -746,10 +746,20 @@ SmallMPlan plan_smallm_plain(int64_t M, int64_t N, int64_t K, int sms)
 }
 
 // Block-scaled products of up to sixteen tokens run on blockwise_smallm_kernel whatever N and K (its header has both sides of the line).
-// Four stages let two CTAs share an SM, which grids of more than one CTA per SM need (16 x 14336 x 4096 14.6 us, with six stages 19.4);
-// where every CTA has an SM to itself six put more bytes in flight (16 x 8192 x 8192 and 16 x 4096 x 14336 with four: 17.7 and 23.8 against 17.8
-// and 26.0 us in one build, 17.5 and 25.5 with six in another: level).
 bool use_blockwise_smallm(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= kBwSmallTokens && N > 0 && K > 0; }
+
+// Its stages.  Four let two CTAs share an SM: grids of more than one CTA per SM need that (us with four / six stages: 16 x 14336 x 4096
+// 13.7 / 18.4, 16 x 57344 x 1024 18.5 / 30.2), and calls back to back gain by it, since the next call's CTAs sit down beside
+// this one's (16 x 4096 x 4096 8.4 / 8.6, 16 x 5120 x 4096 8.6 / 9.4, 16 x 6144 x 2048 6.1 / 6.7, 16 x 9472 x 4096 10.1 / 10.3).  Six put more
+// bytes in flight: ahead where the CTAs fill most of the machine and stay for long (16 x 8192 x 8192 16.0 / 15.6, x 28672 43.9 / 43.0, 1 x
+// 8192 x 8192 15.7 / 15.3; level at 16 x 7168 x 12288 and 16 x 9472 x 8192), and behind a quantiser, whose time their first
+// weights are requested in (layers: 16 x 8192 x 8192 18.0 / 17.2, 8 x 7168 x 8192 18.0 / 17.0, 16 x 9472 x 8192 19.1 / 18.3, 16 x 2048 x 8192
+// 15.9 / 15.6, 16 x 4096 x 14336 23.8 / 23.4; level up to K = 4096).
+bool blockwise_smallm_six_stages(int64_t N, int64_t K, bool after_quant, int sms)
+{
+    const int64_t ctas = (N + kBwSmallTileN - 1) / kBwSmallTileN;
+    return ctas <= sms && (after_quant || (ctas * 5 > sms * static_cast<int64_t>(4) && K >= 8192));
+}
 
 template <int STAGES>
 int launch_blockwise_smallm(DeviceState* st, int slot, const int8_t* x, const int8_t* w, const BlockwiseSmallMParams& p, cudaStream_t stream)
@@ -1403,7 +1413,7 @@ static int blockwise_dispatch(const int8_t* x, const int8_t* y, const float* sa,
         q.ldo = N, q.ld_sa = ld_sa, q.ld_sw = ld_sw, q.M = (int)M, q.N = (int)N, q.K = (int)K;
         q.after_quant = after_quant && knobs().pdl;
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        if (N <= static_cast<int64_t>(kBwSmallTileN) * st->sm_count) return launch_blockwise_smallm<6>(st, 33, x, y, q, s);
+        if (blockwise_smallm_six_stages(N, K, q.after_quant, st->sm_count)) return launch_blockwise_smallm<6>(st, 33, x, y, q, s);
         return launch_blockwise_smallm<4>(st, 32, x, y, q, s);
     }
     if (g_forced_variant == VAR_AUTO && M > 0 && N > 0 && K > 0 && out && reinterpret_cast<uintptr_t>(out) % 16 == 0 && N % 8 == 0) {
