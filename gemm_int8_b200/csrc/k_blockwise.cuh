@@ -50,9 +50,10 @@
 // buffers with barriers of their own (their ring positions are compile-time constants whatever the stage count), six stages
 // instead of four in the two-CTA form (four starved it: 1.5 us a round trip), loads one chunk ahead and a warp-uniform issue
 // loop, all together (DECOUPLED, on column halves): 8192^3 511 -> 492 us, two-CTA 492 -> 478, 512 x 9472 x 16384 two-CTA 73.9 -> 72.1.
-// A tile of few K blocks feels its start: scales requested before the wait for the first partial instead of behind it 4096 x 4096 x
-// 1024 30.0 -> 29.4 us (two-CTA 29.8 -> 29.1), and the waits for either half written as one statement -> 28.0 (28.2); 8192 x 8192 x 512
-// 72.5 -> 68.9; from K = 4096 on level.
+// The waits for the next half are one statement in that loop, not one in each of two branches, which compiled to 6 % more code and a loop
+// that short tiles felt: 4096 x 4096 x 1024 30.0 -> 27.9 us (two-CTA 29.8 -> 28.4), 900 x 12040 x 1024 24.0 -> 22.5, 8192 x 8192 x 512 72.7
+// -> 68.0; level from K = 4096 on.  (The first scales requested before the wait for a tile's first partial: the same there, two-CTA
+// tiles of long K 0.5 % slower.)
 // One-CTA tiles keep the coupled form (one commit per half, plain 32-column loads) on grids of up to two waves, where the other loses,
 // most where weights stream past few tokens, us coupled / decoupled: 64 x 28672 x 8192 46.9 / 49.1, 100 x 37888 x 4096 32.9 / 33.9, 128 x
 // 37888 x 8192 62.0 / 63.5, 384 x 12544 x 8192 46.6 / 47.2, 1024 x 4096 x 8192 level; 1.5 to 2 waves: 384 x 25088 x 4096 50.0 / 52.0, 32 x
@@ -66,7 +67,7 @@
 // before the waiter has consumed the first; the comment at each barrier says what gates its next phase):
 //   bar_full[s]        completed by the TMA bytes of K block `it` (s = it % STAGES).  Waiter: the issuer of K block
 //                      `it` (with column halves: both issuers, each of which visits every K block).  Next phase
-//                      needs the producer to refill stage s, which needs bar_done[s] of K block `it`, i.e. every waiting
+//                      needs the producer to refill stage s, which needs bar_done of K block `it` (of either half), i.e. every waiting
 //                      issuer's own commit: gated by each waiter.
 //   bar_done[h][s]     completed by the issuer's commit for column half h of K block `it`.  Waiters: the producer (before refilling s,
 //                      and at its end for the stages not refilled; the next completion needs its own refill: gated) and all
@@ -703,17 +704,12 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             using J2 = std::integral_constant<int, 2>;
             using J3 = std::integral_constant<int, 3>;
 
-            // DECOUPLED: the tile's first partial and the load of its first chunk.  Called once the first scales have been requested, so
-            // that their way from L2 lies under the wait (see the header).
-            [[maybe_unused]] auto begin_tile = [&]() -> bool {
-                if constexpr (DECOUPLED) {
-                    static_assert(NC >= 2 && NC % 2 == 0, "a half's barrier is tested one chunk ahead; a K block is an even number of chunks");
-                    polled = false;
-                    if (!wait_half(0, 0)) return false;
-                    load_chunk(0, 0, 0, v[0]);
-                }
-                return true;
-            };
+            if constexpr (DECOUPLED) {
+                static_assert(NC >= 2 && NC % 2 == 0, "a half's barrier is tested one chunk ahead; a K block is an even number of chunks");
+                polled = false;
+                if (!wait_half(0, 0)) break;
+                load_chunk(0, 0, 0, v[0]);
+            }
             if (p.scale_vec) {
                 // Scales of four K blocks per load (16 bytes per row): a quarter of the load instructions and of
                 // the sectors touched (a token's scales of eight consecutive K blocks share one 32-byte sector, and
@@ -722,7 +718,6 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 float4 sa_c = ldg4_in_place(p.sa + sa_off), sw_c[SPLIT];
 #pragma unroll
                 for (int h = 0; h < SPLIT; ++h) sw_c[h] = ldg4_in_place(p.sw + sw_off[h]);
-                ok = begin_tile();
                 for (int kb = 0; kb < num_kb && ok; kb += 4) {
                     if constexpr (BIASED) {
                         max_sa = max3_abs(sa_c.x, sa_c.y, max3_abs(sa_c.z, sa_c.w, max_sa));
@@ -785,7 +780,6 @@ blockwise_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     }
                     return j == 0 ? k_block(t, of_two(J0{}), kb + 1 < num_kb) : k_block(t, of_two(J1{}), kb + 1 < num_kb);
                 };
-                ok = begin_tile();
                 for (int kb = 0; kb < num_kb && ok; kb += 2) {
                     ok = k_block_scalar(kb, 0);
                     if (ok && kb + 1 < num_kb) ok = k_block_scalar(kb + 1, 1);
