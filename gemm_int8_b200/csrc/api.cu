@@ -272,14 +272,15 @@ int check_block_scales(const float* sa, int64_t ld_sa, const float* sw, int64_t 
 //   blockwise  128 x 256: 950 | 256 x 256 two-CTA tile: 920 | 128 x 128: 650 | 128 x 64: 490 (fitted when the wide forms still converted
 //              their partials; us per wave and K block between K = 4096 and 16384 since then: 0.56 | 0.56 | 0.37 | 0.27 on full
 //              waves, 0.44 | 0.44 | 0.30 | 0.22 on 32 to 128 CTAs: the same ranking).
-//              The two-CTA tile gains by fewer operand bytes per MAC, which counts the longer the run and the longer K.  0.12 s of
-//              back-to-back calls, one-CTA / two-CTA us, for K = 4096, 6144, 8192, 10240, 12288, 16384:
-//                512 x 8192    23.1/24.2  32.5/33.8  42.8/43.1  52.6/52.6  62.3/62.1  81.2/81.1
-//                1024 x 4096   21.9/22.8  31.7/32.7  41.2/41.7  50.8/50.7  60.6/60.0  79.2/78.8
-//                2048 x 8192   82.7/82.8  120/119    157/154    197/194    235/232    312/307
-//                2048 x 11008  107/106    154/153    200/199    257/250    306/305    414/404
-//              In short bursts, below the power cap, it is level or up to 1 % behind at all of them.  Hence its minimum: twenty
-//              waves, or 96 K blocks, from which on it is not behind on any of these grids in a long run.
+//              The two-CTA tile gains by fewer operand bytes per MAC.  Its minimum, twenty waves or 96 K blocks, was fitted when it had
+//              four stages and was level below that.  With six, back to back, one-CTA / two-CTA us for the product and (in brackets) for
+//              the layer with its quantiser:
+//                one wave   512 x 8192, K = 4096, 8192, 12288    21.9/23.8 (26.8/28.2)  42.7/44.3 (49.7/49.1)  60.0/62.8 (70.2/68.6)
+//                more       2048 x 8192, the same K              83.2/83.2 (92.1/91.7)  157/156 (173/169)  240/235 (264/254)
+//                           2048 x 11008, K = 4096, 8192         107.5/106.8 (117.6/115.2)  202/199 (218/214)
+//                           K = 4096: 4096 x 8192 151/152 (170/166, on another box 165/169), 8192 x 8192 308/299 (337/326)
+//              So the minimum is right for a single wave; in several waves below it the two-CTA tile is level to 4 % ahead by now,
+//              which the table does not use.
 // The table is data: kDenseForms / kBlockwiseForms below.  The narrow tiles cost more per column (the tensor-core instruction is issue
 // bound below N = 128, and the per-K-block hand-overs do not shrink with the tile) and only pay when the wide tile
 // would leave most SMs without work.
@@ -340,7 +341,9 @@ int pick_group_m(int64_t K)
 // CTAs leave (programmatic dependent launch without a wait before its work; it waits before it ends, see
 // BlockwiseParams::pdl_role).  kColumnSplitFixedCycles: set-up and epilogue of the second kernel's CTAs.  Measured on
 // B200, back to back: 512 x 10240 x 8192 (160 tiles) 75.5 -> 60.1 us, 512 x 10240 x 16384 148 -> 112, 512 x 57344 x 8192 302 -> 277,
-// 2048 x 10240 x 8192 202 -> 192.
+// 2048 x 10240 x 8192 202 -> 192.  The first launch on CTA pairs, where the row blocks are even: slower, since a pair starts only where two
+// neighbouring SMs are free (512 x 10240 x 2048 21.8 / 23.9, x 8192 55.6 / 59.7, 256 x 19456 x 4096 34.2 / 37.2, the rotated layer of 499 x
+// 10240 x 8192 78.1 / 81.0; ahead at 256 x 19456 x 8192 behind its quantiser, 69.9 / 69.1).
 constexpr double kColumnSplitFixedCycles = 10000.0;  // measured: a lone 64-wide launch of 64 K blocks takes 5 us more than its K blocks
 struct ColumnSplit {
     bool use;

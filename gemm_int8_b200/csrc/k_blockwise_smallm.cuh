@@ -20,9 +20,9 @@
 //   bar_read[s]   the promotion warps have loaded the partials.  Waiter: the stage's issuer, whose MMAs the next completion needs.
 // Every wait is gated by its waiter's own next action, so parities cannot be missed; STAGES is even, so that a stage has one issuer.
 //
-// Measured, back to back, weights beyond L2, 64-wide tiles of k_blockwise.cuh -> this kernel, us: 16 x 8192 x 8192 19.7 -> 16.5, 16 x 4096 x
-// 4096 14.2 -> 10.4, 16 x 14336 x 4096 20.9 -> 14.6, 16 x 4096 x 14336 28.9 -> 22.0, 8 x 57344 x 8192 108 -> 82, 1 x 1024 x 4096 11.3 -> 10.2.  On the
-// way: sixteen columns a warp and scale products fetched from shared memory between the multiply-adds 17.5 at 16 x 8192 x 8192, the next
+// Measured, back to back, weights beyond L2, 64-wide tiles of k_blockwise.cuh -> this kernel (with the stages that the host takes), us:
+// 16 x 8192 x 8192 18.8 -> 15.9 (six), 16 x 4096 x 4096 13.9 -> 8.3, 16 x 14336 x 4096 20.9 -> 13.7, 16 x 4096 x 14336 28.1 -> 21.3, 8 x 57344 x
+// 8192 108 -> 82, 1 x 1024 x 4096 10.2 -> 7.6 (four), and from K = 16 on (16 x 57344 x 128 11.6 -> 10.2, 16 x 4096 x 16 5.9 -> 5.7).  On the way: sixteen columns a warp and scale products fetched from shared memory between the multiply-adds 17.5 at 16 x 8192 x 8192, the next
 // stage's load not under this one's arithmetic 19.3.  With 32 tokens the same form is no better than the tiles (32 x 8192 x 8192 19.7 ->
 // 20.4, 32 x 28672 x 4096 25.6 -> 41.0, 20 x 14336 x 4096 22.0 -> 22.3), so those keep them.
 #pragma once

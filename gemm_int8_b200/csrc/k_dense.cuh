@@ -3,10 +3,10 @@
 // Replaces the reference's CUTLASS Sm80 mma.sync instantiation (csrc/kernels/gemm.cu:46-65) and its
 // LinearCombination epilogue (csrc/kernels/gemm.cu:59-63, 96).
 //
-// Structure (one persistent CTA per SM, 192 threads):
+// Structure (one persistent CTA per SM, 192 or 320 threads):
 //   warp 0      TMA producer: K-major 128-byte-wide tiles of X and Y into 128B-swizzled shared memory,
 //               STAGES-deep ring guarded by full/empty mbarriers.
-//   warp 1      MMA issuer: one thread issues tcgen05.mma kind::i8 (128 x BN x 32 per instruction),
+//   warp 1      MMA issuer: an elected lane issues tcgen05.mma kind::i8 (128 x BN x 32 per instruction),
 //               int32 accumulators live in tensor memory; two accumulator buffers so the epilogue of
 //               tile i overlaps the main loop of tile i+1.
 //   warps 2..5 or 2..9  epilogue: tcgen05.ld the accumulator (a warp owns the 32-lane quarter warp_id % 4, and with eight warps half
@@ -21,7 +21,7 @@ namespace gi8 {
 constexpr int kBM = 128;       // rows of X per tile = UMMA M
 constexpr int kBK = 128;       // int8 elements (= bytes) of K per pipeline stage = one swizzle row
 constexpr int kUmmaK = 32;     // K per tcgen05.mma kind::i8
-constexpr int kDenseEpilogueWarps = 8;  // at most: the launch has four or eight (see the host's epilogue_warps)
+constexpr int kDenseEpilogueWarps = 8;  // at most: the launch has four or eight (see the host's dense_threads)
 constexpr int kDenseThreads = 64 + 32 * kDenseEpilogueWarps;
 
 enum Epilogue : int {

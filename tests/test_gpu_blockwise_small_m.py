@@ -1,5 +1,5 @@
 """Block-scaled products of up to sixteen tokens run on a kernel of their own (64 weight rows against 16 tokens): bit equality with the oracle
-at the edges of its tiles, at odd counts of K blocks, around the depth of its rings (four and six stages of two K blocks), for scales
+at the edges of its tiles, at odd counts of K blocks, around the depth of its rings (four stages of two K blocks; six: see the test of the stages), for scales
 whose products overflow or vanish, and for outputs of odd width; the seventeenth token is another kernel's."""
 import numpy as np
 import pytest
