@@ -278,7 +278,7 @@ int check_block_scales(const float* sa, int64_t ld_sa, const float* sw, int64_t 
 //                one wave   512 x 8192, K = 4096, 8192, 12288    21.9/23.8 (26.8/28.2)  42.7/44.3 (49.7/49.1)  60.0/62.8 (70.2/68.6)
 //                more       2048 x 8192, the same K              83.2/83.2 (92.1/91.7)  157/156 (173/169)  240/235 (264/254)
 //                           2048 x 11008, K = 4096, 8192         107.5/106.8 (117.6/115.2)  202/199 (218/214)
-//                           K = 4096: 4096 x 8192 151/152 (170/166, on another box 165/169), 8192 x 8192 308/299 (337/326)
+//                           K = 4096: 4096 x 8192 151/152 (170/166, on another machine 165/169), 8192 x 8192 308/299 (337/326)
 //              So the minimum is right for a single wave; in several waves below it the two-CTA tile is level to 4 % ahead by now,
 //              which the table does not use.
 // The table is data: kDenseForms / kBlockwiseForms below.  The narrow tiles cost more per column (the tensor-core instruction is issue

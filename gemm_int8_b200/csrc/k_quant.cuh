@@ -222,7 +222,7 @@ GI8_DEVICE void group_scales(float (&m)[U], float (&s)[U], float (&r)[U])
 // bf16 input, which is closer to the bound of instruction issue, four.
 // Bound: HBM for fp32 (16384 x 8192: 128 -> 113 us, 6.0 TB/s, 0.91 of the copy bandwidth); for bf16 (103 -> 88 us, 4.6 TB/s, 0.71) no
 // single unit; fewer instructions help: maxima on packed bf16 and quant_pack4 with two packed multiply-adds 90.4 -> 85.4 us (another
-// box), 4096 x 14336 40.7 -> 38.6.  Both with the packed arithmetic and one division per lane instead of one or two per block and lane (group_scales).
+// machine), 4096 x 14336 40.7 -> 38.6.  Both with the packed arithmetic and one division per lane instead of one or two per block and lane (group_scales).
 // a [M,K] (K % EPL == 0, rows 16-byte aligned) -> q int8 [M,K], s fp32 [M, ceil(K/128)].
 constexpr int kQuantBlocksPerItem = 8;  // 128-wide blocks per warp and iteration, whatever the type (1 x 8 or 2 x 4)
 
